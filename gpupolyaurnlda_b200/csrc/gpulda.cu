@@ -47,7 +47,7 @@ constexpr u32 kPieceEnd[kPieces] = {1, 3, 7, 12, 18, 24, 29, 32};
 // last pieces do not set the sweep's tail.
 constexpr u32 kLongFactor = 4;
 
-constexpr u32 kWorkCounters = 2 + 2 * kPieces;
+constexpr u32 kWorkCounters = 3 + 2 * kPieces;
 
 struct BufCtx {
   cudaStream_t stream = nullptr;  // sweeps
@@ -59,10 +59,12 @@ struct BufCtx {
   cudaEvent_t offs = nullptr;     // document offsets of the current sweep are ready
   bool used = false;
   u32* order = nullptr;           // device: document processing order
+  u64* rest = nullptr;            // device: documents the list sweep hands on (K > kMapMinK)
   // Device work counters of this buffer's launches (kWorkCounters), so sweeps
   // of different buffers may be in flight at the same time: [0] whole buffer,
   // [1, 1 + kPieces) pieces, [1 + kPieces] short documents beside a split sweep,
-  // [2 + kPieces, 2 + 2 kPieces) the pieces' long documents.
+  // [2 + kPieces, 2 + 2 kPieces) the pieces' long documents, [2 + 2 kPieces] the
+  // number of documents that a list sweep hands on.
   u32* work = nullptr;
   std::vector<u32> order_host;    // host staging of the order
   // The last host-buffer sweep's document lengths and what was derived from
@@ -91,11 +93,10 @@ void longest_first(const u32* d_len, u32 n, std::vector<u32>& order) {
   for (u32 i = 0; i < n; ++i) order[start[max_len - d_len[i]]++] = i;
 }
 
-// Above this many topics a document's counts live in a shared-memory hash map
-// (a dense per-document count array would cost 2 K bytes of shared memory per
-// warp); documents of at most kShortDoc tokens are swept by one launch with a
+// Above kMapMinK topics a document's counts live in a shared-memory hash map
+// or list (a dense per-document count array would cost 2 K bytes of shared
+// memory); documents of at most kShortDoc tokens are swept by one launch with a
 // small map per warp, longer ones by a second launch sized for the longest.
-constexpr u32 kMapMinK = 2048;
 constexpr u32 kShortDoc = 256;
 
 // Documents longer than kShortDoc and at most kMidDoc tokens are swept by a
@@ -108,28 +109,10 @@ constexpr u32 kMidDoc = 1024;
 // are longer than kMidDoc (they come first among them).
 struct DocSplit {
   u32 n_short = 0;
-  u32 lmax_long = 0;
+  u32 lmax_long = 0;  // longest document
   u32 n_huge = 0;    // documents longer than kMidDoc (the first of the long ones)
   u32 lmax_mid = 0;  // longest document of at most kMidDoc tokens among the long ones
 };
-
-DocSplit split_longest_first(const u32* d_len, u32 n, std::vector<u32>& order, u32 K) {
-  longest_first(d_len, n, order);
-  DocSplit sp;
-  if (K <= kMapMinK) return sp;
-  u32 first_short = n;
-  for (u32 i = 0; i < n; ++i)
-    if (d_len[order[i]] <= kShortDoc) {
-      first_short = i;
-      break;
-    }
-  sp.n_short = n - first_short;
-  sp.lmax_long = first_short > 0 ? d_len[order[0]] : 0;
-  while (sp.n_huge < first_short && d_len[order[sp.n_huge]] > kMidDoc) ++sp.n_huge;
-  sp.lmax_mid = sp.n_huge < first_short ? d_len[order[sp.n_huge]] : 0;
-  std::rotate(order.begin(), order.begin() + first_short, order.end());
-  return sp;
-}
 
 struct Model {
   bool live = false;
@@ -169,6 +152,7 @@ struct Model {
   bool noalloc_pending = false;
 
   // device-resident corpus
+  u64* crest = nullptr;  // documents the list sweep hands on (K > kMapMinK)
   u32 *cz = nullptr, *cw = nullptr, *cd_len = nullptr, *cd_idx = nullptr, *cK_d = nullptr, *corder = nullptr;
   u32 c_docs = 0;
   u64 c_tokens = 0;
@@ -176,6 +160,24 @@ struct Model {
 };
 
 Model g;
+
+DocSplit split_longest_first(const u32* d_len, u32 n, std::vector<u32>& order, u32 K) {
+  longest_first(d_len, n, order);
+  DocSplit sp;
+  if (n) sp.lmax_long = d_len[order[0]];
+  if (K <= kMapMinK || !(g.flags & GPULDA_FLAG_HASHMAP)) return sp;
+  u32 first_short = n;
+  for (u32 i = 0; i < n; ++i)
+    if (d_len[order[i]] <= kShortDoc) {
+      first_short = i;
+      break;
+    }
+  sp.n_short = n - first_short;
+  while (sp.n_huge < first_short && d_len[order[sp.n_huge]] > kMidDoc) ++sp.n_huge;
+  sp.lmax_mid = sp.n_huge < first_short ? d_len[order[sp.n_huge]] : 0;
+  std::rotate(order.begin(), order.begin() + first_short, order.end());
+  return sp;
+}
 
 const char* kErrNames[] = {"ok",
                            "CUDA runtime error",
@@ -260,6 +262,7 @@ void free_model() {
   dfree(g.cd_idx);
   dfree(g.cK_d);
   dfree(g.corder);
+  dfree(g.crest);
   for (auto& e : g.ev)
     if (e) cudaEventDestroy(e);
   for (auto& e : g.z_ev)
@@ -310,7 +313,7 @@ int init_impl(const Args* args, Buffer* buffers, u32 n_buffers, const GpuldaExAr
       (rc = dalloc(&g.dev.nnz, g.V)) ||
       (rc = dalloc(&g.C, g.V)) || (rc = dalloc(&g.cdf, (size_t)kPoisN * kPoisW)) ||
       (rc = dalloc(&g.guide, (size_t)kPoisN * 256)) || (rc = dalloc(&g.lfac, kLogFacN)) ||
-      (rc = dalloc(&g.counters, kCtrN)) || (rc = dalloc(&g.ll, 2)) || (rc = dalloc(&g.work, 2 + kPieces)) ||
+      (rc = dalloc(&g.counters, kCtrN)) || (rc = dalloc(&g.ll, 2)) || (rc = dalloc(&g.work, kWorkCounters)) ||
       (rc = dalloc(&g.status, 1))) {
     free_model();
     return rc;
@@ -366,7 +369,8 @@ int init_impl(const Args* args, Buffer* buffers, u32 n_buffers, const GpuldaExAr
     b.gpu_rng = ctx;
     u32 *z, *w, *dl, *di, *kd;
     if ((rc = dalloc(&z, g.buffer_size)) || (rc = dalloc(&w, g.buffer_size)) || (rc = dalloc(&dl, g.max_D)) ||
-        (rc = dalloc(&di, g.max_D)) || (rc = dalloc(&kd, g.max_D)) || (rc = dalloc(&ctx->order, g.max_D)) || (rc = dalloc(&ctx->work, kWorkCounters)))
+        (rc = dalloc(&di, g.max_D)) || (rc = dalloc(&kd, g.max_D)) || (rc = dalloc(&ctx->order, g.max_D)) ||
+        (g.K > kMapMinK && (rc = dalloc(&ctx->rest, g.max_D))) || (rc = dalloc(&ctx->work, kWorkCounters)))
       return rc;
     b.gpu_z = z;
     b.gpu_w = w;
@@ -412,13 +416,8 @@ int phi_step_async(cudaStream_t s) {
   return GPULDA_OK;
 }
 
-// One sweep over documents already on the device.
-// One z-sweep launch over n_docs documents whose d_len / d_idx / order / K_d
-// start at the given pointers; d_idx offsets are relative to z and w, and the
-// tokens' Philox indices start at tok_base.
-int z_launch(cudaStream_t s, u32* z, const u32* w, const u32* d_len, const u32* d_idx, const u32* order, u32* K_d,
-             u32 n_docs, u64 n_tokens, u64 tok_base, u32* work, u32 lmax = 0) {
-  CK(cudaMemsetAsync(work, 0, 4, s));
+ZLaunch z_args(u32* z, const u32* w, const u32* d_len, const u32* d_idx, const u32* order, u32* K_d, u32 n_docs,
+               u64 n_tokens, u64 tok_base, u32* work) {
   ZLaunch zl;
   zl.w = w;
   zl.z = z;
@@ -435,20 +434,50 @@ int z_launch(cudaStream_t s, u32* z, const u32* w, const u32* d_len, const u32* 
   zl.ll = g.ll;
   zl.work = work;
   zl.status = g.status;
-  bool done = false;
-  if (g.K > kMapMinK && lmax)
-    done = (g.flags & GPULDA_FLAG_HASHMAP) ? launch_z_sweep_map(g.dev, zl, s, lmax)
-                                           : launch_z_sweep_pairs(g.dev, zl, s, lmax);
-  if (!done) launch_z_sweep(g.dev, zl, s);
+  return zl;
+}
+
+// One z-sweep launch over n_docs documents whose d_len / d_idx / order / K_d
+// start at the given pointers; d_idx offsets are relative to z and w, and the
+// tokens' Philox indices start at tok_base.
+int z_launch(cudaStream_t s, u32* z, const u32* w, const u32* d_len, const u32* d_idx, const u32* order, u32* K_d,
+             u32 n_docs, u64 n_tokens, u64 tok_base, u32* work, u32 lmax = 0) {
+  CK(cudaMemsetAsync(work, 0, 4, s));
+  const ZLaunch zl = z_args(z, w, d_len, d_idx, order, K_d, n_docs, n_tokens, tok_base, work);
+  // (a document too long for a map in shared memory: dense counts)
+  if (!(g.K > kMapMinK && lmax && launch_z_sweep_map(g.dev, zl, s, lmax))) launch_z_sweep(g.dev, zl, s);
   CK(cudaGetLastError());
   g.launches += 1;
   return GPULDA_OK;
 }
 
-// With a split (large K), `order` lists the short documents first.
-// `work` holds kWorkCounters zeroed-per-launch counters.
+// The large-K sweep without GPULDA_FLAG_HASHMAP: the list sweep, then the
+// documents that outgrew its lists (none when no document is long enough).
+// work: two work counters and the number of documents handed on.
+int z_launch_lists(cudaStream_t s, ZLaunch zl, u32 lmax, u64* rest, u32* work0, u32* work1, u32* n_rest) {
+  CK(cudaMemsetAsync(work0, 0, 4, s));
+  CK(cudaMemsetAsync(n_rest, 0, 4, s));
+  zl.work = work0;
+  zl.rest = rest;
+  zl.n_rest = n_rest;
+  launch_z_sweep_pairs(g.dev, zl, s);
+  CK(cudaGetLastError());
+  g.launches += 1;
+  // a list holds a document's topics and at most 32 more
+  if (std::min(lmax, g.K) + 32 > kListMost) {
+    CK(cudaMemsetAsync(work1, 0, 4, s));
+    zl.work = work1;
+    launch_z_sweep_rest(g.dev, zl, s, lmax);
+    CK(cudaGetLastError());
+    g.launches += 1;
+  }
+  return GPULDA_OK;
+}
+
+// One sweep over documents already on the device.  `work` holds kWorkCounters
+// counters, zeroed per launch.
 int z_step_async(cudaStream_t s, u32* z, const u32* w, const u32* d_len, u32* d_idx, const u32* order, u32* K_d,
-                 u32 n_docs, u64 n_tokens, bool offsets, cudaEvent_t* ev, u32* work, const DocSplit* split = nullptr) {
+                 u32 n_docs, u64 n_tokens, bool offsets, cudaEvent_t* ev, u32* work, const DocSplit& split, u64* rest) {
   CK(cudaEventRecord(ev[0], s));
   if (offsets) {
     launch_doc_offsets(d_len, d_idx, n_docs, s);
@@ -457,22 +486,22 @@ int z_step_async(cudaStream_t s, u32* z, const u32* w, const u32* d_len, u32* d_
   }
   CK(cudaEventRecord(ev[1], s));
   int rc = GPULDA_OK;
-  if (split && g.K > kMapMinK) {
+  if (g.K > kMapMinK && !(g.flags & GPULDA_FLAG_HASHMAP)) {
+    rc = z_launch_lists(s, z_args(z, w, d_len, d_idx, order, K_d, n_docs, n_tokens, g.tok_offset, work),
+                        split.lmax_long, rest, work, work + 1, work + 2 + 2 * kPieces);
+  } else if (g.K > kMapMinK) {
     // Documents over kMidDoc tokens, then those over kShortDoc, then the
-    // short ones, one launch each on `s`, each sized for its longest.  Run
-    // concurrently on two streams the launches competed for whole SMs (each
-    // fills the register file at four blocks per SM): at K=10000 over 8e6
-    // documents the sweep took 489 ms concurrently with three blocks per SM,
-    // 778 ms with four, and 446 ms one after the other with four.
-    const u32 n_long = n_docs - split->n_short;
-    if (split->n_huge)
-      rc = z_launch(s, z, w, d_len, d_idx, order + split->n_short, K_d, split->n_huge, n_tokens, g.tok_offset, work,
-                    split->lmax_long);
-    if (!rc && n_long > split->n_huge)
-      rc = z_launch(s, z, w, d_len, d_idx, order + split->n_short + split->n_huge, K_d, n_long - split->n_huge,
-                    n_tokens, g.tok_offset, work + 1, split->lmax_mid);
-    if (!rc && split->n_short)
-      rc = z_launch(s, z, w, d_len, d_idx, order, K_d, split->n_short, n_tokens, g.tok_offset,
+    // short ones (first in `order`), one launch each on `s`, each sized for its
+    // longest.
+    const u32 n_long = n_docs - split.n_short;
+    if (split.n_huge)
+      rc = z_launch(s, z, w, d_len, d_idx, order + split.n_short, K_d, split.n_huge, n_tokens, g.tok_offset, work,
+                    split.lmax_long);
+    if (!rc && n_long > split.n_huge)
+      rc = z_launch(s, z, w, d_len, d_idx, order + split.n_short + split.n_huge, K_d, n_long - split.n_huge,
+                    n_tokens, g.tok_offset, work + 1, split.lmax_mid);
+    if (!rc && split.n_short)
+      rc = z_launch(s, z, w, d_len, d_idx, order, K_d, split.n_short, n_tokens, g.tok_offset,
                     work + 1 + kPieces, kShortDoc);
   } else {
     rc = z_launch(s, z, w, d_len, d_idx, order, K_d, n_docs, n_tokens, g.tok_offset, work);
@@ -673,7 +702,7 @@ extern "C" void sample_z_async(Buffer* b) {
   CKV(cudaMemcpyAsync(ctx->order, ctx->order_host.data(), db, cudaMemcpyHostToDevice, s));
   CKV(cudaEventRecord(ctx->ev[0], s));
   if (z_step_async(s, (u32*)b->gpu_z, (const u32*)b->gpu_w, (const u32*)b->gpu_d_len, (u32*)b->gpu_d_idx,
-                   ctx->order, (u32*)b->gpu_K_d, b->n_docs, b->n_tokens, true, g.z_ev, ctx->work, &split))
+                   ctx->order, (u32*)b->gpu_K_d, b->n_docs, b->n_tokens, true, g.z_ev, ctx->work, split, ctx->rest))
     return;
   g.z_timed = true;
   CKV(cudaMemcpyAsync(b->z, b->gpu_z, tb, cudaMemcpyDeviceToHost, s));
@@ -729,6 +758,7 @@ extern "C" void cleanup(Buffer* buffers, uint32_t n_buffers) {
       for (auto& ps : ctx->lpiece)
         if (ps) cudaStreamDestroy(ps);
       dfree(ctx->order);
+      dfree(ctx->rest);
       delete ctx;
     }
     delete (cudaStream_t*)b.stream;
@@ -824,10 +854,13 @@ extern "C" int gpulda_corpus_load(const uint32_t* z, const uint32_t* w, const ui
   dfree(g.cd_idx);
   dfree(g.cK_d);
   dfree(g.corder);
+  dfree(g.crest);
+  g.crest = nullptr;
   g.cz = g.cw = g.cd_len = g.cd_idx = g.cK_d = g.corder = nullptr;
   int rc;
   if ((rc = dalloc(&g.cz, n_tokens)) || (rc = dalloc(&g.cw, n_tokens)) || (rc = dalloc(&g.cd_len, n_docs)) ||
-      (rc = dalloc(&g.cd_idx, n_docs)) || (rc = dalloc(&g.cK_d, n_docs)) || (rc = dalloc(&g.corder, n_docs)))
+      (rc = dalloc(&g.cd_idx, n_docs)) || (rc = dalloc(&g.cK_d, n_docs)) || (rc = dalloc(&g.corder, n_docs)) ||
+      (g.K > kMapMinK && (rc = dalloc(&g.crest, n_docs))))
     return rc;
   CK(cudaMemcpy(g.cz, z, n_tokens * 4, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(g.cw, w, n_tokens * 4, cudaMemcpyHostToDevice));
@@ -851,7 +884,7 @@ extern "C" int gpulda_corpus_sweep(uint32_t n_iter) {
     int rc = phi_step_async(s);
     if (rc) return rc;
     rc = z_step_async(s, g.cz, g.cw, g.cd_len, g.cd_idx, g.corder, g.cK_d, g.c_docs, g.c_tokens, false, g.z_ev, g.work,
-                      &g.c_split);
+                      g.c_split, g.crest);
     if (rc) return rc;
     g.z_timed = true;
   }
@@ -1004,9 +1037,9 @@ extern "C" int gpulda_debug_alias(const uint32_t* q, uint32_t K, uint64_t* table
 // For callers that may not allocate device memory at the point of the call:
 // code that owns all device memory through its own pool, services that must
 // not allocate once serving has started, or work issued where cudaMalloc is
-// not permitted.  Its only scratch (document offsets and the work-queue
-// counter) is the file-scope device array below, sized for
-// GPULDA_NOALLOC_MAX_DOCS documents: 4 MiB + 256 B that every GPU which loads
+// not permitted.  Its only scratch (document offsets, work counters and
+// the list of documents a list sweep hands on) is the file-scope device array below, sized for
+// GPULDA_NOALLOC_MAX_DOCS documents: 12 MiB + 256 B that every GPU which loads
 // this library holds until the process exits.  In host code the array's name
 // is only a host-side stand-in; its device address is looked up once per
 // device with cudaGetSymbolAddress (on the first call on that device, which
@@ -1019,8 +1052,9 @@ extern "C" int gpulda_debug_alias(const uint32_t* q, uint32_t K, uint64_t* table
 // ---------------------------------------------------------------------------
 namespace {
 constexpr u32 kNoAllocMaxDocs = GPULDA_NOALLOC_MAX_DOCS;
-constexpr u32 kNoAllocTail = 64;  // work-queue counter and padding
-static __device__ __align__(256) u32 g_noalloc_scratch[kNoAllocMaxDocs + kNoAllocTail];
+constexpr u32 kNoAllocTail = 64;  // work-queue counters and padding
+// document offsets, counters, and (8-byte) the documents that a list sweep hands on
+static __device__ __align__(256) u32 g_noalloc_scratch[kNoAllocMaxDocs + kNoAllocTail + 2 * kNoAllocMaxDocs];
 constexpr int kNoAllocMaxDevices = 64;
 u32* g_noalloc_addr[kNoAllocMaxDevices] = {};
 }  // namespace
@@ -1050,37 +1084,18 @@ extern "C" int gpulda_sample_z_device_noalloc(uint32_t* z, const uint32_t* w, co
   cudaStream_t s = stream ? (cudaStream_t)stream : main_stream();
   // the previous call's use of the shared scratch ends before this one's begins
   if (int rc = after_noalloc(s)) return rc;
-  CK(cudaMemsetAsync(work, 0, sizeof(u32), s));
   launch_doc_offsets(d_len, d_idx, n_docs, s);
   CK(cudaGetLastError());
-  ZLaunch zl;
-  zl.w = w;
-  zl.z = z;
-  zl.d_len = d_len;
-  zl.d_idx = d_idx;
-  zl.order = nullptr;
-  zl.K_d = nullptr;
-  zl.n_docs = n_docs;
-  zl.n_tokens = n_tokens;
-  zl.tok_base = g.tok_offset;
-  zl.t = (u32)g.t;
-  zl.flags = (g.flags & GPULDA_FLAG_LOGLIK) ? kZFlagLoglik : 0u;
-  zl.counters = g.counters;
-  zl.ll = g.ll;
-  zl.work = work;
-  zl.status = g.status;
-  // Above kMapMinK topics, the large-K store the other sweeps use.  The
-  // lengths are on the device only, so the launch accepts any document length
-  // and sizes each document's store for K distinct topics.
-  bool done = false;
-  if (g.K > kMapMinK)
-    done = (g.flags & GPULDA_FLAG_HASHMAP) ? launch_z_sweep_map(g.dev, zl, s, 65535u)
-                                           : launch_z_sweep_pairs(g.dev, zl, s, 65535u);
-  if (!done) launch_z_sweep(g.dev, zl, s);
-  CK(cudaGetLastError());
+  // Above kMapMinK topics, the large-K stores the other sweeps use.  The
+  // lengths are on the device only, so the launches take any document length.
+  const ZLaunch zl = z_args(z, w, d_len, d_idx, nullptr, nullptr, n_docs, n_tokens, g.tok_offset, work);
+  g.launches += 1;
+  const int rc = g.K > kMapMinK && !(g.flags & GPULDA_FLAG_HASHMAP)
+                     ? z_launch_lists(s, zl, 65535u, (u64*)(work + kNoAllocTail), work, work + 1, work + 2)
+                     : z_launch(s, z, w, d_len, d_idx, nullptr, nullptr, n_docs, n_tokens, g.tok_offset, work, 65535u);
+  if (rc) return rc;
   CK(cudaEventRecord(g.noalloc_done, s));
   g.noalloc_pending = true;
-  g.launches += 2;
   g.tok_offset += n_tokens;
   g.swept = true;
   return GPULDA_OK;

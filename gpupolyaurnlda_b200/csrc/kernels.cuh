@@ -19,6 +19,10 @@ enum StatusBits : u32 {
 // Counter slots written by the z sweep.
 enum CounterSlots { kCtrTokens = 0, kCtrDocs = 1, kCtrSparseWork = 2, kCtrSparseDraws = 3, kCtrN = 4 };
 
+// Above this many topics a document's counts live in a list or a hash map (a
+// dense per-document count array would cost 2 K bytes of shared memory).
+constexpr u32 kMapMinK = 2048;
+
 struct ModelDev {
   u32 K, V;
   float alpha, beta;
@@ -87,6 +91,11 @@ struct ZLaunch {
   double* ll;                    // [0] sum, [1] skipped tokens (as double); may be null
   u32* work;                     // zeroed work-queue counter
   u32* status;
+  // Documents that the launch hands on: token reached << 32 | document, and
+  // their number.  The list sweep writes them, the sweep of the rest reads
+  // them in place of `order`.
+  u64* rest = nullptr;
+  u32* n_rest = nullptr;
 };
 
 // Grid sizing helpers need the device's SM count.
@@ -136,10 +145,14 @@ void launch_z_sweep_batch(const ModelDev& arenas, const BatchDev& b, u32 Kmax, c
 // false without launching when lmax needs more shared memory than a block has.
 bool launch_z_sweep_map(const ModelDev& m, const ZLaunch& z, cudaStream_t s, u32 lmax);
 u32 z_map_slots(u32 K, u32 lmax);
-// The same sweep with each document's counts as a sorted list of (topic,
-// count) pairs in shared memory (large K; the default there).
-bool launch_z_sweep_pairs(const ModelDev& m, const ZLaunch& z, cudaStream_t s, u32 lmax);
-u32 z_pairs_cap(u32 K, u32 lmax);
+// The same sweep with each document's topics as a list in a warp's registers
+// (large K; the default there).  Documents whose list outgrows kListMost
+// entries are handed on in z.rest.
+constexpr u32 kListMost = 512;
+void launch_z_sweep_pairs(const ModelDev& m, const ZLaunch& z, cudaStream_t s);
+// The rest of the documents in z.rest, none longer than lmax, lists in shared
+// memory.
+void launch_z_sweep_rest(const ModelDev& m, const ZLaunch& z, cudaStream_t s, u32 lmax);
 
 // Debug hooks.
 void launch_debug_philox(const u32* ctr, u32 n, u32 k0, u32 k1, u32* out, cudaStream_t s);

@@ -1,83 +1,292 @@
-// zsweep_pairs.cu -- the z sweep for large K with each document's topic counts
-// as a sorted list of (topic, count) pairs in shared memory (reference: the
+// zsweep_pairs.cu -- the z sweep with each document's topic counts as a sorted
+// list of (topic, count) pairs spread over a warp's registers (reference: the
 // per-document HashMap of src/cu/hashmap.cuh:13-334 used by sample_topics,
 // src/cu/topics.cu:36-105).
 //
-// The list is the order-preserving map of zsweep_map.cu without empty slots:
-// entries (topic << 16 | count), ascending topic.  A topic whose count falls
-// to zero stays as a dead entry (zero mass, so it never changes B or the
-// selected topic) and is revived if the topic returns; more than kPairsMaxDead
-// dead entries are compacted away.  Lookups are warp-cooperative 32-ary searches
-// (two ballot rounds for lists up to 1024 entries); inserts shift the tail.
-// The walk reads the entries in ascending topic order, so the sparse draw is
-// identical to the dense-count kernel's, the map kernel's and the CPU
-// oracle's.
+// One warp per document, 32 tokens at a time.  Before a chunk's first draw the
+// list is made anew in shared memory: the topics with a count, and the topics
+// that the chunk's dense draws would take, which the alias tables give before
+// the draws' order matters.  A sparse draw takes a topic of the document, so no
+// topic outside this list can come in during the chunk: the list stands still,
+// its entries live in registers (lane l holds the l-th contiguous run, so lane
+// order then slot is ascending topic order), and the gathers of q for the next
+// token are issued before the current one is drawn.  Entries whose count is
+// zero are not gathered, except the dense topic of the draw in flight.
 //
-// Per token the warp walks (i) the document's entries, gathering q[w][k]
-// (counts come with the entries), or (ii) the word's list of nonzero q, each
-// lane finding its topics' counts by binary search in the document's entries,
-// whichever is cheaper (below).  Lane l takes the l-th contiguous chunk of the walked
-// list; chunks of at most 4 elements keep their masses in registers, so the
-// sparse selection needs no second pass.
+// What bounds it: the gathers.  A document's topics lie in different sectors of
+// a word's row (40 KB at K=10000), most of them in HBM: 61 sectors a token at
+// 5.4 TB/s of DRAM traffic (K=10000, V=30000, 3e5 documents of 80 tokens), 225
+// instructions a token.  That sweep takes 13.4 ms; with the list in shared
+// memory, searched and shifted at every draw (430 instructions), it took 25.3
+// ms.  Documents in device memory at K=4096 (2e4 documents of up to 5000
+// tokens, no lengths on the host), whose lists had to be sized for K entries
+// each, 5.8 against 26 ms.
 //
-// Capacity per warp: min(lmax, K) live entries, at most kPairsMaxDead + 1
-// dead ones before a compaction, rounded up: min(lmax, K) + 64.  An insert that would pass it is
-// refused and reported (it cannot happen under that bound).
+// A list in registers holds at most kListMost entries.  A document that outgrows
+// it is handed on with the token it stands at (its earlier tokens' new topics
+// are in z) to a second kernel, whose lists stay in shared memory: the list
+// standing still during a chunk, the positions of the tokens' topics and of
+// their dense draws' topics are looked up before the chunk's first draw, and a
+// draw changes two counts in place.
 #include <algorithm>
 #include <cmath>
 
 #include "kernels.cuh"
 #include "warp.cuh"
 
-namespace {
-// Dead entries tolerated before a compaction: each costs every walk of the
-// document's entries one zero-mass element, a compaction one pass.  At
-// K=10000 (D = 2e6) 8 gave 129 ms per sweep against 133 ms for 16 and 141 ms
-// for 32.
-constexpr unsigned kPairsMaxDead = 8;
-}  // namespace
-
 namespace gpulda {
 
 namespace {
 
 constexpr u32 kMaxDocLen = 65535u;
-constexpr size_t kTokStageBytes = 32 * 32;  // per warp: 32 tokens x 32 bytes
-constexpr u32 kStatusListFull = 32;         // an insert found the list full (cannot happen)
+constexpr u32 kStatusListFull = 32;  // a list sized for its document was too small (cannot happen)
+constexpr u32 kNone = 0xffffu;     // no topic (topics are below 32768)
+constexpr u32 kSparseBit = 0x8000u;
 
-struct PairArgs {
+// Shared memory per warp: the list (topic << 16 | count, `cap` entries), the
+// positions of a merge's new entries, the chunk's staged tokens (32 bytes each,
+// and one behind them), and for lists that stay there the q values of the
+// current token's and the next one's word at the list's topics.
+struct WarpMem {
+  u32* list;
+  u32* q;  // 2 x cap
+  u32* at;
+  uint4* stage;
+  u32 cap;
+};
+
+__host__ __device__ inline size_t warp_mem_bytes(u32 cap, bool with_q) {
+  return (((size_t)cap * (with_q ? 12 : 4) + 15) & ~(size_t)15) + 32 * 4 + 66 * 16;
+}
+
+__device__ __forceinline__ WarpMem warp_mem_at(unsigned char* base, u32 cap) {
+  WarpMem wm;
+  wm.stage = (uint4*)base;
+  wm.at = (u32*)(wm.stage + 66);
+  wm.list = wm.at + 32;
+  wm.q = wm.list + cap;
+  wm.cap = cap;
+  return wm;
+}
+
+struct ListArgs {
   ModelDev m;
   ZLaunch z;
-  u32 cap;       // entries per warp
-  u32 lmax;      // longest document this launch accepts
+  u32 cap;       // entries of a list
   double lg_Ka;  // lgamma(K * alpha)
   double lg_a;   // lgamma(alpha)
 };
 
-__device__ __forceinline__ u32 topic_of(u32 e) { return e >> 16; }
-__device__ __forceinline__ u32 count_of(u32 e) { return e & 0xffffu; }
-
-// First index i in P[0..n) with topic(P[i]) >= k (warp-cooperative).
-__device__ __forceinline__ u32 pairs_lower_bound(const u32* P, u32 n, u32 k, u32 lane) {
-  u32 lo = 0;
-  while (n > 32) {
-    const u32 step = (n + 31) >> 5;
-    const bool lt = lane * step < n && topic_of(P[lo + lane * step]) < k;
-    u32 c = __popc(__ballot_sync(kFullMask, lt));
-    if (c == 0) c = 1;
-    lo += (c - 1) * step;
-    n = min(step, n - (c - 1) * step);
-  }
-  const bool lt = lane < n && topic_of(P[lo + lane]) < k;
-  return lo + __popc(__ballot_sync(kFullMask, lt));
+// Inclusive scan of u64 over the warp: the shuffle's own predicate guards the
+// two-word add.
+__device__ __forceinline__ u64 scan64(u64 x) {
+#pragma unroll
+  for (u32 o = 1; o < 32; o <<= 1)
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .u32 a0, a1, b0, b1;\n\t"
+        "mov.b64 {a0, a1}, %0;\n\t"
+        "shfl.sync.up.b32 b0|p, a0, %1, 0, 0xffffffff;\n\t"
+        "shfl.sync.up.b32 b1, a1, %1, 0, 0xffffffff;\n\t"
+        "@p add.cc.u32 a0, a0, b0;\n\t"
+        "@p addc.u32 a1, a1, b1;\n\t"
+        "mov.b64 %0, {a0, a1};\n\t"
+        "}"
+        : "+l"(x)
+        : "r"(o));
+  return x;
 }
 
-// First index i in P[0..n) with topic(P[i]) >= k, by one lane's binary search.
-__device__ __forceinline__ u32 pairs_find(const u32* P, u32 n, u32 k) {
+// Integers below 2^52 as doubles, exactly: the integer is the low mantissa of
+// 2^52, which is subtracted again.
+__device__ __forceinline__ double exact_double(u64 x) {
+  return __dadd_rn(__hiloint2double((int)(0x43300000u | (u32)(x >> 32)), (int)(u32)x), -4503599627370496.0);
+}
+
+// The mixture test u * (alpha A + B) < B in double, alpha A rounded once; u = r /
+// 2^32, exactly, by the same way from 2^20.  B is below 2^48 (65535 tokens of
+// mass below 2^32).
+__device__ __forceinline__ bool sparse_test(u32 r, double aA, u64 B) {
+  const double b = exact_double(B);
+  const double u = __dadd_rn(__hiloint2double(0x41300000, (int)r), -1048576.0);
+  return __dmul_rn(u, __dadd_rn(aA, b)) < b;
+}
+
+__device__ __forceinline__ u32 scan32(u32 x, u32 lane) {
+#pragma unroll
+  for (u32 o = 1; o < 32; o <<= 1) {
+    const u32 y = __shfl_up_sync(kFullMask, x, o);
+    x += lane >= o ? y : 0u;
+  }
+  return x;
+}
+
+// The warp's 32 keys in ascending order by lane (bitonic network).
+__device__ __forceinline__ u32 sort32(u32 key, u32 lane) {
+#pragma unroll
+  for (u32 size = 2; size <= 32; size <<= 1) {
+#pragma unroll
+    for (u32 o = size >> 1; o > 0; o >>= 1) {
+      const u32 other = __shfl_xor_sync(kFullMask, key, o);
+      const bool low = ((lane & o) == 0) == ((lane & size) == 0 || size == 32);
+      key = low ? min(key, other) : max(key, other);
+    }
+  }
+  return key;
+}
+
+// Adds the lanes' topics (kNone: none) to the sorted list of n entries:
+// `weight` per lane to the topic's count, with a new entry where there is none.
+// Returns the new length; if that would pass the list's capacity, no entry is
+// added and the length that was needed is returned.
+static __device__ __noinline__ u32 list_merge(const WarpMem wm, u32 n, u32 topic, u32 weight, u32 lane) {
+  u32* list = wm.list;
+  const u32 c = sort32(topic, lane);
+  const u32 prev = __shfl_up_sync(kFullMask, c, 1);
+  const bool head = c != kNone && (lane == 0 || c != prev);
+  const u32 heads = __ballot_sync(kFullMask, head);
+  const u32 valid = __popc(__ballot_sync(kFullMask, c != kNone));
+  u32 pos = 0;
+  bool fresh = false;
+  u32 count = 0;
+  if (head) {
+    const u32 later = lane == 31 ? 0u : heads >> (lane + 1);  // heads behind this one
+    count = weight * ((later ? lane + (u32)__ffs((int)later) : valid) - lane);
+    u32 hi = n;
+    while (pos < hi) {  // first entry with a topic >= c
+      const u32 mid = (pos + hi) >> 1;
+      if (list[mid] >> 16 < c)
+        pos = mid + 1;
+      else
+        hi = mid;
+    }
+    fresh = pos == n || list[pos] >> 16 != c;
+    if (!fresh) list[pos] += count;
+  }
+  __syncwarp();
+  const u32 news = __ballot_sync(kFullMask, fresh);
+  const u32 nn = __popc(news);
+  if (n + nn > wm.cap || !nn) return n + nn;
+  const u32 rank = __popc(news & ((1u << lane) - 1u));
+  if (fresh) wm.at[rank] = pos;
+  // An entry moves up by the number of new entries before it.  From the top
+  // down, 32 entries at a time: what a round writes lies at or above what the
+  // rounds after it read, and a round reads before it writes.
+  for (u32 b = (n - 1) & ~31u; n && b < n; b -= 32) {
+    __syncwarp();
+    const u32 e = b + lane;
+    const u32 v = e < n ? list[e] : 0u;
+    u32 lo = 0, hi = nn;
+    while (lo < hi) {  // new entries at positions <= e
+      const u32 mid = (lo + hi) >> 1;
+      if (wm.at[mid] <= e)
+        lo = mid + 1;
+      else
+        hi = mid;
+    }
+    __syncwarp();
+    if (e < n) list[e + lo] = v;
+  }
+  __syncwarp();
+  if (fresh) list[pos + rank] = (c << 16) | count;
+  __syncwarp();
+  return n + nn;
+}
+
+// The draws of the chunk's nt tokens over the list of n entries, at most R per
+// lane.  Drawn topics go to stage[2 j].x (kSparseBit beside them), the distinct
+// topics without the token to stage[2 j].y.  The list in shared
+// memory is left with the live entries; their number is returned.
+template <u32 R>
+__device__ __forceinline__ u32 list_chunk(const WarpMem& wm, u32 n, u32 nt, u32 nz, u32 lane) {
+  const u32 per = (n + 31) >> 5;
+  u32 tp[R], ct[R], qn[R];
+#pragma unroll
+  for (u32 s = 0; s < R; ++s) {
+    const u32 e = lane * per + s;
+    const u32 v = s < per && e < n ? wm.list[e] : kNone << 16;
+    tp[s] = v >> 16;
+    ct[s] = v & 0xffffu;
+    qn[s] = 0;
+  }
+  // moves a token: k in (kNone: none), z out
+  auto move = [&](u32 k, u32 z) {
+    int live = 0;
+#pragma unroll
+    for (u32 s = 0; s < R; ++s) {
+      const u32 old = ct[s];
+      if (tp[s] == k) ++ct[s];
+      if (tp[s] == z) --ct[s];
+      live += (int)min(ct[s], 1u) - (int)min(old, 1u);
+    }
+    nz += (u32)__reduce_add_sync(kFullMask, live);
+  };
+  // Staged token: topic | dense topic << 16, r0, r1, -; row of q, alpha A.
+  uint4 a = wm.stage[0], b = wm.stage[1];
+  auto fetch = [&](u32 pending) {
+    const u32* row = (const u32*)(((u64)b.y << 32) | b.x);
+#pragma unroll
+    for (u32 s = 0; s < R; ++s)
+      if (ct[s] || (tp[s] == pending && pending != kNone)) qn[s] = __ldg(row + tp[s]);
+  };
+  // (the entries of no topic have a zero count; nothing is added to or taken
+  // from them: no token has that topic)
+  fetch(kNone);
+  move(kNone - 1u, a.x & 0xffffu);
+#pragma unroll 1
+  for (u32 j = 0; j < nt; ++j) {
+    const u32 kd = a.x >> 16, r0 = a.y, r1 = a.z;
+    const double aA = __hiloint2double((int)b.w, (int)b.z);
+    u64 P[R];
+    u64 x = 0;
+#pragma unroll
+    for (u32 s = 0; s < R; ++s) {
+      x += (u64)ct[s] * qn[s];
+      P[s] = x;
+    }
+    const bool more = j + 1 < nt;
+    a = wm.stage[2 * (j + 1)];
+    b = wm.stage[2 * (j + 1) + 1];
+    if (more) fetch(kd);
+    const u64 incl = scan64(x);
+    const u64 B = __shfl_sync(kFullMask, incl, 31);
+    const bool sp = sparse_test(r0, aA, B);
+    u64 t = scale_u32(r1, B);
+    const u32 f = __popc(__ballot_sync(kFullMask, incl <= t)) & 31u;
+    t -= incl - x;
+    u32 k = tp[R - 1];
+#pragma unroll
+    for (u32 s = R - 1; s-- > 0;)
+      if (P[s] > t) k = tp[s];
+    k = __shfl_sync(kFullMask, k, f);
+    if (!sp) k = kd;
+    if (lane == 0) {
+      wm.stage[2 * j].x = k | (sp ? kSparseBit : 0u);
+      wm.stage[2 * j].y = nz;
+    }
+    move(k, more ? a.x & 0xffffu : kNone - 1u);
+  }
+  // the live entries, in order
+  u32 mine = 0;
+#pragma unroll
+  for (u32 s = 0; s < R; ++s) mine += min(ct[s], 1u);
+  const u32 incl = scan32(mine, lane);
+  __syncwarp();
+  u32 o = incl - mine;
+#pragma unroll
+  for (u32 s = 0; s < R; ++s)
+    if (ct[s]) wm.list[o++] = (tp[s] << 16) | ct[s];
+  __syncwarp();
+  return nz;
+}
+
+// Position of topic k in the sorted list (it is there).
+__device__ __forceinline__ u32 position(const u32* list, u32 n, u32 k) {
   u32 lo = 0, hi = n;
   while (lo < hi) {
     const u32 mid = (lo + hi) >> 1;
-    if (topic_of(P[mid]) < k)
+    if (list[mid] >> 16 < k)
       lo = mid + 1;
     else
       hi = mid;
@@ -85,237 +294,119 @@ __device__ __forceinline__ u32 pairs_find(const u32* P, u32 n, u32 k) {
   return lo;
 }
 
-// Count of topic k in P[0..n) by one lane's binary search.
-__device__ __forceinline__ u32 pairs_count(const u32* P, u32 n, u32 k) {
-  u32 lo = 0, hi = n;
-  while (lo < hi) {
-    const u32 mid = (lo + hi) >> 1;
-    if (topic_of(P[mid]) < k)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  return (lo < n && topic_of(P[lo]) == k) ? count_of(P[lo]) : 0u;
+__device__ __forceinline__ void copy_word_async(u32* to, const u32* from) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((u32)__cvta_generic_to_shared(to)), "l"(from)
+               : "memory");
 }
 
-// Inserts e at P[pos] in a list of n entries (warp-cooperative shift right).
-__device__ __forceinline__ void pairs_insert(u32* P, u32 n, u32 pos, u32 e, u32 lane) {
-  for (u32 top = n; top > pos; top = top > pos + 32 ? top - 32 : pos) {
-    const u32 src = top - 1 - lane;
-    const bool act = lane < top - pos;
-    const u32 v = act ? P[src] : 0u;
-    __syncwarp();
-    if (act) P[src + 1] = v;
-    __syncwarp();
+// list_chunk with the list left in shared memory, of any length.  The gathers of
+// q for the next token are asynchronous copies, so a long list's gathers are all
+// in flight at once (waiting for eight at a time, a token of a list of about
+// 700 entries took 5 us).
+static __device__ __noinline__ u32 long_chunk(const WarpMem wm, u32 n, u32 nt, u32 nz, u32 lane) {
+  u32* list = wm.list;
+  if (lane < nt) {  // the staged topics become positions
+    const u32 v = wm.stage[2 * lane].x;
+    const u32 pz = position(list, n, v & 0xffffu), pk = position(list, n, v >> 16);
+    wm.stage[2 * lane].x = pz | (pk << 16);
   }
-  if (lane == 0) P[pos] = e;
   __syncwarp();
-}
-
-// Drops dead entries (stable, in place); returns the new length.
-__device__ __forceinline__ u32 pairs_compact(u32* P, u32 n, u32 lane) {
+  const u32 per = (n + 31) >> 5;
+  const u32 e0 = min(n, lane * per), e1 = min(n, e0 + per);
+  // one token into entry `in` and one out of entry `out` (lanes 0 and 1)
+  auto move = [&](bool add, u32 in, bool del, u32 out) {
+    const bool act = !(add && del && in == out) && (lane == 0 ? add : lane == 1 && del);
+    u32* e = list + (lane == 0 ? in : out);
+    u32 c = 2;
+    if (act) {
+      c = *e & 0xffffu;
+      *e += lane == 0 ? 1u : ~0u;
+    }
+    const u32 b = __ballot_sync(kFullMask, c == lane);  // lane 0: the count was 0; lane 1: it was 1
+    nz += (b & 1u) - ((b >> 1) & 1u);
+    __syncwarp();
+  };
+  // Copies token j's q values: entries without a count are left out, but for
+  // the one that the draw in flight may fill.
+  auto fetch = [&](u32 j, u32 pending) {
+    const uint4 b = wm.stage[2 * j + 1];
+    const u32* row = (const u32*)(((u64)b.y << 32) | b.x);
+    u32* q = wm.q + (j & 1) * wm.cap;
+    for (u32 e = lane; e < n; e += 32) {
+      const u32 v = list[e];
+      if ((v & 0xffffu) || e == pending) copy_word_async(q + e, row + (v >> 16));
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(0, n);
+  move(false, 0, true, wm.stage[0].x & 0xffffu);
+  for (u32 j = 0; j < nt; ++j) {
+    const uint4 a = wm.stage[2 * j], b = wm.stage[2 * j + 1];
+    const double aA = __hiloint2double((int)b.w, (int)b.z);
+    const u32* q = wm.q + (j & 1) * wm.cap;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+    if (j + 1 < nt) fetch(j + 1, a.x >> 16);
+    u64 x = 0;
+#pragma unroll 4
+    for (u32 e = e0; e < e1; ++e) {
+      const u32 c = list[e] & 0xffffu;
+      if (c) x += (u64)c * q[e];
+    }
+    __syncwarp();
+    const u64 incl = scan64(x);
+    const u64 B = __shfl_sync(kFullMask, incl, 31);
+    const bool sp = sparse_test(a.y, aA, B);
+    u32 pos = a.x >> 16;
+    if (sp) {
+      u64 t = scale_u32(a.z, B);
+      const u32 f = __popc(__ballot_sync(kFullMask, incl <= t)) & 31u;
+      t -= __shfl_sync(kFullMask, incl - x, f);
+      // the crossing lane's run, 32 entries at a time
+      const u32 f1 = min(n, f * per + per);
+      for (u32 e = f * per; e < f1; e += 32) {
+        const u32 v = e + lane < f1 ? list[e + lane] : 0u;
+        const u64 in2 = scan64(v & 0xffffu ? (u64)(v & 0xffffu) * q[e + lane] : 0ull);
+        const u64 all = __shfl_sync(kFullMask, in2, 31);
+        if (all > t) {
+          pos = e + __popc(__ballot_sync(kFullMask, in2 <= t));
+          break;
+        }
+        t -= all;
+      }
+    }
+    const bool more = j + 1 < nt;
+    if (lane == 0) wm.stage[2 * j].x = (list[pos] >> 16) | (sp ? kSparseBit : 0u);
+    if (lane == 0) wm.stage[2 * j].y = nz;
+    move(true, pos, more, more ? wm.stage[2 * (j + 1)].x & 0xffffu : 0u);
+  }
+  // the live entries, in order
   u32 out = 0;
   for (u32 b = 0; b < n; b += 32) {
-    const u32 i = b + lane;
-    const u32 e = i < n ? P[i] : 0u;
-    const bool keep = i < n && count_of(e) != 0;
-    const u32 ball = __ballot_sync(kFullMask, keep);
+    const u32 v = b + lane < n ? list[b + lane] : 0u;
+    const u32 live = __ballot_sync(kFullMask, (v & 0xffffu) != 0);
     __syncwarp();
-    if (keep) P[out + __popc(ball & ((1u << lane) - 1u))] = e;
-    out += __popc(ball);
+    if (v & 0xffffu) list[out + __popc(live & ((1u << lane) - 1u))] = v;
+    out += __popc(live);
     __syncwarp();
   }
-  return out;
+  return nz;
 }
 
-// Count of topic k += 1 at its position; inserts it if absent.  bm (may be
-// null): the bitmap of topics with a positive count, kept in step.
-__device__ __forceinline__ void pairs_add_at(u32* P, u32& nl, u32& nz, u32 pos, u32 k, u32 cap, u32 lane,
-                                             u32* status, u32* bm) {
-  const u32 e = pos < nl ? P[pos] : 0xffffffffu;
-  __syncwarp();
-  if (pos < nl && topic_of(e) == k) {
-    if (lane == 0) {
-      P[pos] = e + 1u;
-      if (bm && count_of(e) == 0) bm[k >> 5] |= 1u << (k & 31);
-    }
-    if (count_of(e) == 0) ++nz;  // a dead entry revived
-    __syncwarp();
-    return;
-  }
-  if (nl >= cap) {
-    *status |= kStatusListFull;
-    return;
-  }
-  pairs_insert(P, nl, pos, (k << 16) | 1u, lane);
-  if (bm && lane == 0) bm[k >> 5] |= 1u << (k & 31);
-  __syncwarp();
-  ++nl;
-  ++nz;
-}
-
-// Launches whose documents are at most this long keep the topic bitmap.
-constexpr u32 kBitmapMaxLen = 1024;
-
-// Whether topic k has a positive count (always true without the bitmap: the
-// caller then searches).
-template <bool BM>
-__device__ __forceinline__ bool in_doc(const u32* bm, u32 k) {
-  return !BM || ((bm[k >> 5] >> (k & 31)) & 1u);
-}
-
-// One token's draw over the document's entries P[0..nl) (bm: the optional
-// topic bitmap) and the word's row: the walk of the shorter side split into
-// 32 contiguous chunks, chunks of at most R elements kept in registers.
-// Returns the topic; *pos_out receives its entry when the document-side walk
-// found it (else 0xffffffff).
-template <bool BM, u32 R>
-__device__ __forceinline__ u32 pairs_draw(const u32* P, u32 nl, const u32* bm, const u32* __restrict__ qrow,
-                                          const u64* __restrict__ crow, u32 nw, u64 Aw, float alpha, bool word_side,
-                                          u32 zj, u32 r0, u32 r1, u32 my_r3, u64 my_al, u32 j, u32 lane,
-                                          u32* pos_out, int* sp_out, int* degenerate_out) {
-  const u32 len = word_side ? nw : nl;
-  const u32 cper = (len + 31) >> 5;
-  const u32 e0 = min(len, lane * cper), e1 = min(len, e0 + cper);
-  const bool in_regs = cper <= R;
-  u64 ms[R];
-  u64 ls = 0;
-  if (in_regs) {
-    const u32 n_my = e1 - e0;
-    if (word_side) {
-#pragma unroll
-      for (u32 c = 0; c < R; ++c) {
-        const u64 ent = c < n_my ? __ldg(crow + e0 + c) : 0ull;
-        ms[c] = c < n_my && in_doc<BM>(bm, (u32)ent & 0xffffu)
-                    ? (u64)pairs_count(P, nl, (u32)ent & 0xffffu) * (u32)(ent >> 32)
-                    : 0ull;
-      }
-    } else {
-      u32 es[R], qs[R];
-#pragma unroll
-      for (u32 c = 0; c < R; ++c) es[c] = c < n_my ? P[e0 + c] : 0u;
-#pragma unroll
-      for (u32 c = 0; c < R; ++c) qs[c] = c < n_my ? __ldg(qrow + topic_of(es[c])) : 0u;
-#pragma unroll
-      for (u32 c = 0; c < R; ++c) ms[c] = (u64)count_of(es[c]) * qs[c];
-    }
-#pragma unroll
-    for (u32 c = 0; c < R; ++c) ls += ms[c];
-  } else if (word_side) {
-    for (u32 e = e0; e < e1; ++e) {
-      const u64 ent = __ldg(crow + e);
-      if (in_doc<BM>(bm, (u32)ent & 0xffffu))
-        ls += (u64)pairs_count(P, nl, (u32)ent & 0xffffu) * (u32)(ent >> 32);
-    }
-  } else {
-    for (u32 e = e0; e < e1; ++e) {
-      const u32 en = P[e];
-      ls += (u64)count_of(en) * __ldg(qrow + topic_of(en));
-    }
-  }
-  const u64 incl = warp_incl_scan_u64(ls, lane);
-  const u64 B = __shfl_sync(kFullMask, incl, 31);
-  int degenerate;
-  const int sp = take_sparse(r0, alpha, Aw, B, &degenerate);
-  *sp_out = sp;
-  *degenerate_out = degenerate;
-  u32 k = zj;
-  u32 pos = 0xffffffffu;  // the new topic's entry, when the walk found it
-  if (!degenerate) {
-    if (sp) {
-      const u64 target = scale_u32(r1, B);
-      const u32 f = __ffs(__ballot_sync(kFullMask, incl > target)) - 1;
-      u32 ef;
-      if (in_regs) {
-        // lane f's first element whose inclusive prefix exceeds the target
-        u64 pre = incl - ls;
-        u32 cx = R - 1;
-#pragma unroll
-        for (u32 c = R - 1; c-- > 0;) {
-          u64 t = pre;
-#pragma unroll
-          for (u32 d = 0; d <= c; ++d) t += ms[d];
-          if (t > target) cx = c;
-        }
-        ef = f * cper + __shfl_sync(kFullMask, cx, f);
-      } else {
-        u64 run = __shfl_sync(kFullMask, incl - ls, f);
-        const u32 f0 = min(len, f * cper), f1 = min(len, f0 + cper);
-        ef = f1 - 1;
-        for (u32 s0 = f0; s0 < f1; s0 += 32) {
-          const u32 e = s0 + lane;
-          u64 mass = 0;
-          if (e < f1) {
-            if (word_side) {
-              const u64 ent = __ldg(crow + e);
-              if (in_doc<BM>(bm, (u32)ent & 0xffffu))
-                mass = (u64)pairs_count(P, nl, (u32)ent & 0xffffu) * (u32)(ent >> 32);
-            } else {
-              const u32 en = P[e];
-              mass = (u64)count_of(en) * __ldg(qrow + topic_of(en));
-            }
-          }
-          const u64 in2 = warp_incl_scan_u64(mass, lane);
-          const u64 tot = __shfl_sync(kFullMask, in2, 31);
-          if (run + tot > target) {
-            ef = s0 + __ffs(__ballot_sync(kFullMask, run + in2 > target)) - 1;
-            break;
-          }
-          run += tot;
-        }
-      }
-      if (word_side) {
-        k = (u32)__ldg(crow + ef) & 0xffffu;
-      } else {
-        k = topic_of(P[ef]);
-        pos = ef;
-      }
-    } else {
-      const u32 r3 = __shfl_sync(kFullMask, my_r3, j);
-      const u64 e = __shfl_sync(kFullMask, my_al, j);
-      k = alias_pick(e, r3);
-    }
-  }
-  *pos_out = pos;
-  return k;
-}
-
-// Shared memory per warp: entries, staged token data, and the bitmap.
-__host__ __device__ __forceinline__ size_t pairs_warp_bytes(u32 cap, u32 K, bool bm) {
-  return (size_t)cap * 4 + kTokStageBytes + (bm ? ((((size_t)K + 31) / 32 * 4 + 15) & ~(size_t)15) : 0);
-}
-
-// Four blocks per SM (64 registers, no spills).  LL: the launch accumulates
-// the joint log-likelihood (a separate instantiation, so the plain sweep keeps
-// no log-likelihood registers); the statistics are per-chunk sums in one
-// register, flushed to per-block shared counters.  At K=10000 the whole
-// sweep (long-document launch, then short-document launch) takes 446 ms over
-// 8e6 documents and 109 ms over 2e6, against 483 and 131 ms at three blocks.
-//
-// BM (launches whose lists are short, lmax <= kBitmapMaxLen): each warp also
-// keeps a bitmap of the topics with a positive count.  The document's entries
-// are then built from it (bitmap of the tokens' topics, its set bits in order,
-// then one binary search and shared-memory atomic per token) instead of one
-// warp-cooperative insert per token, and a word-side walk skips the binary
-// search of every word topic absent from the document (most of them; a lane
-// slot where no lane's topic is present costs no search at all).
-template <bool LL, bool BM>
-__global__ void __launch_bounds__(256, 4) z_sweep_pairs_kernel(PairArgs a) {
+// LONG: the documents of z.rest, from the token each stands at, lists in shared
+// memory.
+template <bool LL, bool LONG>
+__global__ void __launch_bounds__(256, LONG ? 3 : 2) z_sweep_pairs_kernel(ListArgs a) {
   extern __shared__ __align__(16) unsigned char zsm[];
   __shared__ unsigned long long blk_stats[4];  // tokens, documents, sparse work, sparse draws
   if (threadIdx.x < 4) blk_stats[threadIdx.x] = 0;
   __syncthreads();
   const ModelDev& m = a.m;
   const ZLaunch& p = a.z;
-  const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const u32 lane = threadIdx.x & 31;
   const u32 K = m.K, V = m.V;
-  const u32 bmw = (K + 31) >> 5;  // bitmap words
-  unsigned char* wsm = zsm + (size_t)warp * pairs_warp_bytes(a.cap, K, BM);
-  u32* P = (u32*)wsm;
-  uint4* stage = (uint4*)(wsm + (size_t)a.cap * 4);
-  u32* bm = BM ? (u32*)(wsm + (size_t)a.cap * 4 + kTokStageBytes) : nullptr;
-  const bool want_ll = LL;
-
+  const WarpMem wm = warp_mem_at(zsm + (threadIdx.x >> 5) * warp_mem_bytes(a.cap, LONG), a.cap);
+  const u32 n_items = LONG ? *p.n_rest : p.n_docs;
   double ll_acc = 0.0, ll_skip = 0.0;
   u32 status = 0;
 
@@ -323,11 +414,18 @@ __global__ void __launch_bounds__(256, 4) z_sweep_pairs_kernel(PairArgs a) {
     u32 doc = 0;
     if (lane == 0) doc = atomicAdd(p.work, 1u);
     doc = __shfl_sync(kFullMask, doc, 0);
-    if (doc >= p.n_docs) break;
-    if (p.order) doc = p.order[doc];
+    if (doc >= n_items) break;
+    u32 start = 0;  // the tokens before it are drawn
+    if (LONG) {
+      const u64 item = p.rest[doc];
+      doc = (u32)item;
+      start = (u32)(item >> 32);
+    } else if (p.order) {
+      doc = p.order[doc];
+    }
     const u32 L = p.d_len[doc];
     const u64 off = p.d_idx[doc];
-    if (L > kMaxDocLen || L > a.lmax) {
+    if (L > kMaxDocLen) {
       status |= kStatusDocTooLong;
       continue;
     }
@@ -335,140 +433,96 @@ __global__ void __launch_bounds__(256, 4) z_sweep_pairs_kernel(PairArgs a) {
       status |= kStatusDocRange;
       continue;
     }
-    // build the sorted entries of the document's topics
-    u32 nl = 0, nz = 0;
-    if (BM) {
-      for (u32 i = lane; i < bmw; i += 32) bm[i] = 0;
-      __syncwarp();
-      for (u32 i = lane; i < L; i += 32) {
-        u32 k = p.z[off + i];
-        if (k >= K) {
-          status |= kStatusBadTopic;
-          k %= K;
-        }
-        atomicOr(bm + (k >> 5), 1u << (k & 31));
-      }
-      __syncwarp();
-      // the set bits in ascending order, 32 words per round
-      for (u32 b = 0; b < bmw; b += 32) {
-        const u32 wi = b + lane;
-        u32 bits = wi < bmw ? bm[wi] : 0u;
-        const u32 c = __popc(bits);
-        u32 x = c;
-#pragma unroll
-        for (u32 o = 1; o < 32; o <<= 1) {
-          const u32 y = __shfl_up_sync(kFullMask, x, o);
-          if (lane >= o) x += y;
-        }
-        u32 pos = nl + x - c;
-        while (bits) {
-          P[pos++] = (wi * 32 + (u32)(__ffs(bits) - 1)) << 16;
-          bits &= bits - 1;
-        }
-        nl += __shfl_sync(kFullMask, x, 31);
-      }
-      __syncwarp();
-      // counts: one binary search and shared-memory atomic per token
-      for (u32 i = lane; i < L; i += 32) {
-        const u32 k = p.z[off + i] % K;
-        atomicAdd(P + pairs_find(P, nl, k), 1u);
-      }
-      __syncwarp();
-      nz = nl;
-    } else {
-      for (u32 i = 0; i < L; ++i) {
-        u32 k = p.z[off + i];
-        if (k >= K) {
-          status |= kStatusBadTopic;
-          k %= K;
-        }
-        pairs_add_at(P, nl, nz, pairs_lower_bound(P, nl, k, lane), k, a.cap, lane, &status, nullptr);
-      }
-    }
-
-    for (u32 base = 0; base < L; base += 32) {
-      const u32 i = base + lane;
-      const bool valid = i < L;
-      u32 my_w = valid ? p.w[off + i] : 0;
-      u32 my_z = valid ? p.z[off + i] : 0;
-      if (my_w >= V) {
+    const u32* w = p.w + off;
+    u32* z = p.z + off;
+    auto word = [&](u32 base) {
+      u32 x = base + lane < L ? w[base + lane] : 0u;
+      if (x >= V) {
         status |= kStatusBadWord;
-        my_w %= V;
+        x %= V;
       }
-      if (my_z >= K) my_z %= K;
-      const U4 r = draw4(p.tok_base + off + i, p.t, kStreamZ, 0, m.key0, m.key1);
-      const u32 my_nw = valid ? __ldg(m.nnz + my_w) : 0u;
-      const u64 my_A = valid ? __ldg(m.A + my_w) : 0ull;
-      const u32 my_s = (u32)(((u64)r.z * my_nw) >> 32);
-      const u64 my_row = (u64)my_w * K;
-      const u64 my_al = (valid && my_nw) ? __ldg(m.al + my_row + my_s) : 0ull;
-      u32 new_z = my_z;
-      const u32 nt = min(32u, L - base);
-      // sum over the chunk of (min(nz without the token, nnz[w]) << 6) + sparse
-      // (the first term at most 32 * 32768, the second at most 32)
-      u32 chunk_st = 0;
+      return x;
+    };
+    auto topic = [&](u32 base) {
+      u32 k = base + lane < L ? z[base + lane] : kNone;
+      if (base + lane < L && k >= K) {
+        status |= kStatusBadTopic;
+        k %= K;
+      }
+      return k;
+    };
+    // the words of the first chunks are on their way while the list is built
+    // (word data two chunks ahead, alias entries and topics one ahead)
+    u32 w1 = word(start), w2 = word(start + 32), w3 = word(start + 64);
+    u32 nw1 = __ldg(m.nnz + w1), nw2 = __ldg(m.nnz + w2);
+    u64 A1 = __ldg(m.A + w1), A2 = __ldg(m.A + w2);
+    u32 n = 0;
+    for (u32 base = 0; base < L && n <= a.cap; base += 32) n = list_merge(wm, n, topic(base), 1u, lane);
+    u32 nz = n, work = 0, n_sparse = 0;
+    // the first chunk's topics, Philox words and alias entries
+    u32 z1 = topic(start);
+    U4 r = draw4(p.tok_base + off + start + lane, p.t, kStreamZ, 0, m.key0, m.key1);
+    auto alias = [&](u32 base, u32 wd, u32 nw, u32 r2) {
+      return base + lane < L && nw ? __ldg(m.al + (u64)wd * K + (u32)(((u64)r2 * nw) >> 32)) : 0ull;
+    };
+    u64 al = alias(start, w1, nw1, r.z);
+    bool over = n > a.cap;
+    while (!over && start < L) {
+      const u32 base = start, nt = min(32u, L - base);
+      const bool valid = lane < nt;
+      // a word whose every q is zero keeps the token's topic: nothing else has
+      // mass, and its dense draw is that topic
+      const u32 kd = !valid ? kNone : nw1 ? alias_pick(al, r.w) : z1;
+      n = list_merge(wm, nz, kd, 0u, lane);
+      if (n > a.cap) {
+        over = true;
+        break;
+      }
+      const u64 my_row = (u64)w1 * K;
+      const u32 my_nw = nw1;
+      {
+        const u64 aA = (u64)__double_as_longlong(__dmul_rn((double)m.alpha, exact_double(A1)));
+        const u64 row = (u64)(m.q + my_row);
+        wm.stage[2 * lane] = make_uint4(z1 | (kd << 16), r.x, r.y, 0);
+        wm.stage[2 * lane + 1] = make_uint4((u32)row, (u32)(row >> 32), (u32)aA, (u32)(aA >> 32));
+      }
       __syncwarp();
-      stage[2 * lane] = make_uint4(my_z, r.x, r.y, my_nw);
-      stage[2 * lane + 1] = make_uint4((u32)my_row, (u32)(my_row >> 32), (u32)my_A, (u32)(my_A >> 32));
-      __syncwarp();
-      for (u32 j = 0; j < nt; ++j) {
-        const uint4 s0 = stage[2 * j], s1 = stage[2 * j + 1];
-        const u32 zj = s0.x, r0 = s0.y, r1 = s0.z, nw = s0.w;
-        const size_t row = ((u64)s1.y << 32) | s1.x;
-        const u64 Aw = ((u64)s1.w << 32) | s1.z;
-        const u32* __restrict__ qrow = m.q + row;
-        const u64* __restrict__ crow = m.csr + row;
-        // remove the token's current topic (present with a positive count)
-        {
-          const u32 pz = pairs_lower_bound(P, nl, zj, lane);
-          const u32 e = pz < nl ? P[pz] : 0u;
-          __syncwarp();
-          if (pz < nl && topic_of(e) == zj && count_of(e) > 0) {
-            if (lane == 0) {
-              P[pz] = e - 1u;
-              if (BM && count_of(e) == 1) bm[zj >> 5] &= ~(1u << (zj & 31));
-            }
-            if (count_of(e) == 1) --nz;
-          }
-          __syncwarp();
-        }
-        // The word's list is read contiguously while the document side
-        // gathers scattered q values from rows of 4 K bytes (mostly beyond L2 at
-        // large K), so the word side is taken up to 4x the document's length
-        // (measured best at K=10000 among 1x, 2x, 4x, 8x; again with the
-        // topic bitmap, on 2e6 documents: 103 ms per sweep against 116 for
-        // 2x, 115 for 8x and 126 for 16x).
-        const bool word_side = nw < 4 * nl;
-        // as few register slots as the walk's chunks need: 2, 4 or 6 (K=10000,
-        // 2e6 documents: 101.8 ms per sweep against 102.9 with 2 or 4; an 8-slot
-        // path beside them spilled and took 108.4)
-        const u32 cper_j = ((word_side ? nw : nl) + 31) >> 5;
-        u32 pos;
-        int sp, degenerate;
-        u32 k = cper_j <= 2 ? pairs_draw<BM, 2>(P, nl, bm, qrow, crow, nw, Aw, m.alpha, word_side, zj, r0, r1, r.w, my_al,
-                                                 j, lane, &pos, &sp, &degenerate)
-                : cper_j <= 4 ? pairs_draw<BM, 4>(P, nl, bm, qrow, crow, nw, Aw, m.alpha, word_side, zj, r0, r1, r.w, my_al,
-                                                 j, lane, &pos, &sp, &degenerate)
-                            : pairs_draw<BM, 6>(P, nl, bm, qrow, crow, nw, Aw, m.alpha, word_side, zj, r0, r1, r.w, my_al,
-                                                 j, lane, &pos, &sp, &degenerate);
-        const u32 nzm = nz;
-        if (pos == 0xffffffffu) pos = pairs_lower_bound(P, nl, k, lane);
-        pairs_add_at(P, nl, nz, pos, k, a.cap, lane, &status, bm);
-        if (nl - nz > kPairsMaxDead) nl = pairs_compact(P, nl, lane);
-        if (lane == 0) {
-          atomicAdd(m.n + row + k, 1u);
-          chunk_st += (min(nzm, nw) << 6) + ((sp && !degenerate) ? 1u : 0u);
-        }
-        if (lane == j) new_z = k;
-        __syncwarp();
-      }
-      if (lane == 0) {
-        atomicAdd(blk_stats + 2, (unsigned long long)(chunk_st >> 6));
-        atomicAdd(blk_stats + 3, (unsigned long long)(chunk_st & 63u));
-      }
+      // the chunks ahead
+      w1 = w2;
+      nw1 = nw2;
+      A1 = A2;
+      z1 = topic(base + 32);
+      r = draw4(p.tok_base + off + base + 32 + lane, p.t, kStreamZ, 0, m.key0, m.key1);
+      al = alias(base + 32, w1, nw1, r.z);
+      w2 = w3;
+      nw2 = __ldg(m.nnz + w2);
+      A2 = __ldg(m.A + w2);
+      w3 = word(base + 96);
+      const u32 per = (n + 31) >> 5;
+      if (LONG)
+        n = long_chunk(wm, n, nt, nz, lane);
+      else if (per <= 2)
+        n = list_chunk<2>(wm, n, nt, nz, lane);
+      else if (per == 3)
+        n = list_chunk<3>(wm, n, nt, nz, lane);
+      else if (per == 4)
+        n = list_chunk<4>(wm, n, nt, nz, lane);
+      else if (per <= 6)
+        n = list_chunk<6>(wm, n, nt, nz, lane);
+      else if (per <= 8)
+        n = list_chunk<8>(wm, n, nt, nz, lane);
+      else
+        n = list_chunk<16>(wm, n, nt, nz, lane);
+      nz = n;
+      const u32 res = wm.stage[2 * lane].x, my_nz = wm.stage[2 * lane].y;
+      const u32 new_z = res & 0x7fffu;
+      const bool sp = valid && (res & kSparseBit);
+      work += __reduce_add_sync(kFullMask, valid ? min(my_nz, my_nw) : 0u);
+      n_sparse += __popc(__ballot_sync(kFullMask, sp));
       if (valid) {
-        p.z[off + i] = new_z;
-        if (want_ll) {  // log Phi[new topic][word], one token per lane
+        z[base + lane] = new_z;
+        atomicAdd(m.n + my_row + new_z, 1u);
+        if (LL) {  // log Phi[new topic][word], one token per lane
           const u32 qk = __ldg(m.q + my_row + new_z);
           if (qk)
             ll_acc += log((double)qk) - 22.18070977791825;  // 32 log 2
@@ -476,14 +530,24 @@ __global__ void __launch_bounds__(256, 4) z_sweep_pairs_kernel(PairArgs a) {
             ll_skip += 1.0;
         }
       }
+      start = base + nt;
+      __syncwarp();
+    }
+    if (lane == 0) {
+      atomicAdd(blk_stats + 2, (unsigned long long)work);
+      atomicAdd(blk_stats + 3, (unsigned long long)n_sparse);
+    }
+    if (over) {  // the rest of the document is the other kernel's (whose lists are long enough)
+      if (LONG)
+        status |= kStatusListFull;
+      else if (lane == 0) p.rest[atomicAdd(p.n_rest, 1u)] = (u64)start << 32 | doc;
+      __syncwarp();
+      continue;
     }
     if (lane == 0 && p.K_d) p.K_d[doc] = nz;
-    if (want_ll) {
+    if (LL) {
       double dl = 0.0;
-      for (u32 e = lane; e < nl; e += 32) {
-        const u32 c = count_of(P[e]);
-        if (c) dl += lgamma((double)m.alpha + (double)c) - a.lg_a;
-      }
+      for (u32 e = lane; e < nz; e += 32) dl += lgamma((double)m.alpha + (double)(wm.list[e] & 0xffffu)) - a.lg_a;
       dl = warp_sum_f64(dl);
       if (lane == 0) ll_acc += dl + a.lg_Ka - lgamma((double)K * (double)m.alpha + (double)L);
     }
@@ -493,13 +557,13 @@ __global__ void __launch_bounds__(256, 4) z_sweep_pairs_kernel(PairArgs a) {
     }
     __syncwarp();
   }
-  if (want_ll) {
+  if (LL) {
     ll_acc = warp_sum_f64(ll_acc);
     ll_skip = warp_sum_f64(ll_skip);
-  }
-  if (lane == 0 && want_ll) {
-    atomicAdd(p.ll, ll_acc);
-    atomicAdd(p.ll + 1, ll_skip);
+    if (lane == 0) {
+      atomicAdd(p.ll, ll_acc);
+      atomicAdd(p.ll + 1, ll_skip);
+    }
   }
   status = __reduce_or_sync(kFullMask, status);
   if (lane == 0 && status) atomicOr(p.status, status);
@@ -514,36 +578,38 @@ __global__ void __launch_bounds__(256, 4) z_sweep_pairs_kernel(PairArgs a) {
 
 }  // namespace
 
-u32 z_pairs_cap(u32 K, u32 lmax) { return ((std::min(std::max(lmax, 1u), K) + 64 + 31) / 32) * 32; }
+namespace {
 
-bool launch_z_sweep_pairs(const ModelDev& m, const ZLaunch& z, cudaStream_t s, u32 lmax) {
-  if (!z.n_docs) return true;
-  PairArgs a;
+template <bool LONG>
+void launch_lists(const ModelDev& m, const ZLaunch& z, cudaStream_t s, u32 cap) {
+  if (!z.n_docs) return;
+  ListArgs a;
   a.m = m;
   a.z = z;
-  a.lmax = lmax;
-  a.cap = z_pairs_cap(m.K, lmax);
+  a.cap = cap;
   a.lg_a = std::lgamma((double)m.alpha);
   a.lg_Ka = std::lgamma((double)m.K * (double)m.alpha);
-  const bool bmap = lmax <= kBitmapMaxLen;
-  const size_t per_warp = pairs_warp_bytes(a.cap, m.K, bmap);
+  auto kern = (z.flags & kZFlagLoglik) && z.ll ? z_sweep_pairs_kernel<true, LONG> : z_sweep_pairs_kernel<false, LONG>;
   constexpr size_t kBudget = 200 * 1024;
-  u32 wpb = 8;
-  while (wpb > 1 && per_warp * wpb > kBudget) --wpb;
-  if (per_warp * wpb > kBudget) return false;
-  const size_t smem = per_warp * wpb;
-  const bool ll = (z.flags & 1u) && z.ll;
-  auto kern = bmap ? (ll ? z_sweep_pairs_kernel<true, true> : z_sweep_pairs_kernel<false, true>)
-                   : (ll ? z_sweep_pairs_kernel<true, false> : z_sweep_pairs_kernel<false, false>);
-  if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBudget);
+  u32 warps = 8;
+  while (warps > 1 && warps * warp_mem_bytes(cap, LONG) > kBudget) --warps;
+  const size_t smem = warps * warp_mem_bytes(cap, LONG);
+  if (smem > 47 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBudget);
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * wpb, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem);
   if (per_sm < 1) per_sm = 1;
-  u32 blocks = (u32)(device_sm_count() * per_sm);
-  const u32 need = (z.n_docs + wpb - 1) / wpb;
-  if (blocks > need) blocks = need;
-  kern<<<blocks, 32 * wpb, smem, s>>>(a);
-  return true;
+  const u32 blocks = std::min<u32>((u32)(device_sm_count() * per_sm), (z.n_docs + warps - 1) / warps);
+  kern<<<blocks, 32 * warps, smem, s>>>(a);
+}
+
+}  // namespace
+
+void launch_z_sweep_pairs(const ModelDev& m, const ZLaunch& z, cudaStream_t s) {
+  launch_lists<false>(m, z, s, kListMost);
+}
+
+void launch_z_sweep_rest(const ModelDev& m, const ZLaunch& z, cudaStream_t s, u32 lmax) {
+  launch_lists<true>(m, z, s, std::min(std::max(lmax, 1u), m.K) + 32);
 }
 
 }  // namespace gpulda

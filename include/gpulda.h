@@ -266,7 +266,7 @@ int gpulda_debug_alias(const uint32_t* q, uint32_t K, uint64_t* table_out);
  * one after another from the host are ordered on the GPU as well.
  *
  * It allocates nothing: its scratch (document offsets and a work counter) is
- * a fixed device array of the library, 4 MiB + 256 B held by every GPU that
+ * a fixed device array of the library, 12 MiB + 256 B held by every GPU that
  * loads the library until the process exits.  n_docs above
  * GPULDA_NOALLOC_MAX_DOCS is rejected with GPULDA_ERR_UNSUPPORTED.  The first
  * call on a device looks up that array's address, so make the first call
