@@ -25,7 +25,8 @@ NVCC_FLAGS = ARCH + [
     "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off",
     "-Xptxas", "-v",
 ]
-LIB_SOURCES = ["gpulda.cu", "kernels.cu", "zsweep.cu", "zsweep_map.cu", "batch.cu", "serve.cu", "zsweep_pairs.cu"]
+LIB_SOURCES = ["gpulda.cu", "kernels.cu", "zsweep.cu", "zsweep_map.cu", "batch.cu", "serve.cu", "zsweep_pairs.cu",
+               "zsweep_words.cu"]
 
 
 def _stale(target: str, deps: list[str]) -> bool:

@@ -64,11 +64,13 @@ __global__ void add_u32_kernel(u32* p, u64 n, u32 add) {
   for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x) p[i] += add;
 }
 
-// Per global word w0 + i (i < V): its problem slot and row start.
-__global__ void word_rows_kernel(u32* wpid, u64* row_off, u32 w0, u32 V, u32 slot, u64 cell0, u32 K) {
+// Per global word w0 + i (i < V): its problem slot, row start and list start.
+__global__ void word_rows_kernel(u32* wpid, u64* row_off, u64* list_off, u32 w0, u32 V, u32 slot, u64 cell0,
+                                 u64 list0, u32 K) {
   for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += gridDim.x * blockDim.x) {
     wpid[w0 + i] = slot;
     row_off[w0 + i] = cell0 + (u64)i * K;
+    list_off[w0 + i] = list0 + (u64)i * list_stride(K);
   }
 }
 
@@ -90,6 +92,7 @@ struct Bucket {
   u32 doc0 = 0, doc1 = 0;     // global documents
   u64 tok0 = 0, tok1 = 0;     // global tokens
   u32 block0 = 0, n_blocks = 0;  // Poisson-draw block table section
+  u32 n_chain = 0;            // documents of its order that take a warp each
   bool want_ll = false;
   GpuldaBatchShape shape{8, 0, 65536, 0};
   cudaStream_t s = nullptr;
@@ -102,12 +105,16 @@ struct Slot {  // one problem, in arena order
   float alpha, beta;
   u32 key0, key1, flags;
   u64 n_tokens;
-  u64 cell0, S0, tok0;
+  u64 cell0, list0, S0, tok0;
   u32 word0, doc0;
 };
 
-// Index of the merged launches' work counter (after the buckets').
+// Index of the merged launches' work counters and shares (after the buckets').
 constexpr u32 kMergedWork = GPULDA_BATCH_BUCKETS;
+// Shares of words with short and long lists, two per bucket and for the merged
+// launches, behind the topic sums: an alias build adds to those of the sweep
+// that follows it, so nothing writes them while that sweep's launches choose.
+constexpr u32 kShares = 2 * (GPULDA_BATCH_BUCKETS + 1);
 
 struct Batch {
   u32 P = 0;
@@ -133,7 +140,9 @@ struct Batch {
   ModelDev ar{};
   u32 *z = nullptr, *w = nullptr, *d_len = nullptr, *d_idx = nullptr, *order = nullptr;
   u32 *pid = nullptr, *wpid = nullptr;
-  u64 *row_off = nullptr;
+  u64 *row_off = nullptr, *list_off = nullptr;
+  u32 lmax = 0;         // longest document
+  u32 n_chain = 0;      // documents of order_all that take a warp each
   u32 *K = nullptr, *key0 = nullptr, *key1 = nullptr;
   float *alpha = nullptr, *beta = nullptr;
   u64 *tok_base = nullptr, *cell_base = nullptr, *S_off = nullptr;
@@ -166,10 +175,17 @@ struct Batch {
   }
 
   BatchDev zdev() const {
-    return BatchDev{pid, row_off, K, alpha, key0, key1, tok_base, lg_a, lg_Ka};
+    return BatchDev{pid, row_off, list_off, K, alpha, key0, key1, tok_base, lg_a, lg_Ka};
   }
   BatchPhiDev phidev(u32 block0) const {
-    return BatchPhiDev{blocks + block0, K, cell_base, S_off, beta, key0, key1, wpid, row_off, cdf, guide, lfac};
+    return BatchPhiDev{blocks + block0, K, cell_base, S_off, beta, key0, key1, wpid, row_off, list_off, cdf, guide, lfac};
+  }
+
+  // The arenas with the shares of bucket j's (or the merged) launches.
+  ModelDev arena(u32 j) const {
+    ModelDev m = ar;
+    m.shares = ar.S + S_total + 2 * j;
+    return m;
   }
 
   void drop_graph() {
@@ -254,7 +270,7 @@ ZLaunch z_args(const Batch& b, u32 j, unsigned long long* counters, double* ll) 
   zl.flags = bu.want_ll ? 1u : 0u;
   zl.counters = counters;
   zl.ll = ll;
-  zl.work = b.work + j;
+  zl.work = nullptr;
   zl.status = b.status;
   return zl;
 }
@@ -265,17 +281,34 @@ ZLaunch z_args_merged(const Batch& b, unsigned long long* counters, double* ll) 
   zl.order = b.order_all;
   zl.n_docs = b.D;
   zl.flags = b.want_ll_all ? 1u : 0u;
-  zl.work = b.work + kMergedWork;
   return zl;
 }
 
-// One launch per stage over every problem on stream s (work counter zeroed by
-// the caller).
+// The z sweeps of bucket j's documents and of every document (counters zeroed
+// by the caller).
+void bucket_sweep(const Batch& b, u32 j, unsigned long long* counters, double* ll, const GpuldaBatchShape& shape,
+                  cudaStream_t s) {
+  const Bucket& bu = b.bk[j];
+  const BatchDev bd = b.zdev();
+  launch_sweep(b.arena(j), &bd, bu.Kmax, z_args(b, j, counters, ll),
+               SweepAux{b.work + j * kSweepCtrs, nullptr, b.lmax, bu.n_chain}, s, shape.z_warps_per_block,
+               shape.z_blocks_per_sm);
+}
+
+void merged_sweep(const Batch& b, unsigned long long* counters, double* ll, const GpuldaBatchShape& shape,
+                  cudaStream_t s) {
+  const BatchDev bd = b.zdev();
+  launch_sweep(b.arena(kMergedWork), &bd, b.Kmax_all, z_args_merged(b, counters, ll),
+               SweepAux{b.work + kMergedWork * kSweepCtrs, nullptr, b.lmax, b.n_chain}, s, shape.z_warps_per_block,
+               shape.z_blocks_per_sm);
+}
+
+// One launch per stage over every problem on stream s (counters zeroed by the
+// caller).
 void merged_iteration(const Batch& b, cudaStream_t s) {
   launch_phi_draw_batch(b.ar, b.phidev(b.mblock0), b.m_n_blocks, b.Kmax_all, b.t_dev, s);
-  launch_alias_build_batch(b.ar, b.phidev(b.mblock0), b.Kmax_all, 0, b.Vtot, s);
-  launch_z_sweep_batch(b.ar, b.zdev(), b.Kmax_all, z_args_merged(b, b.counters, b.ll), s, b.mshape.z_warps_per_block,
-                       b.mshape.z_blocks_per_sm);
+  launch_alias_build_batch(b.arena(kMergedWork), b.phidev(b.mblock0), b.Kmax_all, 0, b.Vtot, s);
+  merged_sweep(b, b.counters, b.ll, b.mshape, s);
 }
 
 // Each bucket's Phi draw and alias build as concurrent branches (their own
@@ -288,21 +321,19 @@ void merged_sweep_iteration(const Batch& b, cudaStream_t s) {
     if (!bu.used) continue;
     cudaStreamWaitEvent(bu.s, b.fork, 0);
     launch_phi_draw_batch(b.ar, b.phidev(bu.block0), bu.n_blocks, bu.Kmax, b.t_dev, bu.s);
-    launch_alias_build_batch(b.ar, b.phidev(bu.block0), bu.Kmax, bu.word0, bu.word1, bu.s);
+    launch_alias_build_batch(b.arena(kMergedWork), b.phidev(bu.block0), bu.Kmax, bu.word0, bu.word1, bu.s);
     cudaEventRecord(bu.join, bu.s);
     cudaStreamWaitEvent(s, bu.join, 0);
   }
-  launch_z_sweep_batch(b.ar, b.zdev(), b.Kmax_all, z_args_merged(b, b.counters, b.ll), s, b.mshape.z_warps_per_block,
-                       b.mshape.z_blocks_per_sm);
+  merged_sweep(b, b.counters, b.ll, b.mshape, s);
 }
 
 // The bucket's three kernels on stream s (work counter zeroed by the caller).
 void bucket_iteration(const Batch& b, u32 j, cudaStream_t s) {
   const Bucket& bu = b.bk[j];
   launch_phi_draw_batch(b.ar, b.phidev(bu.block0), bu.n_blocks, bu.Kmax, b.t_dev, s);
-  launch_alias_build_batch(b.ar, b.phidev(bu.block0), bu.Kmax, bu.word0, bu.word1, s);
-  launch_z_sweep_batch(b.ar, b.zdev(), bu.Kmax, z_args(b, j, b.counters, b.ll), s, bu.shape.z_warps_per_block,
-                       bu.shape.z_blocks_per_sm);
+  launch_alias_build_batch(b.arena(j), b.phidev(bu.block0), bu.Kmax, bu.word0, bu.word1, s);
+  bucket_sweep(b, j, b.counters, b.ll, bu.shape, s);
 }
 
 int capture_graph(Batch& b) {
@@ -310,10 +341,10 @@ int capture_graph(Batch& b) {
   cudaStream_t s = b.stream;
   BCK(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
   launch_bump(b.t_dev, s);
-  cudaMemsetAsync(b.ar.S, 0, b.S_total * 8, s);
+  cudaMemsetAsync(b.ar.S, 0, (b.S_total + kShares) * 8, s);  // and the shares behind it
   cudaMemsetAsync(b.ll, 0, (size_t)b.P * 16, s);
   cudaMemsetAsync(b.counters, 0, kCtrN * 8, s);
-  cudaMemsetAsync(b.work, 0, (GPULDA_BATCH_BUCKETS + 1) * 4, s);
+  cudaMemsetAsync(b.work, 0, (GPULDA_BATCH_BUCKETS + 1) * kSweepCtrs * 4, s);
   if (b.mode == GPULDA_BATCH_MERGED) {
     merged_iteration(b, s);
   } else if (b.mode == GPULDA_BATCH_MERGED_SWEEP) {
@@ -394,7 +425,7 @@ int create_impl(const GpuldaProblem* probs, u32 P, Batch** out) {
   std::stable_sort(perm.begin(), perm.end(),
                    [&](u32 x, u32 y) { return bucket_of(probs[x].K) < bucket_of(probs[y].K); });
   b.slot_of.resize(P);
-  u64 cells = 0, S = 0, N = 0, D = 0, W = 0;
+  u64 cells = 0, lists = 0, S = 0, N = 0, D = 0, W = 0;
   for (u32 s = 0; s < P; ++s) {
     const GpuldaProblem& p = probs[perm[s]];
     Slot sl;
@@ -409,11 +440,13 @@ int create_impl(const GpuldaProblem* probs, u32 P, Batch** out) {
     sl.flags = p.flags;
     sl.n_tokens = p.n_tokens;
     sl.cell0 = cells;
+    sl.list0 = lists;
     sl.S0 = S;
     sl.tok0 = N;
     sl.word0 = (u32)W;
     sl.doc0 = (u32)D;
     cells += ((u64)p.K * p.V + kCellAlign - 1) / kCellAlign * kCellAlign;
+    lists += (u64)p.V * list_stride(p.K);
     S += p.K;
     N += p.n_tokens;
     D += p.n_docs;
@@ -460,18 +493,18 @@ int create_impl(const GpuldaProblem* probs, u32 P, Batch** out) {
   ModelDev& ar = b.ar;
   ar.V = b.Vtot;
   if ((rc = b.alloc(&ar.n, cells)) || (rc = b.alloc(&ar.q, cells)) || (rc = b.alloc(&ar.al, cells)) ||
-      (rc = b.alloc(&ar.csr, cells)) || (rc = b.alloc(&ar.A, W)) || (rc = b.alloc(&ar.S, S)) ||
+      (rc = b.alloc(&ar.csr, cells)) || (rc = b.alloc(&ar.lists, lists)) || (rc = b.alloc(&ar.A, W)) || (rc = b.alloc(&ar.S, S + kShares)) ||
       (rc = b.alloc(&ar.nnz, W)) || (rc = b.alloc(&b.z, N)) || (rc = b.alloc(&b.w, N)) ||
       (rc = b.alloc(&b.d_len, D)) || (rc = b.alloc(&b.d_idx, D)) || (rc = b.alloc(&b.order, D)) ||
       (rc = b.alloc(&b.order_all, D)) ||
-      (rc = b.alloc(&b.pid, D)) || (rc = b.alloc(&b.wpid, W)) || (rc = b.alloc(&b.row_off, W)) ||
+      (rc = b.alloc(&b.pid, D)) || (rc = b.alloc(&b.wpid, W)) || (rc = b.alloc(&b.row_off, W)) || (rc = b.alloc(&b.list_off, W)) ||
       (rc = b.alloc(&b.K, P)) || (rc = b.alloc(&b.key0, P)) || (rc = b.alloc(&b.key1, P)) ||
       (rc = b.alloc(&b.alpha, P)) || (rc = b.alloc(&b.beta, P)) || (rc = b.alloc(&b.tok_base, P)) ||
       (rc = b.alloc(&b.cell_base, P)) || (rc = b.alloc(&b.S_off, P)) || (rc = b.alloc(&b.lg_a, P)) ||
       (rc = b.alloc(&b.lg_Ka, P)) || (rc = b.alloc(&b.cdf, (size_t)P * kPoisN * kPoisW)) ||
       (rc = b.alloc(&b.guide, (size_t)P * kPoisN * 256)) || (rc = b.alloc(&b.lfac, (size_t)P * kLogFacN)) ||
       (rc = b.alloc(&b.t_dev, 1)) || (rc = b.alloc(&b.ll, 2 * (size_t)P)) || (rc = b.alloc(&b.counters, kCtrN)) ||
-      (rc = b.alloc(&b.work, GPULDA_BATCH_BUCKETS + 1)) || (rc = b.alloc(&b.status, 1)))
+      (rc = b.alloc(&b.work, (GPULDA_BATCH_BUCKETS + 1) * kSweepCtrs)) || (rc = b.alloc(&b.status, 1)))
     return rc;
 
   // Every upload is ordered on the batch stream: a pageable cudaMemcpy may
@@ -536,7 +569,8 @@ int create_impl(const GpuldaProblem* probs, u32 P, Batch** out) {
         off += p.d_len[d];
       }
     }
-    word_rows_kernel<<<grid_for(sl.V), 256, 0, s>>>(b.wpid, b.row_off, sl.word0, sl.V, si, sl.cell0, sl.K);
+    word_rows_kernel<<<grid_for(sl.V), 256, 0, s>>>(b.wpid, b.row_off, b.list_off, sl.word0, sl.V, si, sl.cell0,
+                                                     sl.list0, sl.K);
     BCK(cudaMemcpyAsync(Cdev + sl.word0, p.C, (size_t)sl.V * 4, cudaMemcpyHostToDevice, b.stream));
     const PoisTables tb{b.cdf + (size_t)si * kPoisN * kPoisW, b.guide + (size_t)si * kPoisN * 256,
                         b.lfac + (size_t)si * kLogFacN};
@@ -558,6 +592,8 @@ int create_impl(const GpuldaProblem* probs, u32 P, Batch** out) {
       return x.first > y.first;
     });
     for (size_t i = 0; i < len.size(); ++i) order[bu.doc0 + i] = len[i].second;
+    const u32 chain = long_document(bu.tok1 - bu.tok0);
+    while (bu.n_chain < len.size() && len[bu.n_chain].first >= chain) ++bu.n_chain;
   }
   if (D) BCK(cudaMemcpyAsync(b.order, order.data(), (size_t)D * 4, cudaMemcpyHostToDevice, b.stream));
   // every document, longest first (stable), for the merged launch
@@ -571,6 +607,9 @@ int create_impl(const GpuldaProblem* probs, u32 P, Batch** out) {
     }
     for (u32 d = 0; d < D; ++d) order_all[d] = d;
     std::stable_sort(order_all.begin(), order_all.end(), [&](u32 x, u32 y) { return lens[x] > lens[y]; });
+    if (D) b.lmax = lens[order_all[0]];
+    const u32 chain = long_document(N);
+    while (b.n_chain < D && lens[order_all[b.n_chain]] >= chain) ++b.n_chain;
   }
   if (D) BCK(cudaMemcpyAsync(b.order_all, order_all.data(), (size_t)D * 4, cudaMemcpyHostToDevice, b.stream));
   static const u32 t0 = 0xffffffffu;  // the first bump makes it iteration 0
@@ -721,19 +760,18 @@ int tune_bucket(Batch& b, u32 j) {
         best.phi_cells_per_block = c;
       }
     }
-    launch_alias_build_batch(b.ar, b.phidev(bu.block0), bu.Kmax, bu.word0, bu.word1, s);
+    BCK(cudaMemsetAsync(b.arena(j).shares, 0, 16, s));
+    launch_alias_build_batch(b.arena(j), b.phidev(bu.block0), bu.Kmax, bu.word0, bu.word1, s);
     BCK(cudaGetLastError());
     // z sweep: documents per block and blocks per SM
     const u32 zc[][2] = {{8, 0}, {4, 0}, {2, 0}, {8, 2}, {4, 4}};
     for (const auto& c : zc) {
       BCK(cudaMemcpyAsync(z_b, z_save, toks * 4, cudaMemcpyDeviceToDevice, s));
       BCK(cudaMemsetAsync(n_b, 0, cells * 4, s));
-      BCK(cudaMemsetAsync(b.work + j, 0, 4, s));
-      ZLaunch zl = z_args(b, j, b.counters, nullptr);
-      zl.flags = 0;
+      BCK(cudaMemsetAsync(b.work + j * kSweepCtrs, 0, kSweepCtrs * 4, s));
       float ms = 0;
-      if ((rc = time_on(s, e0, e1, [&] { launch_z_sweep_batch(b.ar, b.zdev(), bu.Kmax, zl, s, c[0], c[1]); }, &ms)))
-        return rc;
+      const GpuldaBatchShape shape{c[0], c[1], 0, 0};
+      if ((rc = time_on(s, e0, e1, [&] { bucket_sweep(b, j, b.counters, nullptr, shape, s); }, &ms))) return rc;
       if (ms < best_z) {
         best_z = ms;
         best.z_warps_per_block = c[0];
@@ -808,19 +846,17 @@ int tune_merged(Batch& b) {
         best.phi_cells_per_block = c;
       }
     }
-    launch_alias_build_batch(b.ar, b.phidev(b.mblock0), b.Kmax_all, 0, b.Vtot, s);
+    BCK(cudaMemsetAsync(b.arena(kMergedWork).shares, 0, 16, s));
+    launch_alias_build_batch(b.arena(kMergedWork), b.phidev(b.mblock0), b.Kmax_all, 0, b.Vtot, s);
     BCK(cudaGetLastError());
     const u32 zc[][2] = {{8, 0}, {4, 0}, {2, 0}, {8, 2}, {4, 4}};
     for (const auto& c : zc) {
       BCK(cudaMemcpyAsync(b.z, z_save, b.N * 4, cudaMemcpyDeviceToDevice, s));
       BCK(cudaMemsetAsync(b.ar.n, 0, b.cells * 4, s));
-      BCK(cudaMemsetAsync(b.work + kMergedWork, 0, 4, s));
-      ZLaunch zl = z_args_merged(b, b.counters, nullptr);
-      zl.flags = 0;
+      BCK(cudaMemsetAsync(b.work + kMergedWork * kSweepCtrs, 0, kSweepCtrs * 4, s));
       float ms = 0;
-      if ((rc = time_on(s, e0, e1, [&] { launch_z_sweep_batch(b.ar, b.zdev(), b.Kmax_all, zl, s, c[0], c[1]); },
-                        &ms)))
-        return rc;
+      const GpuldaBatchShape shape{c[0], c[1], 0, 0};
+      if ((rc = time_on(s, e0, e1, [&] { merged_sweep(b, b.counters, nullptr, shape, s); }, &ms))) return rc;
       if (ms < best_z) {
         best_z = ms;
         best.z_warps_per_block = c[0];

@@ -1,6 +1,6 @@
 // doc_counts.cuh -- one document's topic counts in shared memory and the
-// per-token topic draw, shared by the Gibbs sweep (zsweep.cu) and the
-// fold-in of new documents against a fixed model (serve.cu).
+// per-token topic draw of the Gibbs sweep of documents whose words have long
+// lists (zsweep.cu) and the fold-in of such documents (serve.cu).
 //
 // Reference: sample_topics / count_topics / compute_product_cumsum /
 // draw_wary_search / draw_alias, src/cu/topics.cu:36-105 and
@@ -48,6 +48,8 @@ constexpr u32 kMaxDead = 4;
 __host__ __device__ __forceinline__ size_t doc_counts_bytes(u32 Kmax) {
   return (size_t)((Kmax + 31) & ~31u) * 2 + (size_t)((Kmax + 7) & ~7u) * 2;
 }
+
+constexpr size_t kTokStageBytes = 32 * 32;  // a chunk's staged tokens: 32 x 32 bytes
 
 struct DocCounts {
   uint16_t* cnt;  // dense counts, Kmax rounded up to 32 entries

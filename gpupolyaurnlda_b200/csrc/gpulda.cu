@@ -47,7 +47,11 @@ constexpr u32 kPieceEnd[kPieces] = {1, 3, 7, 12, 18, 24, 29, 32};
 // last pieces do not set the sweep's tail.
 constexpr u32 kLongFactor = 4;
 
-constexpr u32 kWorkCounters = 3 + 2 * kPieces;
+// A sweep's launches take their counters (SweepCtrs) from slots of a buffer's:
+// [0] whole buffer, [1, 1 + kPieces) pieces, [1 + kPieces, 1 + 2 kPieces) the
+// pieces' long documents.
+constexpr u32 kWorkSlots = 1 + 2 * kPieces;
+constexpr u32 kWorkCounters = kWorkSlots * kSweepCtrs;
 
 struct BufCtx {
   cudaStream_t stream = nullptr;  // sweeps
@@ -59,12 +63,9 @@ struct BufCtx {
   cudaEvent_t offs = nullptr;     // document offsets of the current sweep are ready
   bool used = false;
   u32* order = nullptr;           // device: document processing order
-  u64* rest = nullptr;            // device: documents the list sweep hands on (K > kMapMinK)
-  // Device work counters of this buffer's launches (kWorkCounters), so sweeps
-  // of different buffers may be in flight at the same time: [0] whole buffer,
-  // [1, 1 + kPieces) pieces, [1 + kPieces] short documents beside a split sweep,
-  // [2 + kPieces, 2 + 2 kPieces) the pieces' long documents, [2 + 2 kPieces] the
-  // number of documents that a list sweep hands on.
+  u64* rest = nullptr;            // device: documents that sweeps hand on (K > kMapMinK)
+  // Device counters of this buffer's launches, so sweeps of different buffers
+  // may be in flight at the same time.
   u32* work = nullptr;
   std::vector<u32> order_host;    // host staging of the order
   // The last host-buffer sweep's document lengths and what was derived from
@@ -77,6 +78,7 @@ struct BufCtx {
   u32 dcut[kPieces + 1] = {};
   u64 tcut[kPieces + 1] = {};
   u32 n_long[kPieces] = {};
+  u32 n_chain[kPieces] = {};  // documents that take a warp each
 };
 
 // Documents longest first (counting sort on length, ties in index order), so
@@ -91,6 +93,19 @@ void longest_first(const u32* d_len, u32 n, std::vector<u32>& order) {
   for (u32 i = 0; i < n; ++i) start[max_len - d_len[i] + 1]++;
   for (size_t b = 1; b < start.size(); ++b) start[b] += start[b - 1];
   for (u32 i = 0; i < n; ++i) order[start[max_len - d_len[i]]++] = i;
+}
+
+// How many documents of the longest-first order have at least `len` tokens.
+u32 at_least(const u32* d_len, const std::vector<u32>& order, u32 len) {
+  u32 lo = 0, hi = (u32)order.size();
+  while (lo < hi) {
+    const u32 mid = (lo + hi) / 2;
+    if (d_len[order[mid]] >= len)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  return lo;
 }
 
 // Above kMapMinK topics a document's counts live in a shared-memory hash map
@@ -109,6 +124,7 @@ constexpr u32 kMidDoc = 1024;
 // are longer than kMidDoc (they come first among them).
 struct DocSplit {
   u32 n_short = 0;
+  u32 n_chain = 0;    // documents that take a warp each (the first of the order)
   u32 lmax_long = 0;  // longest document
   u32 n_huge = 0;    // documents longer than kMidDoc (the first of the long ones)
   u32 lmax_mid = 0;  // longest document of at most kMidDoc tokens among the long ones
@@ -152,7 +168,7 @@ struct Model {
   bool noalloc_pending = false;
 
   // device-resident corpus
-  u64* crest = nullptr;  // documents the list sweep hands on (K > kMapMinK)
+  u64* crest = nullptr;  // documents that sweeps hand on (K > kMapMinK)
   u32 *cz = nullptr, *cw = nullptr, *cd_len = nullptr, *cd_idx = nullptr, *cK_d = nullptr, *corder = nullptr;
   u32 c_docs = 0;
   u64 c_tokens = 0;
@@ -165,6 +181,9 @@ DocSplit split_longest_first(const u32* d_len, u32 n, std::vector<u32>& order, u
   longest_first(d_len, n, order);
   DocSplit sp;
   if (n) sp.lmax_long = d_len[order[0]];
+  u64 tokens = 0;
+  for (u32 i = 0; i < n; ++i) tokens += d_len[i];
+  sp.n_chain = at_least(d_len, order, long_document(tokens));
   if (K <= kMapMinK || !(g.flags & GPULDA_FLAG_HASHMAP)) return sp;
   u32 first_short = n;
   for (u32 i = 0; i < n; ++i)
@@ -243,6 +262,7 @@ void free_model() {
   dfree(g.dev.q);
   dfree(g.dev.al);
   dfree(g.dev.csr);
+  dfree(g.dev.lists);
   dfree(g.dev.A);
   dfree(g.dev.S);
   dfree(g.dev.Sinv);
@@ -309,7 +329,8 @@ int init_impl(const Args* args, Buffer* buffers, u32 n_buffers, const GpuldaExAr
   for (auto& e : g.z_ev) CK(cudaEventCreate(&e));
   if ((rc = dalloc(&g.dev.n, cells)) || (rc = dalloc(&g.dev.q, cells)) || (rc = dalloc(&g.dev.al, cells)) ||
       (rc = dalloc(&g.dev.csr, cells)) ||
-      (rc = dalloc(&g.dev.A, g.V)) || (rc = dalloc(&g.dev.S, g.K)) || (rc = dalloc(&g.dev.Sinv, g.K)) ||
+      (g.K <= kMapMinK && (rc = dalloc(&g.dev.lists, (size_t)g.V * list_stride(g.K)))) ||
+      (rc = dalloc(&g.dev.A, g.V)) || (rc = dalloc(&g.dev.S, g.K + 2)) || (rc = dalloc(&g.dev.Sinv, g.K)) ||
       (rc = dalloc(&g.dev.nnz, g.V)) ||
       (rc = dalloc(&g.C, g.V)) || (rc = dalloc(&g.cdf, (size_t)kPoisN * kPoisW)) ||
       (rc = dalloc(&g.guide, (size_t)kPoisN * 256)) || (rc = dalloc(&g.lfac, kLogFacN)) ||
@@ -345,6 +366,7 @@ int init_impl(const Args* args, Buffer* buffers, u32 n_buffers, const GpuldaExAr
   g.dev.beta = g.beta;
   g.dev.key0 = g.key0;
   g.dev.key1 = g.key1;
+  g.dev.shares = g.K <= kMapMinK ? g.dev.S + g.K : nullptr;
   g.dev.tables = PoisTables{g.cdf, g.guide, g.lfac};
 
   for (u32 i = 0; i < n_buffers; ++i) {
@@ -401,7 +423,7 @@ int phi_step_async(cudaStream_t s) {
   g.swept = false;
   g.launches = 0;
   CK(cudaEventRecord(g.ev[0], s));
-  CK(cudaMemsetAsync(g.dev.S, 0, (size_t)g.K * 8, s));
+  CK(cudaMemsetAsync(g.dev.S, 0, ((size_t)g.K + 2) * 8, s));  // and dev.shares behind it
   CK(cudaMemsetAsync(g.counters, 0, kCtrN * 8, s));
   CK(cudaMemsetAsync(g.ll, 0, 16, s));
   CK(cudaEventRecord(g.ev[1], s));
@@ -437,45 +459,23 @@ ZLaunch z_args(u32* z, const u32* w, const u32* d_len, const u32* d_idx, const u
   return zl;
 }
 
-// One z-sweep launch over n_docs documents whose d_len / d_idx / order / K_d
-// start at the given pointers; d_idx offsets are relative to z and w, and the
-// tokens' Philox indices start at tok_base.
-int z_launch(cudaStream_t s, u32* z, const u32* w, const u32* d_len, const u32* d_idx, const u32* order, u32* K_d,
-             u32 n_docs, u64 n_tokens, u64 tok_base, u32* work, u32 lmax = 0) {
-  CK(cudaMemsetAsync(work, 0, 4, s));
-  const ZLaunch zl = z_args(z, w, d_len, d_idx, order, K_d, n_docs, n_tokens, tok_base, work);
-  // (a document too long for a map in shared memory: dense counts)
-  if (!(g.K > kMapMinK && lmax && launch_z_sweep_map(g.dev, zl, s, lmax))) launch_z_sweep(g.dev, zl, s);
-  CK(cudaGetLastError());
-  g.launches += 1;
-  return GPULDA_OK;
-}
-
-// The large-K sweep without GPULDA_FLAG_HASHMAP: the list sweep, then the
-// documents that outgrew its lists (none when no document is long enough).
-// work: two work counters and the number of documents handed on.
-int z_launch_lists(cudaStream_t s, ZLaunch zl, u32 lmax, u64* rest, u32* work0, u32* work1, u32* n_rest) {
-  CK(cudaMemsetAsync(work0, 0, 4, s));
-  CK(cudaMemsetAsync(n_rest, 0, 4, s));
-  zl.work = work0;
-  zl.rest = rest;
-  zl.n_rest = n_rest;
-  launch_z_sweep_pairs(g.dev, zl, s);
-  CK(cudaGetLastError());
-  g.launches += 1;
-  // a list holds a document's topics and at most 32 more
-  if (std::min(lmax, g.K) + 32 > kListMost) {
-    CK(cudaMemsetAsync(work1, 0, 4, s));
-    zl.work = work1;
-    launch_z_sweep_rest(g.dev, zl, s, lmax);
-    CK(cudaGetLastError());
+// One sweep over zl's documents (d_idx offsets are relative to z and w, Philox
+// indices start at zl.tok_base).
+int z_launch(cudaStream_t s, ZLaunch zl, const SweepAux& x) {
+  CK(cudaMemsetAsync(x.ctrs, 0, kSweepCtrs * 4, s));
+  zl.work = x.ctrs + kCtrWork;
+  if (g.K > kMapMinK && (g.flags & GPULDA_FLAG_HASHMAP)) {
+    // (a document too long for a map in shared memory: dense counts)
+    if (!launch_z_sweep_map(g.dev, zl, s, x.lmax)) launch_z_sweep(g.dev, zl, s);
     g.launches += 1;
+  } else {
+    g.launches += launch_sweep(g.dev, nullptr, g.K, zl, x, s, 8, 0);
   }
+  CK(cudaGetLastError());
   return GPULDA_OK;
 }
 
-// One sweep over documents already on the device.  `work` holds kWorkCounters
-// counters, zeroed per launch.
+// One sweep over documents already on the device.
 int z_step_async(cudaStream_t s, u32* z, const u32* w, const u32* d_len, u32* d_idx, const u32* order, u32* K_d,
                  u32 n_docs, u64 n_tokens, bool offsets, cudaEvent_t* ev, u32* work, const DocSplit& split, u64* rest) {
   CK(cudaEventRecord(ev[0], s));
@@ -486,25 +486,22 @@ int z_step_async(cudaStream_t s, u32* z, const u32* w, const u32* d_len, u32* d_
   }
   CK(cudaEventRecord(ev[1], s));
   int rc = GPULDA_OK;
-  if (g.K > kMapMinK && !(g.flags & GPULDA_FLAG_HASHMAP)) {
-    rc = z_launch_lists(s, z_args(z, w, d_len, d_idx, order, K_d, n_docs, n_tokens, g.tok_offset, work),
-                        split.lmax_long, rest, work, work + 1, work + 2 + 2 * kPieces);
-  } else if (g.K > kMapMinK) {
+  // Documents of the order's section [a, b), none longer than lmax.
+  auto section = [&](u32 a, u32 b, u32 lmax) {
+    if (a == b || rc) return;
+    const ZLaunch zl =
+        z_args(z, w, d_len, d_idx, order + a, K_d, b - a, n_tokens, g.tok_offset, nullptr);
+    rc = z_launch(s, zl, SweepAux{work, rest, lmax, split.n_chain});
+  };
+  if (g.K > kMapMinK && (g.flags & GPULDA_FLAG_HASHMAP)) {
     // Documents over kMidDoc tokens, then those over kShortDoc, then the
     // short ones (first in `order`), one launch each on `s`, each sized for its
     // longest.
-    const u32 n_long = n_docs - split.n_short;
-    if (split.n_huge)
-      rc = z_launch(s, z, w, d_len, d_idx, order + split.n_short, K_d, split.n_huge, n_tokens, g.tok_offset, work,
-                    split.lmax_long);
-    if (!rc && n_long > split.n_huge)
-      rc = z_launch(s, z, w, d_len, d_idx, order + split.n_short + split.n_huge, K_d, n_long - split.n_huge,
-                    n_tokens, g.tok_offset, work + 1, split.lmax_mid);
-    if (!rc && split.n_short)
-      rc = z_launch(s, z, w, d_len, d_idx, order, K_d, split.n_short, n_tokens, g.tok_offset,
-                    work + 1 + kPieces, kShortDoc);
+    section(split.n_short, split.n_short + split.n_huge, split.lmax_long);
+    section(split.n_short + split.n_huge, n_docs, split.lmax_mid);
+    section(0, split.n_short, kShortDoc);
   } else {
-    rc = z_launch(s, z, w, d_len, d_idx, order, K_d, n_docs, n_tokens, g.tok_offset, work);
+    section(0, n_docs, split.lmax_long);
   }
   if (rc) return rc;
   CK(cudaEventRecord(ev[2], s));
@@ -525,6 +522,7 @@ int pipelined_sweep(Buffer* b, BufCtx* ctx) {
   u32* const dcut = ctx->dcut;
   u64* const tcut = ctx->tcut;
   u32* const n_long = ctx->n_long;
+  u32* const n_chain = ctx->n_chain;
   u32* gz = (u32*)b->gpu_z;
   u32* gw = (u32*)b->gpu_w;
   u32* gdl = (u32*)b->gpu_d_len;
@@ -565,6 +563,7 @@ int pipelined_sweep(Buffer* b, BufCtx* ctx) {
       const u64 thr = nd ? (u64)kLongFactor * (tcut[p + 1] - tcut[p]) / nd : 0;
       u32 nl = 0;
       while (nl < nd && (u64)b->d[dcut[p] + part[nl]] >= thr && thr > 0) ++nl;
+      n_chain[p] = at_least(b->d + dcut[p], part, long_document(b->n_tokens));
       n_long[p] = nl;
     }
     CK(cudaMemcpyAsync(gdl, b->d, db, cudaMemcpyHostToDevice, s));
@@ -583,6 +582,15 @@ int pipelined_sweep(Buffer* b, BufCtx* ctx) {
   CK(cudaEventRecord(ctx->offs, s));
   if (ctx->used) CK(cudaStreamWaitEvent(ctx->h2d, ctx->ev[1], 0));  // the previous copy out has read gpu_z
   const u64 tok_base = g.tok_offset;
+  // documents [a, b) of piece p's order
+  auto launch = [&](cudaStream_t st, u32 p, u32 a, u32 b2, u32 slot) {
+    const u32 d0 = dcut[p];
+    const u32* order = ctx->order + d0 + a;
+    const ZLaunch zl =
+        z_args(gz, gw, gdl + d0, gdi + d0, order, gkd + d0, b2 - a, b->n_tokens, tok_base, nullptr);
+    return z_launch(st, zl, SweepAux{ctx->work + slot * kSweepCtrs, nullptr, b->d[d0 + ctx->order_host[d0 + a]],
+                                     n_chain[p] > a ? n_chain[p] - a : 0u});
+  };
   for (u32 p = 0; p < kPieces; ++p) {
     const u64 t0 = tcut[p], t1 = tcut[p + 1];
     if (t1 > t0) {
@@ -598,14 +606,12 @@ int pipelined_sweep(Buffer* b, BufCtx* ctx) {
       cudaStream_t ls = ctx->lpiece[p];
       CK(cudaStreamWaitEvent(ls, ctx->in[p], 0));
       CK(cudaStreamWaitEvent(ls, ctx->offs, 0));
-      const int rc = z_launch(ls, gz, gw, gdl + dcut[p], gdi + dcut[p], ctx->order + dcut[p], gkd + dcut[p], nl,
-                              b->n_tokens, tok_base, ctx->work + 2 + kPieces + p);
+      const int rc = launch(ls, p, 0, nl, 1 + kPieces + p);
       if (rc) return rc;
       CK(cudaEventRecord(ctx->lout[p], ls));
     }
     if (nd > nl) {
-      const int rc = z_launch(ps, gz, gw, gdl + dcut[p], gdi + dcut[p], ctx->order + dcut[p] + nl, gkd + dcut[p],
-                              nd - nl, b->n_tokens, tok_base, ctx->work + 1 + p);
+      const int rc = launch(ps, p, nl, nd, 1 + p);
       if (rc) return rc;
     }
     if (nl) CK(cudaStreamWaitEvent(ps, ctx->lout[p], 0));
@@ -1038,7 +1044,7 @@ extern "C" int gpulda_debug_alias(const uint32_t* q, uint32_t K, uint64_t* table
 // code that owns all device memory through its own pool, services that must
 // not allocate once serving has started, or work issued where cudaMalloc is
 // not permitted.  Its only scratch (document offsets, work counters and
-// the list of documents a list sweep hands on) is the file-scope device array below, sized for
+// the documents that sweeps hand on) is the file-scope device array below, sized for
 // GPULDA_NOALLOC_MAX_DOCS documents: 12 MiB + 256 B that every GPU which loads
 // this library holds until the process exits.  In host code the array's name
 // is only a host-side stand-in; its device address is looked up once per
@@ -1053,7 +1059,7 @@ extern "C" int gpulda_debug_alias(const uint32_t* q, uint32_t K, uint64_t* table
 namespace {
 constexpr u32 kNoAllocMaxDocs = GPULDA_NOALLOC_MAX_DOCS;
 constexpr u32 kNoAllocTail = 64;  // work-queue counters and padding
-// document offsets, counters, and (8-byte) the documents that a list sweep hands on
+// document offsets, counters, and (8-byte) the documents that sweeps hand on
 static __device__ __align__(256) u32 g_noalloc_scratch[kNoAllocMaxDocs + kNoAllocTail + 2 * kNoAllocMaxDocs];
 constexpr int kNoAllocMaxDevices = 64;
 u32* g_noalloc_addr[kNoAllocMaxDevices] = {};
@@ -1086,14 +1092,13 @@ extern "C" int gpulda_sample_z_device_noalloc(uint32_t* z, const uint32_t* w, co
   if (int rc = after_noalloc(s)) return rc;
   launch_doc_offsets(d_len, d_idx, n_docs, s);
   CK(cudaGetLastError());
-  // Above kMapMinK topics, the large-K stores the other sweeps use.  The
-  // lengths are on the device only, so the launches take any document length.
-  const ZLaunch zl = z_args(z, w, d_len, d_idx, nullptr, nullptr, n_docs, n_tokens, g.tok_offset, work);
+  // The lengths are on the device only, so the launches take any document
+  // length.
+  const ZLaunch zl = z_args(z, w, d_len, d_idx, nullptr, nullptr, n_docs, n_tokens, g.tok_offset, nullptr);
   g.launches += 1;
-  const int rc = g.K > kMapMinK && !(g.flags & GPULDA_FLAG_HASHMAP)
-                     ? z_launch_lists(s, zl, 65535u, (u64*)(work + kNoAllocTail), work, work + 1, work + 2)
-                     : z_launch(s, z, w, d_len, d_idx, nullptr, nullptr, n_docs, n_tokens, g.tok_offset, work, 65535u);
-  if (rc) return rc;
+  u64* q = (u64*)(work + kNoAllocTail);
+  // (documents of different lengths side by side: a warp each)
+  if (int rc = z_launch(s, zl, SweepAux{work, q, 65535u, n_docs})) return rc;
   CK(cudaEventRecord(g.noalloc_done, s));
   g.noalloc_pending = true;
   g.tok_offset += n_tokens;

@@ -286,10 +286,12 @@ __device__ void alias_build_block(const u64* ent, u32 n, u64 A, u64* vals, uint1
 constexpr u32 kPerThread = 8;
 
 __device__ __forceinline__ void alias_word(u32 K, u32* __restrict__ qrow, const u64* __restrict__ S,
-                                           const u64* __restrict__ Sinv, u64* alrow, u64* csrrow, u64* A_out,
+                                           const u64* __restrict__ Sinv, u64* alrow, u64* csrrow, u64* eighths, u64* A_out,
+                                           u64* s_shares,
                                            u32* nnz_out, u64* s_vals, uint16_t* s_idx, u32 smem_items, u64* g_vals,
                                            uint16_t* g_idx, u64* sh) {
   u64 part = 0, nz = 0;
+  u32 xsum = 0;
   const u32 tile = blockDim.x * kPerThread;
   for (u32 t0 = 0; t0 < K; t0 += tile) {
     const u32 k0 = t0 + threadIdx.x * kPerThread;
@@ -302,6 +304,7 @@ __device__ __forceinline__ void alias_word(u32 K, u32* __restrict__ qrow, const 
       if (k < K) {
         const u32 x = qrow[k];
         if (x) {  // a zero count is already a zero q
+          xsum += x;
           const u64 num = (u64)x << 32, sk = S[k];
           if (Sinv) {
             // floor(num / sk) from the reciprocal: the multiply-high is at
@@ -333,6 +336,19 @@ __device__ __forceinline__ void alias_word(u32 K, u32* __restrict__ qrow, const 
   }
   const u64 A = block_sum_u64(part, sh);  // (also orders the list writes before the build)
   const u32 n = (u32)nz;
+  if (s_shares) {  // the word's tokens (its draws' sum), by its list's length
+    xsum = __reduce_add_sync(kFullMask, xsum);
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd((unsigned long long*)s_shares, (unsigned long long)xsum);
+      if (n > kShortList) atomicAdd((unsigned long long*)s_shares + 1, (unsigned long long)xsum);
+    }
+  }
+  if (eighths && n) {  // the list again, by eighths, with zeros to the end of the last
+    const u32 c = list_pairs(n), recip = list_recip(c);
+    const u32 end = (((n - 1) / 2 * recip >> 20) + 1) * 2 * c;
+    for (u32 i = threadIdx.x; i < end; i += blockDim.x)
+      eighths[list_pos(i, c, recip)] = i < n ? csrrow[i] : 0ull;
+  }
   if (n) {
     const bool in_smem = n <= smem_items;
     alias_build_block(csrrow, n, A, in_smem ? s_vals : g_vals, in_smem ? s_idx : g_idx, alrow, sh);
@@ -347,32 +363,42 @@ __device__ __forceinline__ void alias_word(u32 K, u32* __restrict__ qrow, const 
 __global__ void __launch_bounds__(256) alias_build_kernel(ModelDev m, unsigned char* gscratch, size_t slice,
                                                           u32 smem_items) {
   extern __shared__ __align__(16) unsigned char s_raw[];
-  __shared__ u64 sh[33];
+  __shared__ u64 sh[33], sh_shares[2];
   const u32 K = m.K;
+  if (threadIdx.x < 2) sh_shares[threadIdx.x] = 0;
+  __syncthreads();
   u64* s_vals = (u64*)s_raw;
   uint16_t* s_idx = (uint16_t*)(s_vals + smem_items);
   u64* g_vals = gscratch ? (u64*)(gscratch + (size_t)blockIdx.x * slice) : nullptr;
   uint16_t* g_idx = gscratch ? (uint16_t*)(g_vals + K) : nullptr;
   for (u32 w = blockIdx.x; w < m.V; w += gridDim.x) {
     const size_t row = (size_t)w * K;
-    alias_word(K, m.q + row, m.S, m.Sinv, m.al + row, m.csr + row, m.A + w, m.nnz + w, s_vals, s_idx, smem_items,
+    alias_word(K, m.q + row, m.S, m.Sinv, m.al + row, m.csr + row,
+               m.lists ? m.lists + (size_t)w * list_stride(K) : nullptr, m.A + w, m.shares ? sh_shares : nullptr, m.nnz + w, s_vals, s_idx, smem_items,
                g_vals, g_idx, sh);
   }
+  if (m.shares && threadIdx.x < 2)
+    atomicAdd((unsigned long long*)m.shares + threadIdx.x, (unsigned long long)sh_shares[threadIdx.x]);
 }
 
 // Batched alias build over global words [w0, w1) of any problems; shared
 // memory sized for the largest K among them.
 __global__ void __launch_bounds__(256) alias_build_batch_kernel(ModelDev ar, BatchPhiDev bp, u32 Kmax, u32 w0, u32 w1) {
   extern __shared__ __align__(16) unsigned char s_raw[];
-  __shared__ u64 sh[33];
+  __shared__ u64 sh[33], sh_shares[2];
+  if (threadIdx.x < 2) sh_shares[threadIdx.x] = 0;
+  __syncthreads();
   u64* vals = (u64*)s_raw;
   uint16_t* idx = (uint16_t*)(vals + Kmax);
   for (u32 w = w0 + blockIdx.x; w < w1; w += gridDim.x) {
     const u32 pb = bp.wpid[w], K = bp.K[pb];
     const size_t row = bp.row_off[w];
-    alias_word(K, ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row, ar.A + w, ar.nnz + w, vals,
+    alias_word(K, ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row,
+               ar.lists + bp.list_off[w], ar.A + w, sh_shares, ar.nnz + w, vals,
                idx, Kmax, nullptr, nullptr, sh);
   }
+  if (threadIdx.x < 2)
+    atomicAdd((unsigned long long*)ar.shares + threadIdx.x, (unsigned long long)sh_shares[threadIdx.x]);
 }
 
 // Reciprocals of the per-topic normalisers, inv[k] = floor((2^64 - 1) / S[k])

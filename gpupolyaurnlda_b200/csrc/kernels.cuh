@@ -23,6 +23,53 @@ enum CounterSlots { kCtrTokens = 0, kCtrDocs = 1, kCtrSparseWork = 2, kCtrSparse
 // dense per-document count array would cost 2 K bytes of shared memory).
 constexpr u32 kMapMinK = 2048;
 
+// A word's list (q << 32 | k for q > 0, ascending k) of n entries stored by
+// eighths: it is cut into eighths of 2 c consecutive entries, c = list_pairs(n),
+// and pair p of eighth e stands at pair p * 8 + e, so that eight lanes that walk
+// an eighth each read 128 contiguous bytes at a time (each its own run of an
+// ordinary list: 32 L1 wavefronts a load instead of 4).  Zero entries follow to
+// the end of the eighth that the list ends in.  Beyond 160 entries c is 4 times
+// an odd number: where a list holds most topics, the lanes' counts then lie in
+// different banks.
+
+__host__ __device__ inline u32 list_pairs(u32 n) {
+  return n <= 160 ? (n ? ((n + 31) >> 5) << 1 : 2u) : (((n + 63) >> 6) | 1u) << 2;
+}
+
+// Entries from one word's list to the next.
+__host__ __device__ inline u32 list_stride(u32 K) { return 16 * list_pairs(K); }
+
+// Where entry i of an eighths-stored list with c = list_pairs(n) stands; recip =
+// ceil(2^20 / c) divides the at most 8 c <= 1056 pairs' numbers exactly.
+__host__ __device__ inline u32 list_recip(u32 c) { return ((1u << 20) + c - 1) / c; }
+__host__ __device__ inline u32 list_pos(u32 i, u32 c, u32 recip) {
+  const u32 pi = i >> 1, e = (pi * recip) >> 20, p = pi - e * c;
+  return 2 * (p * 8 + e) + (i & 1);
+}
+
+// A lane's run of a word's list: n pairs of entries from pair `at`, 8 pairs
+// apart; `on` when any of them lies in the list.
+struct Run {
+  u32 at, n;
+  bool on;
+};
+
+// Lane l of W lanes that walk a list of nw entries: W/8 lanes share an eighth.
+template <u32 W>
+__device__ __forceinline__ Run lane_run(u32 nw, u32 l) {
+  constexpr u32 S = W / 8;
+  const u32 c = list_pairs(nw);
+  const u32 per = (c + S - 1) / S, e = l / S, p0 = (l % S) * per;
+  Run r;
+  r.n = S == 1 ? c : min(per, c > p0 ? c - p0 : 0u);
+  r.at = p0 * 8 + e;
+  r.on = 2 * (e * c + p0) < nw && (S == 1 || r.n);
+  return r;
+}
+
+// A word's list is short up to this many entries.
+constexpr u32 kShortList = 160;
+
 struct ModelDev {
   u32 K, V;
   float alpha, beta;
@@ -31,10 +78,12 @@ struct ModelDev {
   u32* q;      // V*K fixed-point Phi (raw x between the two Phi kernels)
   u64* al;     // V*K alias entries
   u64* csr;    // V*K per-word lists of (q << 32 | k) for q > 0, ascending k, nnz[w] used
+  u64* lists;  // the same lists by eighths, list_stride(K) entries apart (K <= kMapMinK, else null)
   u64* A;      // V   dense mass per word
   u64* S;      // K   per-topic normalisers
   u64* Sinv;   // K   floor((2^64 - 1) / S[k]), written by the alias build's launch (null: divide)
   u32* nnz;    // V   nonzero x per word
+  u64* shares; // 2   sum of x, and that of the words with long lists (K <= kMapMinK, else null)
   PoisTables tables;
 };
 
@@ -46,6 +95,7 @@ struct ModelDev {
 struct BatchDev {
   const u32* pid;       // per document
   const u64* row_off;   // per word
+  const u64* list_off;  // per word: where its list starts
   const u32* K;
   const float* alpha;
   const u32* key0;
@@ -69,6 +119,7 @@ struct BatchPhiDev {
   const u32* key1;
   const u32* wpid;
   const u64* row_off;
+  const u64* list_off;
   const u32* cdf;
   const uint8_t* guide;
   const double* lfac;
@@ -91,6 +142,9 @@ struct ZLaunch {
   double* ll;                    // [0] sum, [1] skipped tokens (as double); may be null
   u32* work;                     // zeroed work-queue counter
   u32* status;
+  // The shares of words with short and long lists that decide which of two
+  // launches sweeps; null: this one does.
+  const u64* shares = nullptr;
   // Documents that the launch hands on: token reached << 32 | document, and
   // their number.  The list sweep writes them, the sweep of the rest reads
   // them in place of `order`.
@@ -134,12 +188,23 @@ void launch_doc_offsets(const u32* d_len, u32* d_idx, u32 n_docs, cudaStream_t s
 // ZLaunch.flags bits.
 constexpr u32 kZFlagLoglik = 1u;  // accumulate the joint log-likelihood
 
-// One sweep over a set of documents.
+// One sweep over a set of documents, one warp to a document, walking its topics
+// or its words' lists, whichever is shorter.
 void launch_z_sweep(const ModelDev& m, const ZLaunch& z, cudaStream_t s);
 // One sweep over documents of many problems (arenas + tables), with the given
 // warps per block and cap on blocks per SM (0: as many as fit).
 void launch_z_sweep_batch(const ModelDev& arenas, const BatchDev& b, u32 Kmax, const ZLaunch& z, cudaStream_t s,
                           u32 warps_per_block, u32 blocks_per_sm);
+// The same sweep over the words' lists only, K <= kMapMinK (b: documents of many
+// problems, or null).  The first n_long documents take a warp each, the others a
+// quarter.
+void launch_z_sweep_words(const ModelDev& m, const BatchDev* b, u32 Kmax, const ZLaunch& z, u32 n_long, cudaStream_t s,
+                          u32 warps_per_block, u32 blocks_per_sm);
+// Whether so many tokens' words have long lists that the sweep over the
+// documents' topics and the words' lists is the faster: above one in 12 a step
+// of the other's four documents to a warp is a long one too often (0.17 ns a
+// token with none, 1.8 with mostly long lists, against 0.28 and 0.5).
+__device__ __forceinline__ bool mostly_long_lists(const u64* shares) { return 12 * shares[1] > shares[0]; }
 // The same sweep with each document's counts in a shared-memory hash map
 // (large K).  Documents longer than lmax are reported, not swept.  Returns
 // false without launching when lmax needs more shared memory than a block has.
@@ -150,9 +215,25 @@ u32 z_map_slots(u32 K, u32 lmax);
 // entries are handed on in z.rest.
 constexpr u32 kListMost = 512;
 void launch_z_sweep_pairs(const ModelDev& m, const ZLaunch& z, cudaStream_t s);
-// The rest of the documents in z.rest, none longer than lmax, lists in shared
-// memory.
+// The documents of z.rest, none longer than lmax, lists in shared memory.
 void launch_z_sweep_rest(const ModelDev& m, const ZLaunch& z, cudaStream_t s, u32 lmax);
+
+// A whole sweep over zl's documents by the kernels that suit them: up to kMapMinK
+// topics the sweep over the words' lists or that over the shorter of the two
+// sides, by the words' lists; above, the list sweep, then what outgrows its
+// lists.  Returns the number of launches.
+constexpr u32 kSweepCtrs = 4;  // counters of a sweep's launches, zeroed by the caller
+enum SweepCtrSlots { kCtrWork = 0, kCtrRestWork = 1, kCtrRest = 2 };
+struct SweepAux {
+  u32* ctrs;   // kSweepCtrs
+  u64* queue;  // a document each (K > kMapMinK)
+  u32 lmax;    // longest document
+  u32 n_long;  // documents to take a warp each (K <= kMapMinK; long_document)
+};
+u32 launch_sweep(const ModelDev& m, const BatchDev* b, u32 Kmax, ZLaunch zl, const SweepAux& x, cudaStream_t s,
+                 u32 warps_per_block, u32 blocks_per_sm);
+// Documents of at least this length take a warp each in a sweep of n_tokens.
+u32 long_document(u64 n_tokens);
 
 // Debug hooks.
 void launch_debug_philox(const u32* ctr, u32 n, u32 k0, u32 k1, u32* out, cudaStream_t s);

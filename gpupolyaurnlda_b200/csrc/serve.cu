@@ -40,6 +40,7 @@
 #include "../../include/gpulda_serve.h"
 #include "doc_counts.cuh"
 #include "kernels.cuh"
+#include "word_sweep.cuh"
 
 using namespace gpulda;
 
@@ -80,7 +81,9 @@ static_assert(sizeof(FoldReq) == 32, "FoldReq");
 
 // Shared memory per request warp: the document's counts and the staged
 // per-token data of a 32-token chunk.
-inline size_t fold_smem_bytes(u32 K) { return doc_counts_bytes(K) + 32 * 32; }
+inline size_t fold_smem_bytes(u32 K) {
+  return std::max(word_warp_bytes_one(K), doc_counts_bytes(K) + kTokStageBytes);
+}
 
 // Output record of a request: theta[K] (float), then 8-byte aligned the
 // log-likelihood (double), skipped tokens (u32) and the done flag (u32).
@@ -103,10 +106,40 @@ struct FoldCommon {
 // records (the request is skipped).
 constexpr u32 kStatusBadRequest = 16;
 
+// A request as sweep_doc's source of tokens: n_iter passes over its nc chunks.
+// A chunk's topics are read a chunk ahead: with one chunk they are those just
+// drawn.
+struct FoldSource {
+  const u32* w_;
+  const u32* z_;
+  u32 L, V, lane, nc, n_iter;
+  u64 ridx;
+  u32 k0, k1;
+  u32 status;
+  __device__ __forceinline__ u32 at(u32 c) const { return (c % nc) * 32 + lane; }
+  __device__ __forceinline__ bool valid(u32 c) const { return c < nc * n_iter && at(c) < L; }
+  __device__ __forceinline__ u32 word(u32 c) {
+    u32 w = valid(c) ? __ldcg(w_ + at(c)) : 0u;
+    if (w >= V) {
+      status |= kStatusBadWord;
+      w %= V;
+    }
+    return w;
+  }
+  __device__ __forceinline__ u32 topic(u32 c) const { return z_[at(c)]; }
+  __device__ __forceinline__ U4 words(u32 c) const {
+    return draw4(ridx | at(c), c / nc, kStreamFold, 0, k0, k1);
+  }
+  __device__ __forceinline__ void chunk_done(u32 c, u32 k, u32* z_next) const {
+    if (nc == 1 && valid(c)) *z_next = valid(c + 1) ? k : *z_next;
+  }
+};
+
 // Fold-in of one request by one warp.  Words are read through L2 only: the
 // pool is refilled by copies while kernels run, so an SM's L1 may still hold
 // an earlier request's words at the same address.
-__device__ void fold_request(const FoldCommon& a, DocCounts& dc, uint4* stage, const FoldReq& rq, u32 lane) {
+template <bool WORDS>
+__device__ __forceinline__ void fold_request(const FoldCommon& a, unsigned char* fsm, const FoldReq& rq, u32 lane) {
   if (rq.w_off + rq.len > a.pool_words || rq.z_off + rq.len > a.pool_words || rq.rec >= a.n_recs ||
       rq.len > 65535u) {
     if (lane == 0) atomicOr(a.status, kStatusBadRequest);
@@ -126,59 +159,84 @@ __device__ void fold_request(const FoldCommon& a, DocCounts& dc, uint4* stage, c
     z[i] = (u32)(((u64)r.x * K) >> 32);
   }
   __syncwarp();
-  doc_counts_build(dc, z, L, K, lane, &status, kStatusBadTopic);
+  // The document's counts, in the struct of the walk that draws its topics.
+  WordDoc wd;
+  DocCounts dc;
+  const uint16_t* cnt;
+  if (WORDS) {
+    wd = word_doc_at<32>(fsm, K, lane);
+    uint4* stage = reinterpret_cast<uint4*>(fsm + word_doc_bytes(K));
+    word_doc_build<32>(wd, z, L, K, lane, &status, kStatusBadTopic);
 
-  for (u32 t = 0; t < a.n_iter; ++t) {
-    for (u32 base = 0; base < L; base += 32) {
-      const u32 i = base + lane;
-      const bool valid = i < L;
-      u32 my_w = valid ? __ldcg(w + i) : 0;
-      const u32 my_z = valid ? z[i] : 0;
-      if (my_w >= V) {
-        status |= kStatusBadWord;
-        my_w %= V;
-      }
-      const U4 r = draw4(ridx | i, t, kStreamFold, 0, k0, k1);
-      const u32 my_nw = valid ? __ldg(m.nnz + my_w) : 0u;
-      const u64 my_A = valid ? __ldg(m.A + my_w) : 0ull;
-      const u32 my_s = (u32)(((u64)r.z * my_nw) >> 32);
-      const u64 my_row = (u64)my_w * K;
-      const u64 my_al = (valid && my_nw) ? __ldg(m.al + my_row + my_s) : 0ull;
-      u32 new_z = my_z;
-      const u32 nt = min(32u, L - base);
-      // per-token data staged in shared memory (broadcast loads, not shuffles)
-      __syncwarp();
-      stage[2 * lane] = make_uint4(my_z, r.x, r.y, my_nw);
-      stage[2 * lane + 1] = make_uint4((u32)my_row, (u32)(my_row >> 32), (u32)my_A, (u32)(my_A >> 32));
-      __syncwarp();
-      for (u32 j = 0; j < nt; ++j) {
-        const uint4 s0 = stage[2 * j], s1 = stage[2 * j + 1];
-        const u32 zj = s0.x, r0 = s0.y, r1 = s0.z, nw = s0.w;
-        const size_t row = ((u64)s1.y << 32) | s1.x;
-        const u64 Aw = ((u64)s1.w << 32) | s1.z;
-        u32 nzm;
-        bool sp;
-        // as in the training sweep: as few register slots as the walk needs
-        const u32 cper_j = ((nw < dc.nl ? nw : dc.nl) + 31) >> 5;
-        const u32 k = cper_j <= 2 ? token_step<2u>(dc, zj, r0, r1, r.w, my_al, j, m.q + row, m.csr + row, nw, Aw, alpha,
-                                                   lane, &nzm, &sp)
-                                  : token_step<4u>(dc, zj, r0, r1, r.w, my_al, j, m.q + row, m.csr + row, nw, Aw, alpha,
-                                                   lane, &nzm, &sp);
-        if (lane == j) new_z = k;
+    {
+      const u32 nc = (L + 31) / 32;
+      FoldSource src{w, z, L, V, lane, nc ? nc : 1u, a.n_iter, ridx, k0, k1, 0u};
+      sweep_doc<32>(wd, stage, m, Rows{nullptr, nullptr}, K, alpha, nc * a.n_iter, lane, src,
+                    [&](u32 c, u32 new_z, bool, u32, u64, u32) {
+                      const u32 i = (c % nc) * 32 + lane;
+                      if (i < L) z[i] = new_z;
+                    });
+      status |= src.status;
+    }
+    cnt = wd.cnt;
+  } else {
+    dc = doc_counts_at(fsm, K);
+    uint4* stage = reinterpret_cast<uint4*>(fsm + doc_counts_bytes(K));
+    doc_counts_build(dc, z, L, K, lane, &status, kStatusBadTopic);
+
+    for (u32 t = 0; t < a.n_iter; ++t) {
+      for (u32 base = 0; base < L; base += 32) {
+        const u32 i = base + lane;
+        const bool valid = i < L;
+        u32 my_w = valid ? __ldcg(w + i) : 0;
+        const u32 my_z = valid ? z[i] : 0;
+        if (my_w >= V) {
+          status |= kStatusBadWord;
+          my_w %= V;
+        }
+        const U4 r = draw4(ridx | i, t, kStreamFold, 0, k0, k1);
+        const u32 my_nw = valid ? __ldg(m.nnz + my_w) : 0u;
+        const u64 my_A = valid ? __ldg(m.A + my_w) : 0ull;
+        const u32 my_s = (u32)(((u64)r.z * my_nw) >> 32);
+        const u64 my_row = (u64)my_w * K;
+        const u64 my_al = (valid && my_nw) ? __ldg(m.al + my_row + my_s) : 0ull;
+        u32 new_z = my_z;
+        const u32 nt = min(32u, L - base);
+        // per-token data staged in shared memory (broadcast loads, not shuffles)
+        __syncwarp();
+        stage[2 * lane] = make_uint4(my_z, r.x, r.y, my_nw);
+        stage[2 * lane + 1] = make_uint4((u32)my_row, (u32)(my_row >> 32), (u32)my_A, (u32)(my_A >> 32));
+        __syncwarp();
+        for (u32 j = 0; j < nt; ++j) {
+          const uint4 s0 = stage[2 * j], s1 = stage[2 * j + 1];
+          const u32 zj = s0.x, r0 = s0.y, r1 = s0.z, nw = s0.w;
+          const size_t row = ((u64)s1.y << 32) | s1.x;
+          const u64 Aw = ((u64)s1.w << 32) | s1.z;
+          u32 nzm;
+          bool sp;
+          // as in the training sweep: as few register slots as the walk needs
+          const u32 cper_j = ((nw < dc.nl ? nw : dc.nl) + 31) >> 5;
+          const u32 k = cper_j <= 2 ? token_step<2u>(dc, zj, r0, r1, r.w, my_al, j, m.q + row, m.csr + row, nw, Aw, alpha,
+                                                     lane, &nzm, &sp)
+                                    : token_step<4u>(dc, zj, r0, r1, r.w, my_al, j, m.q + row, m.csr + row, nw, Aw, alpha,
+                                                     lane, &nzm, &sp);
+          if (lane == j) new_z = k;
+          __syncwarp();
+        }
+        if (valid) z[i] = new_z;
         __syncwarp();
       }
-      if (valid) z[i] = new_z;
-      __syncwarp();
     }
+    cnt = dc.cnt;
   }
 
   // theta and the log-likelihood of the document's words under it
   unsigned char* rec = a.recs + (size_t)rq.rec * a.rec_bytes;
   float* theta = (float*)rec;
   const double denom = (double)L + (double)K * (double)alpha;
-  for (u32 k = lane; k < K; k += 32) theta[k] = (float)(((double)dc.cnt[k] + (double)alpha) / denom);
+  for (u32 k = lane; k < K; k += 32) theta[k] = (float)(((double)cnt[k] + (double)alpha) / denom);
   // sum_k (m_k + alpha) q[w][k] = sum_k m_k q[w][k] + alpha A[w]: the first term
-  // exactly (u64) over the shorter of the two lists, the second from the dense mass
+  // exactly (u64) over the word's list or the document's, the second from the dense mass
   double ll = 0.0;
   u32 skipped = 0;
   for (u32 i = 0; i < L; ++i) {
@@ -186,15 +244,17 @@ __device__ void fold_request(const FoldCommon& a, DocCounts& dc, uint4* stage, c
     const u32 nw = __ldg(m.nnz + wi);
     const size_t row = (size_t)wi * K;
     u64 part = 0;
-    if (nw < dc.nl) {
-      for (u32 e = lane; e < nw; e += 32) {
-        const u64 ent = __ldg(m.csr + row + e);
-        part += (u64)dc.cnt[(u32)ent & 0xffffu] * (u32)(ent >> 32);
-      }
+    if (WORDS) {
+      const Run r = lane_run<32>(nw, lane);
+      const ulonglong2* list = reinterpret_cast<const ulonglong2*>(m.lists + (size_t)wi * list_stride(K));
+      for (u32 e = 0; r.on && e < r.n; ++e) part += mass_of(cnt, __ldg(list + r.at + e * 8));
+      __syncwarp();
+    } else if (nw < dc.nl) {
+      for (u32 e = lane; e < nw; e += 32) part += mass_of(cnt, __ldg(m.csr + row + e));
     } else {
       for (u32 e = lane; e < dc.nl; e += 32) {
         const u32 k = dc.tl[e];
-        part += (u64)dc.cnt[k] * __ldg(m.q + row + k);
+        part += (u64)cnt[k] * __ldg(m.q + row + k);
       }
     }
     const u64 Bw = warp_sum_u64(part);
@@ -220,12 +280,11 @@ __device__ void fold_request(const FoldCommon& a, DocCounts& dc, uint4* stage, c
 }
 
 // Launch mode: one request per block of one warp.
-__global__ void __launch_bounds__(32) fold_launch_kernel(FoldCommon a, const FoldReq* items) {
+template <bool WORDS>
+__global__ void __launch_bounds__(32, WORDS ? 24 : 32) fold_launch_kernel(FoldCommon a, const FoldReq* items) {
   extern __shared__ __align__(16) unsigned char fsm[];
-  DocCounts dc = doc_counts_at(fsm, a.m.K);
-  uint4* stage = reinterpret_cast<uint4*>(fsm + doc_counts_bytes(a.m.K));
   const FoldReq rq = items[blockIdx.x];
-  fold_request(a, dc, stage, rq, threadIdx.x);
+  fold_request<WORDS>(a, fsm, rq, threadIdx.x);
 }
 
 struct RingDev {
@@ -266,11 +325,10 @@ __device__ __forceinline__ u64 global_timer_ns() {
 
 // Persistent mode: every block is one warp that serves requests until it has
 // been idle for kIdleNs or the stop flag is up.  Every wait is bounded.
-__global__ void __launch_bounds__(32, 32) fold_persistent_kernel(FoldCommon a, RingDev q) {
+template <bool WORDS>
+__global__ void __launch_bounds__(32, WORDS ? 24 : 32) fold_persistent_kernel(FoldCommon a, RingDev q) {
   extern __shared__ __align__(16) unsigned char fsm[];
   const u32 lane = threadIdx.x;
-  DocCounts dc = doc_counts_at(fsm, a.m.K);
-  uint4* stage = reinterpret_cast<uint4*>(fsm + doc_counts_bytes(a.m.K));
   while (true) {
     unsigned long long mine = ~0ull;
     if (lane == 0) {
@@ -309,7 +367,7 @@ __global__ void __launch_bounds__(32, 32) fold_persistent_kernel(FoldCommon a, R
     rq.rid = ((u64)hi.y << 32) | hi.x;
     rq.len = hi.z;
     rq.rec = hi.w;
-    fold_request(a, dc, stage, rq, lane);
+    fold_request<WORDS>(a, fsm, rq, lane);
   }
 }
 
@@ -388,6 +446,7 @@ struct Server {
   u32 rec_bytes = 0, max_inflight = 0;
   size_t stage_cap = 0;  // bytes of each staging buffer
   FoldCommon fc{};
+  bool words = true;  // the walk that suits the model's lists (choose_walk)
   std::vector<void*> allocs;
   // request pool, u32 units
   u64 pool_words = 0, pool_used = 0;
@@ -513,6 +572,7 @@ int create_common(const GpuldaServeArgs* a, u32 K, u32 V, float alpha, std::uniq
   FoldCommon& fc = s.fc;
   int rc;
   if ((rc = s.alloc(&fc.m.q, cells)) || (rc = s.alloc(&fc.m.al, cells)) || (rc = s.alloc(&fc.m.csr, cells)) ||
+      (rc = s.alloc(&fc.m.lists, (size_t)V * list_stride(K))) ||
       (rc = s.alloc(&fc.m.A, V)) || (rc = s.alloc(&fc.m.nnz, V)) || (rc = s.alloc(&fc.status, 1)))
     return rc;
   fc.m.K = K;
@@ -540,7 +600,7 @@ int create_common(const GpuldaServeArgs* a, u32 K, u32 V, float alpha, std::uniq
   SCK(cudaHostGetDevicePointer((void**)&fc.recs, s.recs_host, 0));
   s.free_recs.resize(s.max_inflight);
   for (u32 i = 0; i < s.max_inflight; ++i) s.free_recs[i] = s.max_inflight - 1 - i;
-  const size_t smem = fold_smem_bytes(K);
+  static_assert(GPULDA_SERVE_MAX_K <= 2048, "a request's shared memory stays below 48 KB");
   if (s.persistent) {
     s.resident_per_sm = a->slots ? a->slots : 32u;
     s.ring_cap = 1;
@@ -553,8 +613,6 @@ int create_common(const GpuldaServeArgs* a, u32 K, u32 V, float alpha, std::uniq
     s.staging.reset(new Staging[kStaging]);
     for (u32 i = 0; i < kStaging; ++i)
       if ((rc = s.staging[i].init(kStagingBytes))) return rc;
-    if (smem > 48 * 1024)
-      SCK(cudaFuncSetAttribute(fold_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   } else {
     s.n_slots = a->slots;
     s.slots.reset(new LaunchSlot[a->slots]);
@@ -564,10 +622,25 @@ int create_common(const GpuldaServeArgs* a, u32 K, u32 V, float alpha, std::uniq
       SCK(cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming));
       if ((rc = sl.st.init(kSlotStagingBytes))) return rc;
     }
-    if (smem > 48 * 1024)
-      SCK(cudaFuncSetAttribute(fold_launch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   }
   SCK(cudaDeviceSynchronize());
+  return GPULDA_OK;
+}
+
+// The walk for the model's requests: over the words' lists unless more than one
+// in 12 of a uniform mixture's tokens has a word with a long list (the training
+// sweep's rule, with the dense masses for the words' tokens).
+int choose_walk(Server& s) {
+  std::vector<u32> nnz(s.V);
+  std::vector<u64> A(s.V);
+  SCK(cudaMemcpy(nnz.data(), s.fc.m.nnz, (size_t)s.V * 4, cudaMemcpyDeviceToHost));
+  SCK(cudaMemcpy(A.data(), s.fc.m.A, (size_t)s.V * 8, cudaMemcpyDeviceToHost));
+  double all = 0.0, in_long = 0.0;
+  for (u32 w = 0; w < s.V; ++w) {
+    all += (double)A[w];
+    if (nnz[w] > kShortList) in_long += (double)A[w];
+  }
+  s.words = 12.0 * in_long <= all;
   return GPULDA_OK;
 }
 
@@ -662,9 +735,10 @@ int ensure_kernel(Server& s) {
   rd.tail = (const u64*)(s.ctl + 8);
   rd.stop = (const u32*)(s.ctl + 16);
   int fit = 0;
-  SCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, fold_persistent_kernel, 32, fold_smem_bytes(s.K)));
+  auto kern = s.words ? fold_persistent_kernel<true> : fold_persistent_kernel<false>;
+  SCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, 32, fold_smem_bytes(s.K)));
   const u32 blocks = (u32)device_sm_count() * std::max<u32>(1, std::min<u32>(s.resident_per_sm, (u32)fit));
-  fold_persistent_kernel<<<blocks, 32, fold_smem_bytes(s.K), s.kern_s>>>(s.fc, rd);
+  kern<<<blocks, 32, fold_smem_bytes(s.K), s.kern_s>>>(s.fc, rd);
   SCK(cudaGetLastError());
   SCK(cudaEventRecord(s.kern_ev, s.kern_s));
   s.kern_live = true;
@@ -744,7 +818,8 @@ int launch_batches(Server& s) {
     u32* items = s.fc.pool + off + 2 * align_up(std::max<u64>(T, 1), 64);
     if (T) SCK(cudaMemcpyAsync(s.fc.pool + off, sl.st.p + head, T * 4, cudaMemcpyHostToDevice, sl.s));
     SCK(cudaMemcpyAsync(items, sl.st.p + 16, n * sizeof(FoldReq), cudaMemcpyHostToDevice, sl.s));
-    fold_launch_kernel<<<(u32)n, 32, fold_smem_bytes(s.K), sl.s>>>(s.fc, (const FoldReq*)items);
+    auto kern = s.words ? fold_launch_kernel<true> : fold_launch_kernel<false>;
+    kern<<<(u32)n, 32, fold_smem_bytes(s.K), sl.s>>>(s.fc, (const FoldReq*)items);
     SCK(cudaGetLastError());
     SCK(cudaEventRecord(sl.done, sl.s));
     sl.busy = true;  // the staging buffer is reused once `done` has passed
@@ -781,9 +856,11 @@ extern "C" int gpulda_serve_create(const GpuldaServeArgs* args, void** handle) {
   SCK(cudaMemcpy(s.fc.m.q, src.q, cells * 4, cudaMemcpyDeviceToDevice));
   SCK(cudaMemcpy(s.fc.m.al, src.al, cells * 8, cudaMemcpyDeviceToDevice));
   SCK(cudaMemcpy(s.fc.m.csr, src.csr, cells * 8, cudaMemcpyDeviceToDevice));
+  SCK(cudaMemcpy(s.fc.m.lists, src.lists, (size_t)src.V * list_stride(src.K) * 8, cudaMemcpyDeviceToDevice));
   SCK(cudaMemcpy(s.fc.m.A, src.A, (size_t)src.V * 8, cudaMemcpyDeviceToDevice));
   SCK(cudaMemcpy(s.fc.m.nnz, src.nnz, (size_t)src.V * 4, cudaMemcpyDeviceToDevice));
   SCK(cudaDeviceSynchronize());
+  if ((rc = choose_walk(s))) return rc;
   *handle = sv.release();
   return GPULDA_OK;
 }
@@ -821,6 +898,7 @@ extern "C" int gpulda_serve_create_from_phi(const GpuldaServeArgs* args, uint32_
   cudaFree(S);
   if (scratch) cudaFree(scratch);
   if (e != cudaSuccess) return report_cuda_error(e, "serving model alias build");
+  if ((rc = choose_walk(s))) return rc;
   *handle = sv.release();
   return GPULDA_OK;
 }

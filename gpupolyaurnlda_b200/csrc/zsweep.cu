@@ -2,6 +2,8 @@
 // src/cu/topics.cu:36-105, with count_topics / compute_product_cumsum /
 // draw_wary_search / draw_alias from src/cu/topics.cuh:63-192).
 //
+// The sweep for words with long lists of topics (zsweep_words.cu has the one for
+// short lists, and which of the two runs when).
 // One warp per document; documents come from a global work counter (longest
 // first when an order is given).  The document's counts and the per-token
 // draw are in doc_counts.cuh; this kernel adds the count rebuild
@@ -19,7 +21,6 @@ namespace {
 
 constexpr u32 kMaxDocLen = 65535u;
 constexpr size_t kZMaxSmem = 200 * 1024;
-constexpr size_t kTokStageBytes = 32 * 32;  // per warp: 32 tokens x 32 bytes
 
 struct ZKernelArgs {
   ModelDev m;
@@ -45,6 +46,7 @@ template <bool BATCH, bool LL>
 __global__ void __launch_bounds__(256, 4) z_sweep_kernel(ZKernelArgs a) {
   extern __shared__ __align__(16) unsigned char zsm[];
   __shared__ unsigned long long blk_stats[4];  // tokens, documents, sparse work, sparse draws
+  if (a.z.shares && !mostly_long_lists(a.z.shares)) return;  // the other sweep's
   if (threadIdx.x < 4) blk_stats[threadIdx.x] = 0;
   __syncthreads();
   const ModelDev& m = a.m;
