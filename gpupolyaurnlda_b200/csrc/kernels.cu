@@ -56,6 +56,9 @@ __device__ __forceinline__ void phi_rows(u32 K, u64 c0, u64 c1, u32* __restrict_
                                          unsigned long long* s_sum) {
   for (u64 gi = c0 / 4 + threadIdx.x; gi * 4 < c1; gi += blockDim.x) {
     const u64 cb = gi * 4;
+    // topic of the group's first cell (c0 is a row's start; a range has fewer
+    // than 2^32 - 4 cells, so 32 bits hold its cells' numbers)
+    u32 k = (cb >= c0 ? (u32)(cb - c0) : K - (u32)(c0 - cb) % K) % K;
     const U4 r = draw4(gi, t, kStreamPhi, 0, key0, key1);
     const bool whole = cb >= c0 && cb + 4 <= c1;
     u32 nv[4];
@@ -79,18 +82,19 @@ __device__ __forceinline__ void phi_rows(u32 K, u64 c0, u64 c1, u32* __restrict_
 #pragma unroll
     for (u32 u = 0; u < 4; ++u) {
       const u64 c = cb + u;
-      if (c < c0 || c >= c1) continue;
-      if (!whole) {
-        q[c] = xv[u];
-        n[c] = 0;
+      if (c >= c0 && c < c1) {
+        if (!whole) {
+          q[c] = xv[u];
+          n[c] = 0;
+        }
+        if (xv[u]) {
+          if (s_sum)
+            atomicAdd(&s_sum[k], (unsigned long long)xv[u]);
+          else
+            atomicAdd((unsigned long long*)&S[k], (unsigned long long)xv[u]);
+        }
       }
-      if (xv[u]) {
-        const u32 k = (u32)(c % K);
-        if (s_sum)
-          atomicAdd(&s_sum[k], (unsigned long long)xv[u]);
-        else
-          atomicAdd((unsigned long long*)&S[k], (unsigned long long)xv[u]);
-      }
+      k = k + 1 == K ? 0u : k + 1;
     }
   }
 }
@@ -116,13 +120,15 @@ __global__ void __launch_bounds__(256, 4) phi_draw_kernel(ModelDev m, u32 t, u32
 }
 
 // Phi draw for K a multiple of 4 (the common case): block (bx, by) draws rows
-// [bx * rows, (bx + 1) * rows) of topics [1024 by, 1024 (by + 1)); thread i
-// owns the four topics 1024 by + 4 i .. + 3 for every row of the block, so its
-// 16-byte loads and stores of consecutive threads are contiguous, and it keeps
-// the four per-topic sums in registers across the rows: the normalisers need
-// no shared memory and one 64-bit atomic per (block, topic) at the end.  Cell
-// c = w K + k uses word c & 3 of Philox block c >> 2, exactly as phi_rows, so
-// the draws are the same.
+// [bx * rows, (bx + 1) * rows) of topics [1024 by, 1024 (by + 1)).  A thread
+// owns four consecutive topics, of every row of the block or, where a row's
+// groups of four do not fill the block, of every 256 / (K / 4)-th: its 16-byte
+// loads and stores are contiguous with its neighbours', and it keeps the four
+// per-topic sums in registers across its rows (then one 64-bit atomic per block
+// and topic, after a sum over the threads of a topic in shared memory where
+// there are several).  With one row at a time whatever K, a block of K=20 had 5
+// threads at work (K=20, V=5000: 1.7 ms, 36 us now).  Cell c = w K + k uses word
+// c & 3 of Philox block c >> 2, exactly as phi_rows, so the draws are the same.
 // Rows whose counts each thread loads before drawing any of them: the draw of
 // a row waits on its 16-byte load, so loads of several rows in flight hide
 // the memory latency one row at a time would expose.  With four rows the loop
@@ -131,12 +137,23 @@ __global__ void __launch_bounds__(256, 4) phi_draw_kernel(ModelDev m, u32 t, u32
 // one row at a time and four blocks per SM).
 constexpr u32 kPhiRowsInFlight = 4;
 
+// MANY: several rows side by side (K <= 512: one tile).
+template <bool MANY>
 __global__ void __launch_bounds__(256, 2) phi_draw_cols_kernel(ModelDev m, u32 t, u32 rows_per_block) {
+  __shared__ unsigned long long s_sum[MANY ? 512 : 1];
   const u32 K = m.K;
-  const u32 k0 = blockIdx.y * 1024u + 4u * threadIdx.x;
-  if (k0 >= K) return;
-  const u32 w0 = blockIdx.x * rows_per_block;
-  const u32 w1 = min(m.V, w0 + rows_per_block);
+  const u32 groups = MANY ? K / 4 : 256u;         // of a row
+  const u32 side = MANY ? 256u / groups : 1u;     // rows side by side
+  const u32 r = MANY ? threadIdx.x / groups : 0u;  // this thread's among them
+  const u32 k0 = blockIdx.y * 1024u + 4u * (threadIdx.x - r * groups);
+  if (MANY) {
+    for (u32 i = threadIdx.x; i < K; i += 256) s_sum[i] = 0;
+    __syncthreads();
+  } else if (k0 >= K) {
+    return;
+  }
+  const u32 w0 = blockIdx.x * rows_per_block + r;
+  const u32 w1 = !MANY || r < side ? min(m.V, blockIdx.x * rows_per_block + rows_per_block) : 0u;
   const double beta = (double)m.beta;
   // Most cells hold no tokens, and for n = 0 the inversion returns 0 exactly
   // when the cell's word is below the table's first CDF entry: that entry in
@@ -144,15 +161,16 @@ __global__ void __launch_bounds__(256, 2) phi_draw_cols_kernel(ModelDev m, u32 t
   // 4.06 against 3.86 TB/s; no difference at K=1000).
   const u32 cdf00 = __ldg(m.tables.cdf);
   u64 acc[4] = {0, 0, 0, 0};
-  for (u32 wb = w0; wb < w1; wb += kPhiRowsInFlight) {
+  for (u32 wb = w0; wb < w1; wb += kPhiRowsInFlight * side) {
     uint4 v[kPhiRowsInFlight];
 #pragma unroll
     for (u32 i = 0; i < kPhiRowsInFlight; ++i)
-      v[i] = wb + i < w1 ? *reinterpret_cast<const uint4*>(m.n + (u64)(wb + i) * K + k0) : make_uint4(0, 0, 0, 0);
+      v[i] = wb + i * side < w1 ? *reinterpret_cast<const uint4*>(m.n + (u64)(wb + i * side) * K + k0)
+                                : make_uint4(0, 0, 0, 0);
 #pragma unroll
     for (u32 i = 0; i < kPhiRowsInFlight; ++i) {
-      if (wb + i >= w1) break;
-      const u64 cb = (u64)(wb + i) * K + k0;
+      if (wb + i * side >= w1) break;
+      const u64 cb = (u64)(wb + i * side) * K + k0;
       const U4 r = draw4(cb >> 2, t, kStreamPhi, 0, m.key0, m.key1);
       const u32 nv[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
       u32 xv[4];
@@ -167,6 +185,17 @@ __global__ void __launch_bounds__(256, 2) phi_draw_cols_kernel(ModelDev m, u32 t
       *reinterpret_cast<uint4*>(m.q + cb) = make_uint4(xv[0], xv[1], xv[2], xv[3]);
       *reinterpret_cast<uint4*>(m.n + cb) = make_uint4(0, 0, 0, 0);
     }
+  }
+  if (MANY) {
+    if (r < side) {
+#pragma unroll
+      for (u32 u = 0; u < 4; ++u)
+        if (acc[u]) atomicAdd(&s_sum[k0 + u], (unsigned long long)acc[u]);
+    }
+    __syncthreads();
+    for (u32 i = threadIdx.x; i < K; i += 256)
+      if (s_sum[i]) atomicAdd((unsigned long long*)&m.S[i], s_sum[i]);
+    return;
   }
 #pragma unroll
   for (u32 u = 0; u < 4; ++u)
@@ -581,14 +610,24 @@ void launch_bump(u32* t, cudaStream_t s) { bump_kernel<<<1, 1, 0, s>>>(t); }
 
 void launch_phi_draw(const ModelDev& m, u32 t, cudaStream_t s) {
   if (m.K % 4 == 0) {
-    // rows per block: about 64 Ki cells per block, at least 8 rows
+    // Rows per block: about 64 Ki cells per block, at least 8 rows; fewer where
+    // that would leave SMs without a block (two are resident on each), down to
+    // what the threads have in flight.
     const u32 tiles = (m.K + 1023) / 1024;
-    const u32 rows = std::max<u32>(8u, 65536u / std::min<u32>(m.K, 1024u));
+    const u32 side = m.K <= 512 ? 256u / (m.K / 4) : 1u;
+    const u32 fill = (u32)((u64)m.V * tiles / (4u * device_sm_count()));
+    const u32 rows = std::max<u32>(kPhiRowsInFlight * side,
+                                   std::min<u32>(std::max<u32>(8u, 65536u / std::min<u32>(m.K, 1024u)), fill));
     const dim3 grid((m.V + rows - 1) / rows, tiles);
-    phi_draw_cols_kernel<<<grid, 256, 0, s>>>(m, t, rows);
+    if (side > 1)
+      phi_draw_cols_kernel<true><<<grid, 256, 0, s>>>(m, t, rows);
+    else
+      phi_draw_cols_kernel<false><<<grid, 256, 0, s>>>(m, t, rows);
     return;
   }
-  const u32 rows = std::max<u32>(1u, 65536u / m.K);
+  // (at most 64 Ki cells a block, and blocks for every SM: K=333, V=20011 went
+  // from 102 blocks and 320 us to 58 us, with 32-bit topic arithmetic)
+  const u32 rows = std::max<u32>(1u, std::min<u32>(65536u / m.K, m.V / (16u * device_sm_count())));
   const u32 blocks = (m.V + rows - 1) / rows;
   const int smem_sums = m.K <= 8192;
   const size_t smem = smem_sums ? (size_t)m.K * 8 : 0;
