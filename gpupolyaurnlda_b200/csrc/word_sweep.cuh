@@ -283,9 +283,10 @@ static __device__ __noinline__ u32 long_draw(const uint16_t* cnt, Staged c, u32 
 // so they are issued a token ahead.  Longer lists go through long_draw.  Drawn
 // topics go to gs[2 j].x (with kWordSparse); returns counts_move's answers, a bit
 // per token.
-template <u32 W>
-__device__ __forceinline__ u32 draw_chunk(const WordDoc& dc, uint4* gs, u32 n, u32 lane) {
-  constexpr u32 NP = W == 8 ? 10 : W == 16 ? 5 : 3;  // pairs per lane of a list of kShortList entries
+//
+// This one for four documents to a warp.
+__device__ __forceinline__ u32 draw_chunk_quarter(const WordDoc& dc, uint4* gs, u32 n, u32 lane) {
+  constexpr u32 W = 8, NP = 10;  // pairs per lane of a list of kShortList entries
   const u32 l = group_lane<W>(lane);
   const uint16_t* cnt = dc.cnt;
   u32 h = 0;
@@ -293,19 +294,20 @@ __device__ __forceinline__ u32 draw_chunk(const WordDoc& dc, uint4* gs, u32 n, u
 #pragma unroll
   for (u32 p = 0; p < NP; ++p) pre[p] = make_ulonglong2(0, 0);
   Staged s = staged(gs, 0);
-  Run run;
-  bool wide;
+  u32 c8 = 0;  // pairs per lane
+  bool on = false, wide;
   auto fetch = [&]() {
     wide = __any_sync(kFullMask, s.nw() > kShortList);
     if (wide) return;
-    run = lane_run<W>(s.nw(), l);
-    const ulonglong2* at = s.list() + run.at;
-    if (run.on) {
+    c8 = ((s.nw() + 31) >> 5) << 1;  // list_pairs, or 0 for an empty list
+    on = 2 * c8 * l < s.nw();
+    const ulonglong2* at = s.list() + l;
+    if (on) {
 #pragma unroll
-      for (u32 p = 0; p < NP; p += W == 8 ? 2 : 1)
-        if (p == 0 || run.n > p) {
+      for (u32 p = 0; p < NP; p += 2)
+        if (p == 0 || c8 > p) {
           pre[p] = __ldg(at + 8 * p);
-          if (W == 8) pre[(p + 1) % NP] = __ldg(at + 8 * p + 8);
+          pre[p + 1] = __ldg(at + 8 * p + 8);
         }
     }
   };
@@ -319,32 +321,15 @@ __device__ __forceinline__ u32 draw_chunk(const WordDoc& dc, uint4* gs, u32 n, u
       s = staged(gs, j + 1);
       fetch();
     } else {
-      const Run rj = run;
+      const u32 cj = c8;
       u64 x = 0;
-      u64 m[2 * NP];
-      u32 T[2 * NP];
-      if (W == 32) {
-        // (a lane whose run is off or shorter has entries of an earlier token
-        // there: what it makes of them is dropped)
-#pragma unroll
-        for (u32 p = 0; p < NP; ++p) {
-          T[2 * p] = (u32)pre[p].x;
-          T[2 * p + 1] = (u32)pre[p].y;
-          if (p < 1 || __any_sync(kFullMask, run.n > p)) {
-            m[2 * p] = x + (run.n > p ? mass_of(cnt, pre[p].x) : 0ull);
-            x = m[2 * p + 1] = m[2 * p] + (run.n > p ? mass_of(cnt, pre[p].y) : 0ull);
-          } else {
-            m[2 * p] = m[2 * p + 1] = x;
-          }
-        }
-        if (!run.on) x = 0;
-      } else if (run.on) {
+      if (on) {
         u64 y = 0;
 #pragma unroll
-        for (u32 p = 0; p < NP; p += W == 8 ? 2 : 1)
-          if (p == 0 || run.n > p) {
+        for (u32 p = 0; p < NP; p += 2)
+          if (p == 0 || c8 > p) {
             x += mass_of(cnt, pre[p]);
-            if (W == 8) y += mass_of(cnt, pre[(p + 1) % NP]);
+            y += mass_of(cnt, pre[p + 1]);
           }
         x += y;
       }
@@ -356,60 +341,123 @@ __device__ __forceinline__ u32 draw_chunk(const WordDoc& dc, uint4* gs, u32 n, u
       const bool sp = sparse_test(c.r0(), c.aA(), B);
       u64 t = scale_u32(c.r1(), B);
       u32 f = __popc(group_ballot<W>(incl <= t, lane)) & (W - 1);
-      if (W == 32) {
-        // the crossing lane has the prefixes of its entries
-        t -= incl - x;
-        k = T[2 * NP - 1];
-#pragma unroll
-        for (u32 i = 2 * NP - 1; i-- > 0;)
-          if (m[i] > t) k = T[i];
-      } else {
-        // the crossing lane's run is spread over the group, a pair per lane
-        // (two, where runs are longer than the group)
-        t -= group_get<W>(incl - x, f);
-        const u32 at = group_get<W>(rj.at, f), len = group_get<W>(rj.n, f);
-        const ulonglong2* list = c.list() + at;
-        u64 m0 = 0, m1 = 0;
-        u32 k0 = 0, k1 = 0;
-        if (NP <= W) {
-          if (sp && l < len) {
-            const ulonglong2 e = __ldg(list + 8 * l);
-            k0 = (u32)e.x;
-            k1 = (u32)e.y;
-            m0 = mass_of(cnt, e.x);
-            m1 = mass_of(cnt, e.y);
-          }
-          const u64 in2 = group_scan<W>(m0 + m1);
-          f = __popc(group_ballot<W>(in2 <= t, lane)) & (W - 1);
-          k = in2 - m1 > t ? k0 : k1;
-        } else {
-          u64 m2 = 0, m3 = 0;
-          u32 k2 = 0, k3 = 0;
-          if (sp && 2 * l < len) {  // runs have an even number of pairs here
-            const ulonglong2 e = __ldg(list + 16 * l), g = __ldg(list + 16 * l + 8);
-            k0 = (u32)e.x;
-            k1 = (u32)e.y;
-            k2 = (u32)g.x;
-            k3 = (u32)g.y;
-            m0 = mass_of(cnt, e.x);
-            m1 = m0 + mass_of(cnt, e.y);
-            m2 = m1 + mass_of(cnt, g.x);
-            m3 = m2 + mass_of(cnt, g.y);
-          }
-          const u64 in2 = group_scan<W>(m3);
-          f = __popc(group_ballot<W>(in2 <= t, lane)) & (W - 1);
-          const u64 u = t - (in2 - m3);
-          k = k3;
-          if (m2 > u) k = k2;
-          if (m1 > u) k = k1;
-          if (m0 > u) k = k0;
-        }
+      // the crossing lane's run (an even number of pairs, at most 10) is spread
+      // over the group, two pairs per lane
+      t -= group_get<W>(incl - x, f);
+      const ulonglong2* list = c.list() + f;
+      u64 m0 = 0, m1 = 0, m2 = 0, m3 = 0;
+      u32 k0 = 0, k1 = 0, k2 = 0, k3 = 0;
+      if (sp && 2 * l < cj) {
+        const ulonglong2 e = __ldg(list + 16 * l), g = __ldg(list + 16 * l + 8);
+        k0 = (u32)e.x;
+        k1 = (u32)e.y;
+        k2 = (u32)g.x;
+        k3 = (u32)g.y;
+        m0 = mass_of(cnt, e.x);
+        m1 = m0 + mass_of(cnt, e.y);
+        m2 = m1 + mass_of(cnt, g.x);
+        m3 = m2 + mass_of(cnt, g.y);
       }
+      const u64 in2 = group_scan<W>(m3);
+      f = __popc(group_ballot<W>(in2 <= t, lane)) & (W - 1);
+      const u64 u = t - (in2 - m3);
+      k = k3;
+      if (m2 > u) k = k2;
+      if (m1 > u) k = k1;
+      if (m0 > u) k = k0;
       k = group_get<W>(k, f);
       k = sp ? k | kWordSparse : c.kd();
     }
     if (l == 0) gs[2 * j].x = k;
     if (counts_move<W>(dc, k & 0xffffu, s.z(), l)) h |= 1u << j;
+  }
+  return h;
+}
+
+// And for one document to a warp, where the time from one token to the next is
+// what counts: every instruction between them adds to it.  Lists of up to 64
+// entries, a pair per lane, have steps of their own.
+__device__ __forceinline__ u32 draw_chunk_whole(const WordDoc& dc, uint4* gs, u32 n, u32 lane) {
+  constexpr u32 W = 32, NP = 3;  // pairs per lane of a list of kShortList entries
+  const uint16_t* cnt = dc.cnt;
+  // the lane's pair of a list of up to 32 entries (lanes 0..15) and up to 64
+  const u32 at2 = (lane & 1) * 8 + (lane >> 1), at4 = (lane & 3) * 8 + (lane >> 2);
+  u32 h = 0;
+  ulonglong2 pre[NP];
+#pragma unroll
+  for (u32 p = 0; p < NP; ++p) pre[p] = make_ulonglong2(0, 0);
+  Staged s = staged(gs, 0);
+  Run run{0, 0, false};
+  u32 kind = 0;  // 0: up to 64 entries, 1: up to kShortList, 2: longer
+  auto fetch = [&]() {
+    const u32 nw = s.nw();
+    if (!__any_sync(kFullMask, nw > 64)) {
+      kind = 0;
+      run.on = 2 * lane < nw;
+      if (run.on) pre[0] = __ldg(s.list() + (nw <= 32 ? at2 : at4));
+    } else if (!__any_sync(kFullMask, nw > kShortList)) {
+      kind = 1;
+      run = lane_run<W>(nw, lane);
+      const ulonglong2* at = s.list() + run.at;
+#pragma unroll
+      for (u32 p = 0; p < NP; ++p)
+        if (run.on && run.n > p) pre[p] = __ldg(at + 8 * p);
+    } else {
+      kind = 2;
+    }
+  };
+  fetch();
+#pragma unroll 2
+  for (u32 j = 0; j < n; ++j) {
+    const Staged c = s;
+    u32 k;
+    if (kind == 0) {
+      // (a lane past the list's end has entries of an earlier token)
+      const u32 T0 = (u32)pre[0].x, T1 = (u32)pre[0].y;
+      const u64 m0 = mass_of(cnt, pre[0].x);
+      const u64 m1 = m0 + mass_of(cnt, pre[0].y);
+      const u64 x = run.on ? m1 : 0ull;
+      s = staged(gs, j + 1);
+      fetch();
+      const u64 incl = group_scan<W>(x);
+      const u64 B = group_get<W>(incl, W - 1);
+      const bool sp = sparse_test(c.r0(), c.aA(), B);
+      const u64 t = scale_u32(c.r1(), B);
+      const u32 f = __popc(__ballot_sync(kFullMask, incl <= t)) & (W - 1);
+      k = group_get<W>(m0 > t - (incl - x) ? T0 : T1, f);
+      k = sp ? k | kWordSparse : c.kd();
+    } else if (kind == 1) {
+      u64 m[2 * NP];
+      u32 T[2 * NP];
+      u64 x = 0;
+#pragma unroll
+      for (u32 p = 0; p < NP; ++p) {
+        T[2 * p] = (u32)pre[p].x;
+        T[2 * p + 1] = (u32)pre[p].y;
+        m[2 * p] = x + (run.n > p ? mass_of(cnt, pre[p].x) : 0ull);
+        x = m[2 * p + 1] = m[2 * p] + (run.n > p ? mass_of(cnt, pre[p].y) : 0ull);
+      }
+      if (!run.on) x = 0;
+      s = staged(gs, j + 1);
+      fetch();
+      const u64 incl = group_scan<W>(x);
+      const u64 B = group_get<W>(incl, W - 1);
+      const bool sp = sparse_test(c.r0(), c.aA(), B);
+      const u64 t = scale_u32(c.r1(), B), u = t - (incl - x);
+      const u32 f = __popc(__ballot_sync(kFullMask, incl <= t)) & (W - 1);
+      k = T[2 * NP - 1];
+#pragma unroll
+      for (u32 i = 2 * NP - 1; i-- > 0;)
+        if (m[i] > u) k = T[i];
+      k = group_get<W>(k, f);
+      k = sp ? k | kWordSparse : c.kd();
+    } else {
+      k = long_draw<W>(cnt, c, lane);
+      s = staged(gs, j + 1);
+      fetch();
+    }
+    if (lane == 0) gs[2 * j].x = k;
+    if (counts_move<W>(dc, k & 0xffffu, s.z(), lane)) h |= 1u << j;
   }
   return h;
 }
@@ -494,7 +542,7 @@ __device__ __forceinline__ void sweep_doc(WordDoc& dc, uint4* stage, const Model
     dc.nz -= (group_ballot<W>(gone, lane) >> 1) & 1u;
     const u32 left = __ballot_sync(kFullMask, z != dc.none);
     const u32 n = W == 32 ? 32u - __clz((int)left) : W;
-    const u32 hist = draw_chunk<W>(dc, gs, n, lane);
+    const u32 hist = W == 8 ? draw_chunk_quarter(dc, gs, n, lane) : draw_chunk_whole(dc, gs, n, lane);
     __syncwarp();
     // results: the lane's topic, and the document's distinct topics without it
     const u32 kk = gs[2 * l].x;
