@@ -482,6 +482,85 @@ __global__ void __launch_bounds__(1024) doc_offsets_kernel(const u32* __restrict
 }
 
 // ---------------------------------------------------------------------------
+// Document offsets, and the documents longest first, for lengths that are on
+// the device only.  Three launches over blocks of kPlanDocs documents: token
+// sums per block and a histogram of lengths; a scan of both; offsets and places
+// in the order.  The order is by length bins (exact below 512 tokens, 128 tokens
+// wide above), in no particular order inside a bin.  Bound by its launches (three
+// of 3 us at 6e4 documents; one block scanning them all took 14 us).
+// ---------------------------------------------------------------------------
+constexpr u32 kPlanThreads = 256, kPlanDocs = 4096, kPlanBins = 1024;
+static_assert(kPlanMostDocs <= kPlanDocs * kPlanBins, "the scan's block takes a block sum per thread");
+
+// The bin of a length, longest first.
+__host__ __device__ __forceinline__ u32 plan_bin(u32 len) {
+  const u32 up = len < 512 ? len : 512 + (len - 512) / 128;
+  return kPlanBins - 1 - (up < kPlanBins ? up : kPlanBins - 1);
+}
+
+__global__ void __launch_bounds__(kPlanThreads) doc_survey_kernel(const u32* __restrict__ d_len, u32 n_docs,
+                                                                  DocPlan plan) {
+  __shared__ u32 hist[kPlanBins];
+  __shared__ u64 sh[33];
+  for (u32 i = threadIdx.x; i < kPlanBins; i += kPlanThreads) hist[i] = 0;
+  __syncthreads();
+  u64 sum = 0;
+  const u32 d1 = min(n_docs, (blockIdx.x + 1) * kPlanDocs);
+  for (u32 d = blockIdx.x * kPlanDocs + threadIdx.x; d < d1; d += kPlanThreads) {
+    const u32 len = d_len[d];
+    sum += len;
+    atomicAdd(hist + plan_bin(len), 1u);
+  }
+  sum = block_sum_u64(sum, sh);  // (orders the histogram before its flush)
+  if (threadIdx.x == 0) plan.sums[blockIdx.x] = sum;
+  for (u32 i = threadIdx.x; i < kPlanBins; i += kPlanThreads)
+    if (hist[i]) atomicAdd(plan.bins + i, hist[i]);
+}
+
+// plan.sums and plan.bins become exclusive prefixes; *n_long receives the
+// documents in the bins before long_bin's end.
+__global__ void __launch_bounds__(kPlanBins) doc_scan_kernel(u32 n_blocks, u32 long_bin, DocPlan plan) {
+  __shared__ u64 sh[33];
+  const u32 i = threadIdx.x;
+  u64 total;
+  const u64 s0 = block_excl_scan_u64(i < n_blocks ? plan.sums[i] : 0, sh, &total);
+  const u32 here = plan.bins[i];
+  const u64 b0 = block_excl_scan_u64(here, sh, &total);
+  if (i < n_blocks) plan.sums[i] = s0;
+  plan.bins[i] = (u32)b0;
+  if (i == long_bin) *plan.n_long = (u32)b0 + here;
+}
+
+__global__ void __launch_bounds__(kPlanThreads) doc_place_kernel(const u32* __restrict__ d_len, u32 n_docs,
+                                                                 u32* __restrict__ d_idx, u32* __restrict__ order,
+                                                                 DocPlan plan) {
+  __shared__ u32 lens[kPlanDocs];
+  __shared__ u32 bins[kPlanBins];  // the block's documents of a bin, then their next place
+  __shared__ u64 sh[33];
+  const u32 d0 = blockIdx.x * kPlanDocs, n = min(kPlanDocs, n_docs - d0);
+  for (u32 i = threadIdx.x; i < kPlanBins; i += kPlanThreads) bins[i] = 0;
+  __syncthreads();
+  for (u32 i = threadIdx.x; i < n; i += kPlanThreads) {
+    lens[i] = d_len[d0 + i];
+    atomicAdd(bins + plan_bin(lens[i]), 1u);
+  }
+  __syncthreads();
+  for (u32 i = threadIdx.x; i < kPlanBins; i += kPlanThreads)
+    if (bins[i]) bins[i] = atomicAdd(plan.bins + i, bins[i]);
+  constexpr u32 kEach = kPlanDocs / kPlanThreads;
+  const u32 i0 = min(n, threadIdx.x * kEach), i1 = min(n, i0 + kEach);
+  u64 s = 0;
+  for (u32 i = i0; i < i1; ++i) s += lens[i];
+  u64 total;
+  u64 off = plan.sums[blockIdx.x] + block_excl_scan_u64(s, sh, &total);  // (orders the bins' places too)
+  for (u32 i = i0; i < i1; ++i) {
+    d_idx[d0 + i] = off < 0xffffffffull ? (u32)off : 0xffffffffu;  // as doc_offsets_kernel
+    off += lens[i];
+    order[atomicAdd(bins + plan_bin(lens[i]), 1u)] = d0 + i;
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Count rebuild n[w][z] += 1 over a token range (reference: the atomicAdd per
 // token at the end of sample_topics, src/cu/topics.cu:95).  Tokens are read
 // four at a time (16-byte loads of w and z); per load slot the warp groups
@@ -688,6 +767,22 @@ void launch_count_rebuild(u32* n, const u32* w, const u32* z, u64 n_tokens, u32 
 void launch_doc_offsets(const u32* d_len, u32* d_idx, u32 n_docs, cudaStream_t s) {
   if (!n_docs) return;
   doc_offsets_kernel<<<1, 1024, 0, s>>>(d_len, d_idx, n_docs);
+}
+
+cudaError_t launch_doc_plan(const u32* d_len, u32* d_idx, u32* order, u32 n_docs, u32 long_len, const DocPlan& plan,
+                            cudaStream_t s) {
+  const cudaError_t e = cudaMemsetAsync(plan.bins, 0, kPlanBins * 4, s);
+  if (e != cudaSuccess) return e;
+  const u32 blocks = (n_docs + kPlanDocs - 1) / kPlanDocs;
+  doc_survey_kernel<<<blocks, kPlanThreads, 0, s>>>(d_len, n_docs, plan);
+  doc_scan_kernel<<<1, kPlanBins, 0, s>>>(blocks, plan_bin(long_len), plan);
+  doc_place_kernel<<<blocks, kPlanThreads, 0, s>>>(d_len, n_docs, d_idx, order, plan);
+  return cudaGetLastError();
+}
+
+DocPlan doc_plan_at(u32* scratch) {
+  static_assert(kPlanWords == 2 * kPlanBins + kPlanBins + 16, "DocPlan's arrays");
+  return DocPlan{(u64*)scratch, scratch + 2 * kPlanBins, scratch + 3 * kPlanBins};
 }
 
 void launch_debug_philox(const u32* ctr, u32 n, u32 k0, u32 k1, u32* out, cudaStream_t s) {

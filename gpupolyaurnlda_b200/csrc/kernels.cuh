@@ -145,6 +145,7 @@ struct ZLaunch {
   // The shares of words with short and long lists that decide which of two
   // launches sweeps; null: this one does.
   const u64* shares = nullptr;
+  const u32* n_long_dev = nullptr;  // documents that take a warp each, where the device counted them
   // Documents that the launch hands on: token reached << 32 | document, and
   // their number.  The list sweep writes them, the sweep of the rest reads
   // them in place of `order`.
@@ -185,6 +186,19 @@ void launch_count_rebuild(u32* n, const u32* w, const u32* z, u64 n_tokens, u32 
                           cudaStream_t s);
 // d_idx = exclusive scan of d_len.
 void launch_doc_offsets(const u32* d_len, u32* d_idx, u32 n_docs, cudaStream_t s);
+// The same offsets and the documents' order, longest first, for at most
+// kPlanMostDocs documents; *plan.n_long receives how many have at least about
+// long_len tokens (the first of the order).
+constexpr u32 kPlanMostDocs = 1u << 20;
+constexpr u32 kPlanWords = 3 * 1024 + 16;
+struct DocPlan {
+  u64* sums;
+  u32* bins;
+  u32* n_long;
+};
+DocPlan doc_plan_at(u32* scratch);  // of kPlanWords words, 8-byte aligned
+cudaError_t launch_doc_plan(const u32* d_len, u32* d_idx, u32* order, u32 n_docs, u32 long_len, const DocPlan& plan,
+                            cudaStream_t s);
 // ZLaunch.flags bits.
 constexpr u32 kZFlagLoglik = 1u;  // accumulate the joint log-likelihood
 

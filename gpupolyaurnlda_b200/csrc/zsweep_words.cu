@@ -187,9 +187,10 @@ __global__ void __launch_bounds__(256, 2) z_sweep_words_kernel(ZWordArgs a) {
     return __shfl_sync(kFullMask, i, 0);
   };
   u32 item = claim();
-  for (; item < a.n_long; item = claim()) sweep_documents<32, BATCH, LL>(a, wsm, item, blk_stats, sums, lane);
+  const u32 n_long = p.n_long_dev ? *p.n_long_dev : a.n_long;
+  for (; item < n_long; item = claim()) sweep_documents<32, BATCH, LL>(a, wsm, item, blk_stats, sums, lane);
   while (true) {
-    const u64 first = a.n_long + 4 * (u64)(item - a.n_long);
+    const u64 first = n_long + 4 * (u64)(item - n_long);
     if (first >= p.n_docs) break;
     sweep_documents<8, BATCH, LL>(a, wsm, first, blk_stats, sums, lane);
     item = claim();
@@ -228,7 +229,7 @@ void launch_impl(const ZWordArgs& a, cudaStream_t s, u32 wpb, u32 blocks_per_sm)
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, z_sweep_words_kernel<BATCH, LL>, 32 * wpb, smem);
   if (per_sm < 1) per_sm = 1;
   if (blocks_per_sm && (int)blocks_per_sm < per_sm) per_sm = (int)blocks_per_sm;
-  const u64 items = a.n_long + ((u64)a.z.n_docs - a.n_long + 3) / 4;
+  const u64 items = a.z.n_long_dev ? a.z.n_docs : a.n_long + ((u64)a.z.n_docs - a.n_long + 3) / 4;
   const u32 blocks = (u32)std::min<u64>((u64)device_sm_count() * per_sm, (items + wpb - 1) / wpb);
   z_sweep_words_kernel<BATCH, LL><<<blocks, 32 * wpb, smem, s>>>(a);
 }

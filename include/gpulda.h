@@ -265,8 +265,8 @@ int gpulda_debug_alias(const uint32_t* q, uint32_t K, uint64_t* table_out);
  * gpulda_counters and gpulda_debug_read synchronize the device.  Calls made
  * one after another from the host are ordered on the GPU as well.
  *
- * It allocates nothing: its scratch (document offsets and a work counter) is
- * a fixed device array of the library, 12 MiB + 256 B held by every GPU that
+ * It allocates nothing: its scratch (document offsets and order, work counters) is
+ * a fixed device array of the library, 16 MiB + 13 KiB held by every GPU that
  * loads the library until the process exits.  n_docs above
  * GPULDA_NOALLOC_MAX_DOCS is rejected with GPULDA_ERR_UNSUPPORTED.  The first
  * call on a device looks up that array's address, so make the first call
