@@ -305,6 +305,26 @@ __device__ void alias_build_block(const u64* ent, u32 n, u64 A, u64* vals, uint1
   }
 }
 
+// q = floor(x * 2^32 / S[k]), clamped to 32 bits.
+__device__ __forceinline__ u64 fixed_phi(u32 x, u32 k, const u64* __restrict__ S, const u64* __restrict__ Sinv) {
+  const u64 num = (u64)x << 32, sk = S[k];
+  u64 qq;
+  if (Sinv) {
+    // floor(num / sk) from the reciprocal: the multiply-high is at most 2
+    // below the quotient
+    qq = __umul64hi(num, Sinv[k]);
+    u64 r = num - qq * sk;
+    if (r >= sk) {
+      ++qq;
+      r -= sk;
+    }
+    if (r >= sk) ++qq;
+  } else {
+    qq = num / sk;
+  }
+  return qq > 0xffffffffULL ? 0xffffffffULL : qq;
+}
+
 // Per word: q = floor(x * 2^32 / S[k]) (clamped) written back densely; the
 // word's topics with q > 0 compacted in ascending order into its list
 // (q << 32 | k, which is also the alias build's input), the dense mass A, nnz,
@@ -313,6 +333,13 @@ __device__ void alias_build_block(const u64* ent, u32 n, u64 A, u64* vals, uint1
 // The alias build's scratch (10 bytes per nonzero) is shared memory when the
 // word's nonzeros fit smem_items, else the block's slice of global scratch.
 constexpr u32 kPerThread = 8;
+constexpr u32 kAliasWarps = 4;  // a block's, a word each
+// Most topics of a word that a warp takes (18 bytes each set how many warps are
+// resident); a longer word takes the block.  K=1000: 128, 256 and 512 take 218,
+// 210 and 243 us at the mid corpus; K=10000, whose words' lists are longer: 1350,
+// 900 and 700 us.
+inline u32 alias_items(u32 K) { return std::min(K, K <= kMapMinK ? 256u : 512u); }
+__host__ __device__ constexpr size_t alias_warp_bytes(u32 most) { return ((size_t)most * 18 + 15) & ~(size_t)15; }
 
 __device__ __forceinline__ void alias_word(u32 K, u32* __restrict__ qrow, const u64* __restrict__ S,
                                            const u64* __restrict__ Sinv, u64* alrow, u64* csrrow, u64* eighths, u64* A_out,
@@ -334,21 +361,7 @@ __device__ __forceinline__ void alias_word(u32 K, u32* __restrict__ qrow, const 
         const u32 x = qrow[k];
         if (x) {  // a zero count is already a zero q
           xsum += x;
-          const u64 num = (u64)x << 32, sk = S[k];
-          if (Sinv) {
-            // floor(num / sk) from the reciprocal: the multiply-high is at
-            // most 2 below the quotient
-            qq = __umul64hi(num, Sinv[k]);
-            u64 r = num - qq * sk;
-            if (r >= sk) {
-              ++qq;
-              r -= sk;
-            }
-            if (r >= sk) ++qq;
-          } else {
-            qq = num / sk;
-          }
-          if (qq > 0xffffffffULL) qq = 0xffffffffULL;
+          qq = fixed_phi(x, k, S, Sinv);
           qrow[k] = (u32)qq;
         }
       }
@@ -389,22 +402,216 @@ __device__ __forceinline__ void alias_word(u32 K, u32* __restrict__ qrow, const 
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(256) alias_build_kernel(ModelDev m, unsigned char* gscratch, size_t slice,
-                                                          u32 smem_items) {
+// The same by one warp, for a word of at most `most` topics.  Returns false
+// with nothing written for a word of more, or with a draw that rounds to q = 0
+// (a topic's sum above 2^32).  A trained word has some tens of topics, so a
+// block on it waited at barriers: six scans of eight warps' sums for one or two
+// entries a lane.  Here the row is only looked through for its nonzero draws,
+// and everything after works on those: ent[most] holds them, vals and idx are
+// the alias build's scratch, all the warp's own.  Bound by instructions (about
+// 1,500 a word beside 4 KB of row at K=1000).  1e5 words of 65 topics (K=1000)
+// 622 -> 212 us, 1.4e5 words 816 -> 259; 3e4 words, K=10000, 1185 -> 726 us
+// where the rows' 1.2 GB take 183; from a random start (50,000 words of 100
+// to 1000 topics) 337 -> 146.
+__device__ __forceinline__ bool alias_word_warp(u32 K, u32* qrow, const u64* __restrict__ S,
+                                                const u64* __restrict__ Sinv, u64* alrow, u64* csrrow, u64* eighths,
+                                                u64* A_out, u32* nnz_out, u64& x_all, u64& x_long, u64* ent, u64* vals,
+                                                uint16_t* idx, u32 most) {
+  constexpr u32 kInFlight = 4;  // loads of 512 bytes; 8 take registers and a resident block (mid 212 -> 239 us)
+  const u32 lane = threadIdx.x & 31, before = (1u << lane) - 1;
+  const u32 head = (u32)((uintptr_t)qrow >> 2) & 3;  // the row starts inside an aligned group of four
+  const u32 groups = (K + head + 3) / 4;
+  u32 n = 0;
+  for (u32 g0 = 0; g0 < groups; g0 += 32 * kInFlight) {
+    u32 v[kInFlight][4];
+#pragma unroll
+    for (u32 u = 0; u < kInFlight; ++u) {
+      const i32 k = (i32)(4 * (g0 + 32 * u + lane)) - (i32)head;
+      if (k >= 0 && k + 4 <= (i32)K) {
+        const uint4 x = *reinterpret_cast<const uint4*>(qrow + k);
+        v[u][0] = x.x, v[u][1] = x.y, v[u][2] = x.z, v[u][3] = x.w;
+      } else {
+#pragma unroll
+        for (i32 c = 0; c < 4; ++c) v[u][c] = k + c >= 0 && k + c < (i32)K ? qrow[k + c] : 0u;
+      }
+    }
+#pragma unroll
+    for (u32 u = 0; u < kInFlight; ++u) {
+      const u32 cnt = (v[u][0] != 0) + (v[u][1] != 0) + (v[u][2] != 0) + (v[u][3] != 0);
+      if (!__any_sync(kFullMask, cnt)) continue;
+      const u32 b0 = __ballot_sync(kFullMask, cnt & 1), b1 = __ballot_sync(kFullMask, cnt & 2),
+                b2 = __ballot_sync(kFullMask, cnt & 4);
+      u32 pos = n + __popc(b0 & before) + 2 * __popc(b1 & before) + 4 * __popc(b2 & before);
+      n += __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
+      if (n > most) return false;
+      const u32 k = 4 * (g0 + 32 * u + lane) - head;
+#pragma unroll
+      for (u32 c = 0; c < 4; ++c)
+        if (v[u][c]) ent[pos++] = ((u64)v[u][c] << 32) | (k + c);
+    }
+  }
+  __syncwarp();
+  u64 part = 0, xsum = 0;
+  bool zero = false;
+  for (u32 i = lane; i < n; i += 32) {
+    const u64 e = ent[i];
+    const u64 qq = fixed_phi((u32)(e >> 32), (u32)e, S, Sinv);
+    zero |= !qq;
+    part += qq;
+    xsum += e >> 32;
+    ent[i] = (qq << 32) | (u32)e;
+  }
+  if (__any_sync(kFullMask, zero)) return false;
+  __syncwarp();
+  const u64 A = warp_sum_u64(part);
+  x_all += xsum;
+  if (n > kShortList) x_long += xsum;
+  for (u32 i = lane; i < n; i += 32) {
+    const u64 e = ent[i];
+    qrow[(u32)e] = (u32)(e >> 32);
+    csrrow[i] = e;
+  }
+  if (eighths && n) {  // as alias_word
+    const u32 c = list_pairs(n), recip = list_recip(c);
+    const u32 end = (((n - 1) / 2 * recip >> 20) + 1) * 2 * c;
+    for (u32 i = lane; i < end; i += 32) eighths[list_pos(i, c, recip)] = i < n ? ent[i] : 0ull;
+  }
+  if (lane == 0) {
+    *A_out = A;
+    *nnz_out = n;
+  }
+  if (!n) return true;
+  // alias_build_block's steps
+  const u32 chunk = (n + 31) / 32, i0 = min(n, lane * chunk), i1 = min(n, i0 + chunk);
+  u32 nl = 0;
+  u64 dl = 0, eh = 0;
+  for (u32 i = i0; i < i1; ++i) {
+    const u64 wi = (u64)n * (ent[i] >> 32);
+    if (wi < A) {
+      ++nl;
+      dl += A - wi;
+    } else {
+      eh += wi - A;
+    }
+  }
+  u32 ol = nl;
+#pragma unroll
+  for (u32 d = 1; d < 32; d *= 2) {
+    const u32 o = __shfl_up_sync(kFullMask, ol, d);
+    if (lane >= d) ol += o;
+  }
+  const u32 nL = __shfl_sync(kFullMask, ol, 31);
+  ol -= nl;
+  u64 od = warp_incl_scan_u64(dl, lane);
+  const u64 Dtot = __shfl_sync(kFullMask, (unsigned long long)od, 31);
+  od -= dl;
+  u64 oe = warp_incl_scan_u64(eh, lane) - eh;
+  u32 oh = nL + i0 - ol;
+  for (u32 i = i0; i < i1; ++i) {
+    const u64 wi = (u64)n * (ent[i] >> 32);
+    if (wi < A) {
+      vals[ol] = od;
+      idx[ol++] = (uint16_t)i;
+      od += A - wi;
+    } else {
+      oe += wi - A;
+      vals[oh] = oe;
+      idx[oh++] = (uint16_t)i;
+    }
+  }
+  __syncwarp();
+  for (u32 j = lane; j < n; j += 32) {
+    const u32 i = idx[j];
+    const u64 e = ent[i], v = vals[j], own = e & 0xffffu;
+    if (j < nL) {
+      u32 lo = nL, hi = n - 1;  // the first heavy with E >= D
+      while (lo < hi) {
+        const u32 mid = (lo + hi) >> 1;
+        if (vals[mid] >= v) hi = mid; else lo = mid + 1;
+      }
+      alrow[i] = ((ent[idx[lo]] & 0xffffu) << 48) | (own << 32) | alias_threshold((u64)n * (e >> 32), A);
+    } else if (v < Dtot) {
+      u32 lo = 0, hi = nL - 1;  // the last light with D <= E (D_0 = 0)
+      while (lo < hi) {
+        const u32 mid = (lo + hi + 1) >> 1;
+        if (vals[mid] <= v) lo = mid; else hi = mid - 1;
+      }
+      const u64 d = A - (u64)n * (ent[idx[lo]] >> 32);
+      const u64 over = vals[lo] + d - v;
+      alrow[i] = ((ent[idx[j + 1]] & 0xffffu) << 48) | (own << 32) | alias_threshold(A - over, A);
+    } else {
+      alrow[i] = (own << 48) | (own << 32) | 0xffffffffu;
+    }
+  }
+  __syncwarp();
+  return true;
+}
+
+// A block's shared memory: its warps' scratch, or all of it for one word.
+struct AliasSmem {
+  u64 *ent, *vals;      // this warp's
+  uint16_t* idx;
+  u64* all_vals;        // the block's
+  uint16_t* all_idx;
+};
+__device__ __forceinline__ AliasSmem alias_smem(unsigned char* raw, u32 most, u32 all) {
+  AliasSmem a;
+  unsigned char* own = raw + (size_t)(threadIdx.x >> 5) * alias_warp_bytes(most);
+  a.ent = (u64*)own;
+  a.vals = a.ent + most;
+  a.idx = (uint16_t*)(a.vals + most);
+  a.all_vals = (u64*)raw;
+  a.all_idx = (uint16_t*)(a.all_vals + all);
+  return a;
+}
+
+constexpr u32 kNnzWide = 0xffffffffu;  // marks a word that its warp left to the block
+
+__global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_kernel(ModelDev m, unsigned char* gscratch, size_t slice,
+                                                                       u32 most, u32 smem_items) {
   extern __shared__ __align__(16) unsigned char s_raw[];
   __shared__ u64 sh[33], sh_shares[2];
-  const u32 K = m.K;
+  __shared__ u32 wide;
+  const u32 K = m.K, nw = blockDim.x >> 5, warp = threadIdx.x >> 5;
   if (threadIdx.x < 2) sh_shares[threadIdx.x] = 0;
+  if (threadIdx.x == 0) wide = 0;
   __syncthreads();
-  u64* s_vals = (u64*)s_raw;
-  uint16_t* s_idx = (uint16_t*)(s_vals + smem_items);
-  u64* g_vals = gscratch ? (u64*)(gscratch + (size_t)blockIdx.x * slice) : nullptr;
-  uint16_t* g_idx = gscratch ? (uint16_t*)(g_vals + K) : nullptr;
-  for (u32 w = blockIdx.x; w < m.V; w += gridDim.x) {
+  const AliasSmem sm = alias_smem(s_raw, most, smem_items);
+  u64 x_all = 0, x_long = 0;
+  const u64 step = (u64)gridDim.x * nw;
+  for (u64 w = (u64)blockIdx.x * nw + warp; w < m.V; w += step) {
     const size_t row = (size_t)w * K;
-    alias_word(K, m.q + row, m.S, m.Sinv, m.al + row, m.csr + row,
-               m.lists ? m.lists + (size_t)w * list_stride(K) : nullptr, m.A + w, m.shares ? sh_shares : nullptr, m.nnz + w, s_vals, s_idx, smem_items,
-               g_vals, g_idx, sh);
+    if (alias_word_warp(K, m.q + row, m.S, m.Sinv, m.al + row, m.csr + row,
+                        m.lists ? m.lists + (size_t)w * list_stride(K) : nullptr, m.A + w, m.nnz + w, x_all, x_long,
+                        sm.ent, sm.vals, sm.idx, most))
+      continue;
+    if ((threadIdx.x & 31) == 0) {
+      m.nnz[w] = kNnzWide;
+      wide = 1;
+    }
+    __syncwarp();
+  }
+  if (m.shares) {
+    x_all = warp_sum_u64(x_all);
+    x_long = warp_sum_u64(x_long);
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd((unsigned long long*)sh_shares, (unsigned long long)x_all);
+      atomicAdd((unsigned long long*)sh_shares + 1, (unsigned long long)x_long);
+    }
+  }
+  __syncthreads();
+  if (wide) {
+    u64* g_vals = gscratch ? (u64*)(gscratch + (size_t)blockIdx.x * slice) : nullptr;
+    uint16_t* g_idx = gscratch ? (uint16_t*)(g_vals + K) : nullptr;
+    for (u64 w0 = (u64)blockIdx.x * nw; w0 < m.V; w0 += step)
+      for (u64 w = w0; w < min((u64)m.V, w0 + nw); ++w) {
+        if (m.nnz[w] != kNnzWide) continue;
+        const size_t row = (size_t)w * K;
+        alias_word(K, m.q + row, m.S, m.Sinv, m.al + row, m.csr + row,
+                   m.lists ? m.lists + (size_t)w * list_stride(K) : nullptr, m.A + w, m.shares ? sh_shares : nullptr,
+                   m.nnz + w, sm.all_vals, sm.all_idx, smem_items, g_vals, g_idx, sh);
+      }
+    __syncthreads();
   }
   if (m.shares && threadIdx.x < 2)
     atomicAdd((unsigned long long*)m.shares + threadIdx.x, (unsigned long long)sh_shares[threadIdx.x]);
@@ -412,19 +619,47 @@ __global__ void __launch_bounds__(256) alias_build_kernel(ModelDev m, unsigned c
 
 // Batched alias build over global words [w0, w1) of any problems; shared
 // memory sized for the largest K among them.
-__global__ void __launch_bounds__(256) alias_build_batch_kernel(ModelDev ar, BatchPhiDev bp, u32 Kmax, u32 w0, u32 w1) {
+__global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_batch_kernel(ModelDev ar, BatchPhiDev bp, u32 most,
+                                                                             u32 Kmax, u32 w0, u32 w1) {
   extern __shared__ __align__(16) unsigned char s_raw[];
   __shared__ u64 sh[33], sh_shares[2];
+  __shared__ u32 wide;
+  const u32 nw = blockDim.x >> 5, warp = threadIdx.x >> 5;
   if (threadIdx.x < 2) sh_shares[threadIdx.x] = 0;
+  if (threadIdx.x == 0) wide = 0;
   __syncthreads();
-  u64* vals = (u64*)s_raw;
-  uint16_t* idx = (uint16_t*)(vals + Kmax);
-  for (u32 w = w0 + blockIdx.x; w < w1; w += gridDim.x) {
+  const AliasSmem sm = alias_smem(s_raw, most, Kmax);
+  u64 x_all = 0, x_long = 0;
+  const u64 step = (u64)gridDim.x * nw, first = (u64)w0 + (u64)blockIdx.x * nw;
+  for (u64 w = first + warp; w < w1; w += step) {
     const u32 pb = bp.wpid[w], K = bp.K[pb];
     const size_t row = bp.row_off[w];
-    alias_word(K, ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row,
-               ar.lists + bp.list_off[w], ar.A + w, sh_shares, ar.nnz + w, vals,
-               idx, Kmax, nullptr, nullptr, sh);
+    if (alias_word_warp(K, ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row,
+                        ar.lists + bp.list_off[w], ar.A + w, ar.nnz + w, x_all, x_long, sm.ent, sm.vals, sm.idx, most))
+      continue;
+    if ((threadIdx.x & 31) == 0) {
+      ar.nnz[w] = kNnzWide;
+      wide = 1;
+    }
+    __syncwarp();
+  }
+  x_all = warp_sum_u64(x_all);
+  x_long = warp_sum_u64(x_long);
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd((unsigned long long*)sh_shares, (unsigned long long)x_all);
+    atomicAdd((unsigned long long*)sh_shares + 1, (unsigned long long)x_long);
+  }
+  __syncthreads();
+  if (wide) {
+    for (u64 wb = first; wb < w1; wb += step)
+      for (u64 w = wb; w < min((u64)w1, wb + nw); ++w) {
+        if (ar.nnz[w] != kNnzWide) continue;
+        const u32 pb = bp.wpid[w], K = bp.K[pb];
+        const size_t row = bp.row_off[w];
+        alias_word(K, ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row, ar.lists + bp.list_off[w],
+                   ar.A + w, sh_shares, ar.nnz + w, sm.all_vals, sm.all_idx, Kmax, nullptr, nullptr, sh);
+      }
+    __syncthreads();
   }
   if (threadIdx.x < 2)
     atomicAdd((unsigned long long*)ar.shares + threadIdx.x, (unsigned long long)sh_shares[threadIdx.x]);
@@ -675,14 +910,14 @@ void launch_phi_draw_batch(const ModelDev& ar, const BatchPhiDev& bp, u32 n_bloc
 
 void launch_alias_build_batch(const ModelDev& ar, const BatchPhiDev& bp, u32 Kmax, u32 w0, u32 w1, cudaStream_t s) {
   if (w1 <= w0) return;
-  const u32 nt = alias_threads(Kmax);
-  const size_t need = alias_scratch_item_bytes(Kmax);
-  if (need > 48 * 1024) cudaFuncSetAttribute(alias_build_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
+  const u32 most = alias_items(Kmax);
+  const size_t need = std::max(kAliasWarps * alias_warp_bytes(most), alias_scratch_item_bytes(Kmax));
+  if (need > 47 * 1024) cudaFuncSetAttribute(alias_build_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, alias_build_batch_kernel, nt, need);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, alias_build_batch_kernel, 32 * kAliasWarps, need);
   if (per_sm < 1) per_sm = 1;
-  const u32 blocks = std::min<u32>(w1 - w0, (u32)(device_sm_count() * per_sm * 4));
-  alias_build_batch_kernel<<<blocks, nt, need, s>>>(ar, bp, Kmax, w0, w1);
+  const u32 blocks = std::min<u32>((w1 - w0 + kAliasWarps - 1) / kAliasWarps, (u32)(device_sm_count() * per_sm * 4));
+  alias_build_batch_kernel<<<blocks, 32 * kAliasWarps, need, s>>>(ar, bp, most, Kmax, w0, w1);
 }
 
 void launch_bump(u32* t, cudaStream_t s) { bump_kernel<<<1, 1, 0, s>>>(t); }
@@ -739,20 +974,21 @@ size_t alias_build_scratch_bytes(u32 K) {
 
 void launch_alias_build(const ModelDev& m, cudaStream_t s, void* scratch, size_t scratch_bytes) {
   if (m.Sinv) topic_recip_kernel<<<(m.K + 255) / 256, 256, 0, s>>>(m.S, m.Sinv, m.K);
-  const u32 nt = alias_threads(m.K);
-  const u32 items = std::min(m.K, kAliasSmemItems);
-  const size_t smem = alias_scratch_item_bytes(items);
+  const u32 items = std::min(m.K, kAliasSmemItems), most = alias_items(m.K);
+  const size_t smem = std::max(kAliasWarps * alias_warp_bytes(most), alias_scratch_item_bytes(items));
+  if (smem > 47 * 1024) cudaFuncSetAttribute(alias_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, alias_build_kernel, nt, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, alias_build_kernel, 32 * kAliasWarps, smem);
   if (per_sm < 1) per_sm = 1;
-  u32 blocks = std::min<u32>(m.V, (u32)(device_sm_count() * per_sm * (m.K <= kAliasSmemItems ? 4 : 1)));
+  u32 blocks = std::min<u32>((m.V + kAliasWarps - 1) / kAliasWarps,
+                             (u32)(device_sm_count() * per_sm * (m.K <= kAliasSmemItems ? 4 : 1)));
   if (m.K > kAliasSmemItems) {
     const size_t slice = alias_slice_bytes(m.K);
     blocks = std::min<u32>(blocks, (u32)(scratch_bytes / slice));
     if (!blocks) return;  // no scratch: the caller allocates alias_build_scratch_bytes(K)
-    alias_build_kernel<<<blocks, nt, smem, s>>>(m, (unsigned char*)scratch, slice, items);
+    alias_build_kernel<<<blocks, 32 * kAliasWarps, smem, s>>>(m, (unsigned char*)scratch, slice, most, items);
   } else {
-    alias_build_kernel<<<blocks, nt, smem, s>>>(m, nullptr, 0, items);
+    alias_build_kernel<<<blocks, 32 * kAliasWarps, smem, s>>>(m, nullptr, 0, most, items);
   }
 }
 
