@@ -263,6 +263,7 @@ void free_model() {
   dfree(g.dev.al);
   dfree(g.dev.csr);
   dfree(g.dev.lists);
+  dfree(g.dev.bits);
   dfree(g.dev.A);
   dfree(g.dev.S);
   dfree(g.dev.Sinv);
@@ -330,6 +331,7 @@ int init_impl(const Args* args, Buffer* buffers, u32 n_buffers, const GpuldaExAr
   if ((rc = dalloc(&g.dev.n, cells)) || (rc = dalloc(&g.dev.q, cells)) || (rc = dalloc(&g.dev.al, cells)) ||
       (rc = dalloc(&g.dev.csr, cells)) ||
       (g.K <= kMapMinK && (rc = dalloc(&g.dev.lists, (size_t)g.V * list_stride(g.K)))) ||
+      (bits_pay(g.K, g.V) && (rc = dalloc(&g.dev.bits, (size_t)g.V * bits_stride(g.K)))) ||
       (rc = dalloc(&g.dev.A, g.V)) || (rc = dalloc(&g.dev.S, g.K + 2)) || (rc = dalloc(&g.dev.Sinv, g.K)) ||
       (rc = dalloc(&g.dev.nnz, g.V)) ||
       (rc = dalloc(&g.C, g.V)) || (rc = dalloc(&g.cdf, (size_t)kPoisN * kPoisW)) ||

@@ -341,13 +341,27 @@ constexpr u32 kAliasWarps = 4;  // a block's, a word each
 inline u32 alias_items(u32 K) { return std::min(K, K <= kMapMinK ? 256u : 512u); }
 __host__ __device__ constexpr size_t alias_warp_bytes(u32 most) { return ((size_t)most * 18 + 15) & ~(size_t)15; }
 
+// Sets the bits of a list's topics; the first of the entries of a 32-bit word
+// writes it.
+__device__ __forceinline__ void list_bits(const u64* ent, u32 n, u32* bits, u32 first, u32 step) {
+  for (u32 i = first; i < n; i += step) {
+    const u32 at = ((u32)ent[i] & 0xffffu) >> 5;
+    if (i && ((u32)ent[i - 1] & 0xffffu) >> 5 == at) continue;
+    u32 b = 0;
+    for (u32 j = i; j < n && ((u32)ent[j] & 0xffffu) >> 5 == at; ++j) b |= 1u << (ent[j] & 31);
+    bits[at] = b;
+  }
+}
+
 __device__ __forceinline__ void alias_word(u32 K, u32* __restrict__ qrow, const u64* __restrict__ S,
-                                           const u64* __restrict__ Sinv, u64* alrow, u64* csrrow, u64* eighths, u64* A_out,
+                                           const u64* __restrict__ Sinv, u64* alrow, u64* csrrow, u64* eighths, u32* bits, u64* A_out,
                                            u64* s_shares,
                                            u32* nnz_out, u64* s_vals, uint16_t* s_idx, u32 smem_items, u64* g_vals,
                                            uint16_t* g_idx, u64* sh) {
   u64 part = 0, nz = 0;
   u32 xsum = 0;
+  if (bits)
+    for (u32 i = threadIdx.x; i < bits_stride(K); i += blockDim.x) bits[i] = 0;
   const u32 tile = blockDim.x * kPerThread;
   for (u32 t0 = 0; t0 < K; t0 += tile) {
     const u32 k0 = t0 + threadIdx.x * kPerThread;
@@ -378,6 +392,7 @@ __device__ __forceinline__ void alias_word(u32 K, u32* __restrict__ qrow, const 
   }
   const u64 A = block_sum_u64(part, sh);  // (also orders the list writes before the build)
   const u32 n = (u32)nz;
+  if (bits) list_bits(csrrow, n, bits, threadIdx.x, blockDim.x);
   if (s_shares) {  // the word's tokens (its draws' sum), by its list's length
     xsum = __reduce_add_sync(kFullMask, xsum);
     if ((threadIdx.x & 31) == 0) {
@@ -415,7 +430,7 @@ __device__ __forceinline__ void alias_word(u32 K, u32* __restrict__ qrow, const 
 // to 1000 topics) 337 -> 146.
 __device__ __forceinline__ bool alias_word_warp(u32 K, u32* qrow, const u64* __restrict__ S,
                                                 const u64* __restrict__ Sinv, u64* alrow, u64* csrrow, u64* eighths,
-                                                u64* A_out, u32* nnz_out, u64& x_all, u64& x_long, u64* ent, u64* vals,
+                                                u32* bits, u64* A_out, u32* nnz_out, u64& x_all, u64& x_long, u64* ent, u64* vals,
                                                 uint16_t* idx, u32 most) {
   constexpr u32 kInFlight = 4;  // loads of 512 bytes; 8 take registers and a resident block (mid 212 -> 239 us)
   const u32 lane = threadIdx.x & 31, before = (1u << lane) - 1;
@@ -470,6 +485,11 @@ __device__ __forceinline__ bool alias_word_warp(u32 K, u32* qrow, const u64* __r
     const u64 e = ent[i];
     qrow[(u32)e] = (u32)(e >> 32);
     csrrow[i] = e;
+  }
+  if (bits) {
+    for (u32 i = lane; i < bits_stride(K) / 4; i += 32) reinterpret_cast<uint4*>(bits)[i] = make_uint4(0, 0, 0, 0);
+    __syncwarp();
+    list_bits(ent, n, bits, lane, 32);
   }
   if (eighths && n) {  // as alias_word
     const u32 c = list_pairs(n), recip = list_recip(c);
@@ -582,7 +602,8 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_kernel(ModelD
   for (u64 w = (u64)blockIdx.x * nw + warp; w < m.V; w += step) {
     const size_t row = (size_t)w * K;
     if (alias_word_warp(K, m.q + row, m.S, m.Sinv, m.al + row, m.csr + row,
-                        m.lists ? m.lists + (size_t)w * list_stride(K) : nullptr, m.A + w, m.nnz + w, x_all, x_long,
+                        m.lists ? m.lists + (size_t)w * list_stride(K) : nullptr,
+                        m.bits ? m.bits + (size_t)w * bits_stride(K) : nullptr, m.A + w, m.nnz + w, x_all, x_long,
                         sm.ent, sm.vals, sm.idx, most))
       continue;
     if ((threadIdx.x & 31) == 0) {
@@ -608,7 +629,8 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_kernel(ModelD
         if (m.nnz[w] != kNnzWide) continue;
         const size_t row = (size_t)w * K;
         alias_word(K, m.q + row, m.S, m.Sinv, m.al + row, m.csr + row,
-                   m.lists ? m.lists + (size_t)w * list_stride(K) : nullptr, m.A + w, m.shares ? sh_shares : nullptr,
+                   m.lists ? m.lists + (size_t)w * list_stride(K) : nullptr,
+                   m.bits ? m.bits + (size_t)w * bits_stride(K) : nullptr, m.A + w, m.shares ? sh_shares : nullptr,
                    m.nnz + w, sm.all_vals, sm.all_idx, smem_items, g_vals, g_idx, sh);
       }
     __syncthreads();
@@ -635,7 +657,7 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_batch_kernel(
     const u32 pb = bp.wpid[w], K = bp.K[pb];
     const size_t row = bp.row_off[w];
     if (alias_word_warp(K, ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row,
-                        ar.lists + bp.list_off[w], ar.A + w, ar.nnz + w, x_all, x_long, sm.ent, sm.vals, sm.idx, most))
+                        ar.lists + bp.list_off[w], nullptr, ar.A + w, ar.nnz + w, x_all, x_long, sm.ent, sm.vals, sm.idx, most))
       continue;
     if ((threadIdx.x & 31) == 0) {
       ar.nnz[w] = kNnzWide;
@@ -656,7 +678,7 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_batch_kernel(
         if (ar.nnz[w] != kNnzWide) continue;
         const u32 pb = bp.wpid[w], K = bp.K[pb];
         const size_t row = bp.row_off[w];
-        alias_word(K, ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row, ar.lists + bp.list_off[w],
+        alias_word(K, ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row, ar.lists + bp.list_off[w], nullptr,
                    ar.A + w, sh_shares, ar.nnz + w, sm.all_vals, sm.all_idx, Kmax, nullptr, nullptr, sh);
       }
     __syncthreads();

@@ -39,6 +39,15 @@ __host__ __device__ inline u32 list_pairs(u32 n) {
 // Entries from one word's list to the next.
 __host__ __device__ inline u32 list_stride(u32 K) { return 16 * list_pairs(K); }
 
+// Words from one word's bits to the next: whole sectors.
+__host__ __device__ inline u32 bits_stride(u32 K) { return (K + 255) / 256 * 8; }
+
+// Whether a large-K model keeps them: where q takes several times the 126 MB of
+// L2, a gather of q mostly goes to HBM.  At 233 MB (K=7275) the bits made the
+// sweep 2.23 -> 2.44 ms and the alias build 0.36 -> 0.46; at 1.2 GB 13.7 -> 9.6
+// and 0.73 -> 0.78.
+inline bool bits_pay(u32 K, u32 V) { return K > kMapMinK && (u64)K * V * 4 > (512ull << 20); }
+
 // Where entry i of an eighths-stored list with c = list_pairs(n) stands; recip =
 // ceil(2^20 / c) divides the at most 8 c <= 1056 pairs' numbers exactly.
 __host__ __device__ inline u32 list_recip(u32 c) { return ((1u << 20) + c - 1) / c; }
@@ -79,6 +88,7 @@ struct ModelDev {
   u64* al;     // V*K alias entries
   u64* csr;    // V*K per-word lists of (q << 32 | k) for q > 0, ascending k, nnz[w] used
   u64* lists;  // the same lists by eighths, list_stride(K) entries apart (K <= kMapMinK, else null)
+  u32* bits;   // a bit for each of a word's topics with q > 0, bits_stride(K) words a row (training, if bits_pay, else null)
   u64* A;      // V   dense mass per word
   u64* S;      // K   per-topic normalisers
   u64* Sinv;   // K   floor((2^64 - 1) / S[k]), written by the alias build's launch (null: divide)

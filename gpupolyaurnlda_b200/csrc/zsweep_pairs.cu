@@ -16,9 +16,12 @@
 // What bounds it: the gathers.  A document's topics lie in different sectors of
 // a word's row (40 KB at K=10000), most of them in HBM: 61 sectors a token at
 // 5.4 TB/s of DRAM traffic (K=10000, V=30000, 3e5 documents of 80 tokens), 225
-// instructions a token.  That sweep takes 13.4 ms; with the list in shared
-// memory, searched and shifted at every draw (430 instructions), it took 25.3
-// ms.  Documents in device memory at K=4096 (2e4 documents of up to 5000
+// instructions a token, 13.7 ms.  But 7% of those entries are not zero.  FEW:
+// where q does not fit L2, a bit for each of a word's topics does (38 MB for 1.2
+// GB there); before a chunk's draws each lane collects its topics' bits for the
+// chunk's words, many loads at a time, and only entries with mass are gathered:
+// 9.6 ms.  (With the list in shared memory, searched and shifted at every draw,
+// 430 instructions, it was 25.3 ms.)  Documents in device memory at K=4096 (2e4 documents of up to 5000
 // tokens, no lengths on the host), whose lists had to be sized for K entries
 // each, 5.8 against 26 ms.
 //
@@ -42,6 +45,8 @@ constexpr u32 kMaxDocLen = 65535u;
 constexpr u32 kStatusListFull = 32;  // a list sized for its document was too small (cannot happen)
 constexpr u32 kNone = 0xffffu;     // no topic (topics are below 32768)
 constexpr u32 kSparseBit = 0x8000u;
+constexpr u32 kBitsAhead = 4;  // tokens whose words' bits are loaded at a time (1: 11.3 ms, 2: 10.3, 8: 10.0)
+constexpr u32 kBitsMost = 8;   // entries a lane with room for the bits in registers
 
 // Shared memory per warp: the list (topic << 16 | count, `cap` entries), the
 // positions of a merge's new entries, the chunk's staged tokens (32 bytes each,
@@ -198,10 +203,13 @@ static __device__ __noinline__ u32 list_merge(const WarpMem wm, u32 n, u32 topic
 // lane.  Drawn topics go to stage[2 j].x (kSparseBit beside them), the distinct
 // topics without the token to stage[2 j].y.  The list in shared
 // memory is left with the live entries; their number is returned.
-template <u32 R>
-__device__ __forceinline__ u32 list_chunk(const WarpMem& wm, u32 n, u32 nt, u32 nz, u32 lane) {
+template <u32 R, bool FEW>
+__device__ __forceinline__ u32 list_chunk(const WarpMem& wm, const u32* __restrict__ bits, u32 stride, u32 n, u32 nt,
+                                          u32 nz, u32 lane) {
   const u32 per = (n + 31) >> 5;
+  constexpr bool BITS = FEW && R <= kBitsMost;
   u32 tp[R], ct[R], qn[R];
+  u32 has[BITS ? R : 1];  // bit j: the topic has mass in token j's word
 #pragma unroll
   for (u32 s = 0; s < R; ++s) {
     const u32 e = lane * per + s;
@@ -209,6 +217,16 @@ __device__ __forceinline__ u32 list_chunk(const WarpMem& wm, u32 n, u32 nt, u32 
     tp[s] = v >> 16;
     ct[s] = v & 0xffffu;
     qn[s] = 0;
+    if constexpr (BITS) has[s] = 0;
+  }
+  if constexpr (BITS) {
+#pragma unroll(kBitsAhead)
+    for (u32 j = 0; j < nt; ++j) {
+      const u32* row = bits + (size_t)wm.stage[2 * j].w * stride;
+#pragma unroll
+      for (u32 s = 0; s < R; ++s)
+        if (tp[s] != kNone) has[s] |= ((__ldg(row + (tp[s] >> 5)) >> (tp[s] & 31)) & 1u) << j;
+    }
   }
   // moves a token: k in (kNone: none), z out
   auto move = [&](u32 k, u32 z) {
@@ -222,13 +240,19 @@ __device__ __forceinline__ u32 list_chunk(const WarpMem& wm, u32 n, u32 nt, u32 
     }
     nz += (u32)__reduce_add_sync(kFullMask, live);
   };
-  // Staged token: topic | dense topic << 16, r0, r1, -; row of q, alpha A.
+  // Staged token: topic | dense topic << 16, r0, r1, word; row of q, alpha A.
   uint4 a = wm.stage[0], b = wm.stage[1];
   auto fetch = [&](u32 pending) {
     const u32* row = (const u32*)(((u64)b.y << 32) | b.x);
 #pragma unroll
-    for (u32 s = 0; s < R; ++s)
-      if (ct[s] || (tp[s] == pending && pending != kNone)) qn[s] = __ldg(row + tp[s]);
+    for (u32 s = 0; s < R; ++s) {
+      if constexpr (BITS) {
+        qn[s] = (has[s] & 1u) && (ct[s] || tp[s] == pending) ? __ldg(row + tp[s]) : 0u;
+        has[s] >>= 1;
+      } else if (ct[s] || (tp[s] == pending && pending != kNone)) {
+        qn[s] = __ldg(row + tp[s]);
+      }
+    }
   };
   // (the entries of no topic have a zero count; nothing is added to or taken
   // from them: no token has that topic)
@@ -395,7 +419,7 @@ static __device__ __noinline__ u32 long_chunk(const WarpMem wm, u32 n, u32 nt, u
 
 // LONG: the documents of z.rest, from the token each stands at, lists in shared
 // memory.
-template <bool LL, bool LONG>
+template <bool LL, bool LONG, bool FEW>
 __global__ void __launch_bounds__(256, LONG ? 3 : 2) z_sweep_pairs_kernel(ListArgs a) {
   extern __shared__ __align__(16) unsigned char zsm[];
   __shared__ unsigned long long blk_stats[4];  // tokens, documents, sparse work, sparse draws
@@ -404,7 +428,7 @@ __global__ void __launch_bounds__(256, LONG ? 3 : 2) z_sweep_pairs_kernel(ListAr
   const ModelDev& m = a.m;
   const ZLaunch& p = a.z;
   const u32 lane = threadIdx.x & 31;
-  const u32 K = m.K, V = m.V;
+  const u32 K = m.K, V = m.V, stride = bits_stride(m.K);
   const WarpMem wm = warp_mem_at(zsm + (threadIdx.x >> 5) * warp_mem_bytes(a.cap, LONG), a.cap);
   const u32 n_items = LONG ? *p.n_rest : p.n_docs;
   double ll_acc = 0.0, ll_skip = 0.0;
@@ -483,7 +507,7 @@ __global__ void __launch_bounds__(256, LONG ? 3 : 2) z_sweep_pairs_kernel(ListAr
       {
         const u64 aA = (u64)__double_as_longlong(__dmul_rn((double)m.alpha, exact_double(A1)));
         const u64 row = (u64)(m.q + my_row);
-        wm.stage[2 * lane] = make_uint4(z1 | (kd << 16), r.x, r.y, 0);
+        wm.stage[2 * lane] = make_uint4(z1 | (kd << 16), r.x, r.y, FEW ? w1 : 0u);
         wm.stage[2 * lane + 1] = make_uint4((u32)row, (u32)(row >> 32), (u32)aA, (u32)(aA >> 32));
       }
       __syncwarp();
@@ -502,17 +526,17 @@ __global__ void __launch_bounds__(256, LONG ? 3 : 2) z_sweep_pairs_kernel(ListAr
       if (LONG)
         n = long_chunk(wm, n, nt, nz, lane);
       else if (per <= 2)
-        n = list_chunk<2>(wm, n, nt, nz, lane);
+        n = list_chunk<2, FEW>(wm, m.bits, stride, n, nt, nz, lane);
       else if (per == 3)
-        n = list_chunk<3>(wm, n, nt, nz, lane);
+        n = list_chunk<3, FEW>(wm, m.bits, stride, n, nt, nz, lane);
       else if (per == 4)
-        n = list_chunk<4>(wm, n, nt, nz, lane);
+        n = list_chunk<4, FEW>(wm, m.bits, stride, n, nt, nz, lane);
       else if (per <= 6)
-        n = list_chunk<6>(wm, n, nt, nz, lane);
+        n = list_chunk<6, FEW>(wm, m.bits, stride, n, nt, nz, lane);
       else if (per <= 8)
-        n = list_chunk<8>(wm, n, nt, nz, lane);
+        n = list_chunk<8, FEW>(wm, m.bits, stride, n, nt, nz, lane);
       else
-        n = list_chunk<16>(wm, n, nt, nz, lane);
+        n = list_chunk<16, FEW>(wm, m.bits, stride, n, nt, nz, lane);
       nz = n;
       const u32 res = wm.stage[2 * lane].x, my_nz = wm.stage[2 * lane].y;
       const u32 new_z = res & 0x7fffu;
@@ -580,7 +604,7 @@ __global__ void __launch_bounds__(256, LONG ? 3 : 2) z_sweep_pairs_kernel(ListAr
 
 namespace {
 
-template <bool LONG>
+template <bool LONG, bool FEW>
 void launch_lists(const ModelDev& m, const ZLaunch& z, cudaStream_t s, u32 cap) {
   if (!z.n_docs) return;
   ListArgs a;
@@ -589,7 +613,8 @@ void launch_lists(const ModelDev& m, const ZLaunch& z, cudaStream_t s, u32 cap) 
   a.cap = cap;
   a.lg_a = std::lgamma((double)m.alpha);
   a.lg_Ka = std::lgamma((double)m.K * (double)m.alpha);
-  auto kern = (z.flags & kZFlagLoglik) && z.ll ? z_sweep_pairs_kernel<true, LONG> : z_sweep_pairs_kernel<false, LONG>;
+  auto kern = (z.flags & kZFlagLoglik) && z.ll ? z_sweep_pairs_kernel<true, LONG, FEW>
+                                                   : z_sweep_pairs_kernel<false, LONG, FEW>;
   constexpr size_t kBudget = 200 * 1024;
   u32 warps = 8;
   while (warps > 1 && warps * warp_mem_bytes(cap, LONG) > kBudget) --warps;
@@ -605,11 +630,17 @@ void launch_lists(const ModelDev& m, const ZLaunch& z, cudaStream_t s, u32 cap) 
 }  // namespace
 
 void launch_z_sweep_pairs(const ModelDev& m, const ZLaunch& z, cudaStream_t s) {
-  launch_lists<false>(m, z, s, kListMost);
+  // The words' bits where q is in HBM (m.bits) and the sweep is bound by it: 8
+  // documents for each of the GPU's warps.  With 7,900 documents of 110 tokens
+  // (K=3683) their loads only made the documents' chains longer: 1.78 -> 1.9 ms.
+  if (m.bits && z.n_docs >= 8u * 16u * (u32)device_sm_count())
+    launch_lists<false, true>(m, z, s, kListMost);
+  else
+    launch_lists<false, false>(m, z, s, kListMost);
 }
 
 void launch_z_sweep_rest(const ModelDev& m, const ZLaunch& z, cudaStream_t s, u32 lmax) {
-  launch_lists<true>(m, z, s, std::min(std::max(lmax, 1u), m.K) + 32);
+  launch_lists<true, false>(m, z, s, std::min(std::max(lmax, 1u), m.K) + 32);
 }
 
 }  // namespace gpulda
