@@ -172,13 +172,14 @@ def roofline_profile(workload: str, c) -> dict:
     scaled to this launch only for that workload."""
     if c.K > 2048:
         return {"kernel": "z_sweep_pairs_kernel", "traffic": None,
-                "traffic_note": "the committed ncu capture of this kernel is a V=14,000 case "
-                                "(profiles/z_sweep_pairs_kernel_K10000_small_case.md: about 1.2 kB of DRAM traffic per "
-                                "token at a 49 % L2 hit rate); its hit rate does not carry over to V=140,000, so no "
-                                "traffic is scaled to this launch"}
+                "traffic_note": "the committed ncu capture is a V=14,000 case of the kernel before its lists moved to "
+                                "registers (profiles/z_sweep_pairs_kernel_K10000_small_case.md), so no traffic is "
+                                "scaled to this launch"}
     out = {"kernel": "z_sweep_kernel",
            "binding_resource": "L1 data pipe (74 % of wavefront slots in the ncu profile), issue (66 %) and "
-                               "gather latency; DRAM at 2.6 %: 93 % of the gathers hit L2, half of them L1"}
+                               "gather latency; DRAM at 2.6 %: 93 % of the gathers hit L2, half of them L1",
+           "trained": "once most words' lists are short z_sweep_words_kernel runs instead: latency of a token's "
+                      "dependent steps at 16 warps an SM, L1 data pipe 62 %"}
     tpt = measured_traffic_per_token()
     if workload == "mid" and tpt:
         out.update(traffic=tpt * c.n_tokens, traffic_note="ncu dram bytes per token of a 3.4e7-token slice, scaled to N")
@@ -509,7 +510,7 @@ def large_k_measure(args, local: int, hbm: float, workload: str = "large_k10000"
                        f"3..{2 + args.large_steps} of a chain from random topics",
            "tokens_per_s": c.n_tokens / (ms / 1e3), "ms_per_iteration": ms,
            "z_sweep_ms": float(np.mean(z_ms)), "phi_step_ms": float(np.mean(phi_ms)),
-           "z_kernel": "z_sweep_pairs_kernel (sorted (topic, count) lists)",
+           "z_kernel": "z_sweep_pairs_kernel (sorted (topic, count) lists in registers)",
            "roofline_frac": z_gbs / hbm, "z_achieved_gbs": z_gbs,
            "sparse_work_per_token": float(np.mean(S_work)) / c.n_tokens, "generate_s": t_gen, "clocks": clk}
     del c
