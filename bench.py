@@ -179,7 +179,7 @@ def roofline_profile(workload: str, c) -> dict:
            "binding_resource": "L1 data pipe (74 % of wavefront slots in the ncu profile), issue (66 %) and "
                                "gather latency; DRAM at 2.6 %: 93 % of the gathers hit L2, half of them L1",
            "trained": "once most words' lists are short z_sweep_words_kernel runs instead: latency of a token's "
-                      "dependent steps at 16 warps an SM, L1 data pipe 62 %"}
+                      "dependent steps at 16 warps an SM, L1 data pipe 72 %"}
     tpt = measured_traffic_per_token()
     if workload == "mid" and tpt:
         out.update(traffic=tpt * c.n_tokens, traffic_note="ncu dram bytes per token of a 3.4e7-token slice, scaled to N")

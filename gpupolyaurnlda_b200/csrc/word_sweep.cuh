@@ -21,7 +21,7 @@
 // instructions a token with four documents to a warp against 240 with one, and
 // 313 with the walks of doc_counts.cuh: W = 8 for throughput, W = 32 for the
 // fewest steps between a document's tokens.  Bound by the latency of those steps
-// at 16 warps an SM and by the L1 data pipe (62 %, the random count gathers).
+// at 16 warps an SM and by the L1 data pipe (72 %, the random count gathers).
 #pragma once
 
 #include "common.cuh"
