@@ -20,7 +20,8 @@
 // where q does not fit L2, a bit for each of a word's topics does (38 MB for 1.2
 // GB there); before a chunk's draws each lane collects its topics' bits for the
 // chunk's words, many loads at a time, and only entries with mass are gathered:
-// 9.6 ms.  (With the list in shared memory, searched and shifted at every draw,
+// 9.5 ms, 321 instead of 1,083 bytes of DRAM traffic a token, bound by issue (60
+// %) and a token's dependent steps.  (With the list in shared memory, searched and shifted at every draw,
 // 430 instructions, it was 25.3 ms.)  Documents in device memory at K=4096 (2e4 documents of up to 5000
 // tokens, no lengths on the host), whose lists had to be sized for K entries
 // each, 5.8 against 26 ms.
