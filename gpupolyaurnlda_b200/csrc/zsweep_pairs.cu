@@ -168,8 +168,9 @@ static __device__ __noinline__ u32 list_merge(const WarpMem wm, u32 n, u32 topic
         hi = mid;
     }
     fresh = pos == n || list[pos] >> 16 != c;
-    if (!fresh) list[pos] += count;
   }
+  __syncwarp();  // every lane has searched the list
+  if (head && !fresh) list[pos] += count;
   __syncwarp();
   const u32 news = __ballot_sync(kFullMask, fresh);
   const u32 nn = __popc(news);
@@ -364,6 +365,7 @@ static __device__ __noinline__ u32 long_chunk(const WarpMem wm, u32 n, u32 nt, u
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   fetch(0, n);
+  __syncwarp();  // every lane has read the list before the move writes it
   move(false, 0, true, wm.stage[0].x & 0xffffu);
   for (u32 j = 0; j < nt; ++j) {
     const uint4 a = wm.stage[2 * j], b = wm.stage[2 * j + 1];
