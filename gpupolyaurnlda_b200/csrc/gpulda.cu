@@ -1069,6 +1069,33 @@ static __device__ __align__(256) u32 g_noalloc_scratch[kNoAllocWords];
 static_assert(kNoAllocMaxDocs <= kPlanMostDocs, "the order covers every call");
 constexpr int kNoAllocMaxDevices = 64;
 u32* g_noalloc_addr[kNoAllocMaxDevices] = {};
+
+// The launches of an allocation-free sweep on `s`; scratch from d_idx and work on.
+int noalloc_launches(cudaStream_t s, u32* z, const u32* w, const u32* d_len, u32 n_docs, u64 n_tokens, u32* d_idx,
+                     u32* work) {
+  u64* q = (u64*)(work + kNoAllocTail);
+  u32* order = (u32*)(q + kNoAllocMaxDocs);
+  // The lengths are on the device only, so the launches take any document
+  // length.  More documents than the GPU's warps (16 an SM) are swept longest
+  // first, which the device finds out: 60,000 of 340 tokens' mean from a random
+  // start 17.5 -> 13.2 ms an iteration.  Fewer start at once, a warp each,
+  // in any order, and the three launches (9 us) would be lost on them.
+  ZLaunch zl = z_args(z, w, d_len, d_idx, nullptr, nullptr, n_docs, n_tokens, g.tok_offset, nullptr);
+  u32 n_long = n_docs;
+  if (n_docs > 16u * (u32)device_sm_count()) {
+    const DocPlan plan = doc_plan_at(order + kNoAllocMaxDocs);
+    CK(launch_doc_plan(d_len, d_idx, order, n_docs, long_document(n_tokens), plan, s));
+    zl.order = order;
+    if (g.K <= kMapMinK) zl.n_long_dev = plan.n_long;
+    n_long = 0;
+    g.launches += 3;
+  } else {
+    launch_doc_offsets(d_len, d_idx, n_docs, s);
+    CK(cudaGetLastError());
+    g.launches += 1;
+  }
+  return z_launch(s, zl, SweepAux{work, q, 65535u, n_long});
+}
 }  // namespace
 
 extern "C" int gpulda_sample_z_device_noalloc(uint32_t* z, const uint32_t* w, const uint32_t* d_len,
@@ -1096,30 +1123,12 @@ extern "C" int gpulda_sample_z_device_noalloc(uint32_t* z, const uint32_t* w, co
   cudaStream_t s = stream ? (cudaStream_t)stream : main_stream();
   // the previous call's use of the shared scratch ends before this one's begins
   if (int rc = after_noalloc(s)) return rc;
-  u64* q = (u64*)(work + kNoAllocTail);
-  u32* order = (u32*)(q + kNoAllocMaxDocs);
-  // The lengths are on the device only, so the launches take any document
-  // length.  More documents than the GPU's warps (16 an SM) are swept longest
-  // first, which the device finds out: 60,000 of 340 tokens' mean from a random
-  // start 17.5 -> 13.2 ms an iteration.  Fewer start at once, a warp each,
-  // in any order, and the three launches (9 us) would be lost on them.
-  ZLaunch zl = z_args(z, w, d_len, d_idx, nullptr, nullptr, n_docs, n_tokens, g.tok_offset, nullptr);
-  u32 n_long = n_docs;
-  if (n_docs > 16u * (u32)device_sm_count()) {
-    const DocPlan plan = doc_plan_at(order + kNoAllocMaxDocs);
-    CK(launch_doc_plan(d_len, d_idx, order, n_docs, long_document(n_tokens), plan, s));
-    zl.order = order;
-    if (g.K <= kMapMinK) zl.n_long_dev = plan.n_long;
-    n_long = 0;
-    g.launches += 3;
-  } else {
-    launch_doc_offsets(d_len, d_idx, n_docs, s);
-    CK(cudaGetLastError());
-    g.launches += 1;
-  }
-  if (int rc = z_launch(s, zl, SweepAux{work, q, 65535u, n_long})) return rc;
+  const int rc = noalloc_launches(s, z, w, d_len, n_docs, n_tokens, d_idx, work);
+  // What was queued uses the shared scratch, the counts and the statistics, so
+  // what comes next waits for it even where a later launch was refused.
   CK(cudaEventRecord(g.noalloc_done, s));
   g.noalloc_pending = true;
+  if (rc) return rc;
   g.tok_offset += n_tokens;
   g.swept = true;
   return GPULDA_OK;
