@@ -35,6 +35,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "../../include/gpulda.h"
 #include "kernels.cuh"
 #include "warp.cuh"
 
@@ -51,26 +52,26 @@ constexpr u32 kBitsMost = 8;   // entries a lane with room for the bits in regis
 
 // Shared memory per warp: the list (topic << 16 | count, `cap` entries), the
 // positions of a merge's new entries, the chunk's staged tokens (32 bytes each,
-// and one behind them), and for lists that stay there the q values of the
-// current token's and the next one's word at the list's topics.
+// and one behind them), and for lists that stay there, if they fit, the q values
+// of the current token's and the next one's word at the list's topics.
 struct WarpMem {
   u32* list;
-  u32* q;  // 2 x cap
+  u32* q;  // 2 x cap, or null
   u32* at;
   uint4* stage;
   u32 cap;
 };
 
-__host__ __device__ inline size_t warp_mem_bytes(u32 cap, bool with_q) {
+__host__ __device__ constexpr size_t warp_mem_bytes(u32 cap, bool with_q) {
   return (((size_t)cap * (with_q ? 12 : 4) + 15) & ~(size_t)15) + 32 * 4 + 66 * 16;
 }
 
-__device__ __forceinline__ WarpMem warp_mem_at(unsigned char* base, u32 cap) {
+__device__ __forceinline__ WarpMem warp_mem_at(unsigned char* base, u32 cap, bool with_q) {
   WarpMem wm;
   wm.stage = (uint4*)base;
   wm.at = (u32*)(wm.stage + 66);
   wm.list = wm.at + 32;
-  wm.q = wm.list + cap;
+  wm.q = with_q ? wm.list + cap : nullptr;
   wm.cap = cap;
   return wm;
 }
@@ -79,6 +80,7 @@ struct ListArgs {
   ModelDev m;
   ZLaunch z;
   u32 cap;       // entries of a list
+  bool with_q;   // lists that stay in shared memory have their q values there
   double lg_Ka;  // lgamma(K * alpha)
   double lg_a;   // lgamma(alpha)
 };
@@ -328,7 +330,8 @@ __device__ __forceinline__ void copy_word_async(u32* to, const u32* from) {
 // list_chunk with the list left in shared memory, of any length.  The gathers of
 // q for the next token are asynchronous copies, so a long list's gathers are all
 // in flight at once (waiting for eight at a time, a token of a list of about
-// 700 entries took 5 us).
+// 700 entries took 5 us).  Where there is no room for them they are loaded, eight
+// at a time, as they are summed.
 static __device__ __noinline__ u32 long_chunk(const WarpMem wm, u32 n, u32 nt, u32 nz, u32 lane) {
   u32* list = wm.list;
   if (lane < nt) {  // the staged topics become positions
@@ -355,6 +358,7 @@ static __device__ __noinline__ u32 long_chunk(const WarpMem wm, u32 n, u32 nt, u
   // Copies token j's q values: entries without a count are left out, but for
   // the one that the draw in flight may fill.
   auto fetch = [&](u32 j, u32 pending) {
+    if (!wm.q) return;
     const uint4 b = wm.stage[2 * j + 1];
     const u32* row = (const u32*)(((u64)b.y << 32) | b.x);
     u32* q = wm.q + (j & 1) * wm.cap;
@@ -370,15 +374,25 @@ static __device__ __noinline__ u32 long_chunk(const WarpMem wm, u32 n, u32 nt, u
   for (u32 j = 0; j < nt; ++j) {
     const uint4 a = wm.stage[2 * j], b = wm.stage[2 * j + 1];
     const double aA = __hiloint2double((int)b.w, (int)b.z);
+    const u32* row = (const u32*)(((u64)b.y << 32) | b.x);
     const u32* q = wm.q + (j & 1) * wm.cap;
+    // entry e's mass, v its topic and count
+    auto mass = [&](u32 e, u32 v) {
+      return v & 0xffffu ? (u64)(v & 0xffffu) * (wm.q ? q[e] : __ldg(row + (v >> 16))) : 0ull;
+    };
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncwarp();
     if (j + 1 < nt) fetch(j + 1, a.x >> 16);
     u64 x = 0;
+    if (wm.q) {
 #pragma unroll 4
-    for (u32 e = e0; e < e1; ++e) {
-      const u32 c = list[e] & 0xffffu;
-      if (c) x += (u64)c * q[e];
+      for (u32 e = e0; e < e1; ++e) {
+        const u32 c = list[e] & 0xffffu;
+        if (c) x += (u64)c * q[e];
+      }
+    } else {
+#pragma unroll 8
+      for (u32 e = e0; e < e1; ++e) x += mass(e, list[e]);
     }
     __syncwarp();
     const u64 incl = scan64(x);
@@ -393,7 +407,7 @@ static __device__ __noinline__ u32 long_chunk(const WarpMem wm, u32 n, u32 nt, u
       const u32 f1 = min(n, f * per + per);
       for (u32 e = f * per; e < f1; e += 32) {
         const u32 v = e + lane < f1 ? list[e + lane] : 0u;
-        const u64 in2 = scan64(v & 0xffffu ? (u64)(v & 0xffffu) * q[e + lane] : 0ull);
+        const u64 in2 = scan64(mass(e + lane, v));
         const u64 all = __shfl_sync(kFullMask, in2, 31);
         if (all > t) {
           pos = e + __popc(__ballot_sync(kFullMask, in2 <= t));
@@ -432,7 +446,8 @@ __global__ void __launch_bounds__(256, LONG ? 3 : 2) z_sweep_pairs_kernel(ListAr
   const ZLaunch& p = a.z;
   const u32 lane = threadIdx.x & 31;
   const u32 K = m.K, V = m.V, stride = bits_stride(m.K);
-  const WarpMem wm = warp_mem_at(zsm + (threadIdx.x >> 5) * warp_mem_bytes(a.cap, LONG), a.cap);
+  const WarpMem wm = warp_mem_at(zsm + (threadIdx.x >> 5) * warp_mem_bytes(a.cap, LONG && a.with_q), a.cap,
+                                 LONG && a.with_q);
   const u32 n_items = LONG ? *p.n_rest : p.n_docs;
   double ll_acc = 0.0, ll_skip = 0.0;
   u32 status = 0;
@@ -619,9 +634,11 @@ void launch_lists(const ModelDev& m, const ZLaunch& z, cudaStream_t s, u32 cap) 
   auto kern = (z.flags & kZFlagLoglik) && z.ll ? z_sweep_pairs_kernel<true, LONG, FEW>
                                                    : z_sweep_pairs_kernel<false, LONG, FEW>;
   constexpr size_t kBudget = 200 * 1024;
+  static_assert(warp_mem_bytes(GPULDA_MAX_K + 32, false) <= kBudget, "a list of every topic fits");
+  a.with_q = LONG && warp_mem_bytes(cap, true) <= kBudget;
   u32 warps = 8;
-  while (warps > 1 && warps * warp_mem_bytes(cap, LONG) > kBudget) --warps;
-  const size_t smem = warps * warp_mem_bytes(cap, LONG);
+  while (warps > 1 && warps * warp_mem_bytes(cap, a.with_q) > kBudget) --warps;
+  const size_t smem = warps * warp_mem_bytes(cap, a.with_q);
   if (smem > 47 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBudget);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem);
