@@ -432,10 +432,9 @@ int phi_step_async(cudaStream_t s) {
   launch_phi_draw(g.dev, (u32)g.t, s);
   CK(cudaGetLastError());
   CK(cudaEventRecord(g.ev[2], s));
-  launch_alias_build(g.dev, s, g.alias_scratch, g.alias_scratch_bytes);
+  g.launches += 1 + launch_alias_build(g.dev, s, g.alias_scratch, g.alias_scratch_bytes);
   CK(cudaGetLastError());
   CK(cudaEventRecord(g.ev[3], s));
-  g.launches += 3;  // Poisson draw, topic reciprocals, alias build
   g.phi_timed = true;
   return GPULDA_OK;
 }

@@ -335,7 +335,8 @@ __device__ __forceinline__ u64 fixed_phi(u32 x, u32 k, const u64* __restrict__ S
 constexpr u32 kPerThread = 8;
 constexpr u32 kAliasWarps = 4;  // a block's, a word each
 // Most topics of a word that a warp takes (18 bytes each set how many warps are
-// resident); a longer word takes the block.  K=1000: 128, 256 and 512 take 218,
+// resident); a longer word takes a block, of a launch of its own where K has room
+// for such words.  K=1000: 128, 256 and 512 take 218,
 // 210 and 243 us at the mid corpus; K=10000, whose words' lists are longer: 1350,
 // 900 and 700 us.
 inline u32 alias_items(u32 K) { return std::min(K, K <= kMapMinK ? 256u : 512u); }
@@ -567,28 +568,75 @@ __device__ __forceinline__ bool alias_word_warp(u32 K, u32* qrow, const u64* __r
   return true;
 }
 
+// The block's alias scratch for one word of up to `items` topics.
+struct AliasScratch {
+  u64* vals;
+  uint16_t* idx;
+};
+__device__ __forceinline__ AliasScratch alias_scratch_at(unsigned char* raw, u32 items) {
+  AliasScratch a;
+  a.vals = (u64*)raw;
+  a.idx = (uint16_t*)(a.vals + items);
+  return a;
+}
+
 // A block's shared memory: its warps' scratch, or all of it for one word.
 struct AliasSmem {
   u64 *ent, *vals;      // this warp's
   uint16_t* idx;
-  u64* all_vals;        // the block's
-  uint16_t* all_idx;
+  AliasScratch all;     // the block's
 };
-__device__ __forceinline__ AliasSmem alias_smem(unsigned char* raw, u32 most, u32 all) {
+__device__ __forceinline__ AliasSmem alias_smem(unsigned char* raw, u32 most) {
   AliasSmem a;
   unsigned char* own = raw + (size_t)(threadIdx.x >> 5) * alias_warp_bytes(most);
   a.ent = (u64*)own;
   a.vals = a.ent + most;
   a.idx = (uint16_t*)(a.vals + most);
-  a.all_vals = (u64*)raw;
-  a.all_idx = (uint16_t*)(a.all_vals + all);
+  a.all = alias_scratch_at(raw, most);
   return a;
 }
 
-constexpr u32 kNnzWide = 0xffffffffu;  // marks a word that its warp left to the block
+constexpr u32 kNnzWide = 0xffffffffu;  // marks a word that its warp left to a block
 
-__global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_kernel(ModelDev m, unsigned char* gscratch, size_t slice,
-                                                                       u32 most, u32 smem_items) {
+// f(w) for the block's words of [w0, w1) that are marked, every gridDim-th, all
+// threads together.
+template <class F>
+__device__ __forceinline__ void for_wide_words(const u32* nnz, u64 w0, u64 w1, F&& f) {
+  __shared__ u32 marked[8];  // by warp
+  const u32 nw = blockDim.x >> 5;
+  for (u64 first = w0 + blockIdx.x; first < w1; first += (u64)gridDim.x * blockDim.x) {
+    const u64 w = first + (u64)threadIdx.x * gridDim.x;
+    const u32 b = __ballot_sync(kFullMask, w < w1 && nnz[w] == kNnzWide);
+    if ((threadIdx.x & 31) == 0) marked[threadIdx.x >> 5] = b;
+    __syncthreads();
+    for (u32 i = 0; i < nw; ++i)
+      for (u32 left = marked[i]; left; left &= left - 1)
+        f(first + (u64)(32 * i + (u32)__ffs((int)left) - 1) * gridDim.x);
+    __syncthreads();
+  }
+}
+
+// Word w of the model by the block; g: its slice of global scratch.
+__device__ __forceinline__ void alias_word_of(const ModelDev& m, u64 w, u64* s_shares, const AliasScratch& all,
+                                              u32 smem_items, unsigned char* g, u64* sh) {
+  const u32 K = m.K;
+  const size_t row = (size_t)w * K;
+  alias_word(K, m.q + row, m.S, m.Sinv, m.al + row, m.csr + row,
+             m.lists ? m.lists + (size_t)w * list_stride(K) : nullptr,
+             m.bits ? m.bits + (size_t)w * bits_stride(K) : nullptr, m.A + w, s_shares, m.nnz + w, all.vals, all.idx,
+             smem_items, (u64*)g, g ? (uint16_t*)((u64*)g + K) : nullptr, sh);
+}
+
+// Word w of a batch.
+__device__ __forceinline__ void alias_word_of(const ModelDev& ar, const BatchPhiDev& bp, u64 w, u64* s_shares,
+                                              const AliasScratch& all, u32 smem_items, u64* sh) {
+  const u32 pb = bp.wpid[w];
+  const size_t row = bp.row_off[w];
+  alias_word(bp.K[pb], ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row, ar.lists + bp.list_off[w],
+             nullptr, ar.A + w, s_shares, ar.nnz + w, all.vals, all.idx, smem_items, nullptr, nullptr, sh);
+}
+
+__global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_kernel(ModelDev m, u32 most) {
   extern __shared__ __align__(16) unsigned char s_raw[];
   __shared__ u64 sh[33], sh_shares[2];
   __shared__ u32 wide;
@@ -596,7 +644,7 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_kernel(ModelD
   if (threadIdx.x < 2) sh_shares[threadIdx.x] = 0;
   if (threadIdx.x == 0) wide = 0;
   __syncthreads();
-  const AliasSmem sm = alias_smem(s_raw, most, smem_items);
+  const AliasSmem sm = alias_smem(s_raw, most);
   u64 x_all = 0, x_long = 0;
   const u64 step = (u64)gridDim.x * nw;
   for (u64 w = (u64)blockIdx.x * nw + warp; w < m.V; w += step) {
@@ -621,21 +669,34 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_kernel(ModelD
     }
   }
   __syncthreads();
-  if (wide) {
-    u64* g_vals = gscratch ? (u64*)(gscratch + (size_t)blockIdx.x * slice) : nullptr;
-    uint16_t* g_idx = gscratch ? (uint16_t*)(g_vals + K) : nullptr;
+  if (wide && K <= most) {  // (draws that round to q = 0: no launch of their own)
     for (u64 w0 = (u64)blockIdx.x * nw; w0 < m.V; w0 += step)
-      for (u64 w = w0; w < min((u64)m.V, w0 + nw); ++w) {
-        if (m.nnz[w] != kNnzWide) continue;
-        const size_t row = (size_t)w * K;
-        alias_word(K, m.q + row, m.S, m.Sinv, m.al + row, m.csr + row,
-                   m.lists ? m.lists + (size_t)w * list_stride(K) : nullptr,
-                   m.bits ? m.bits + (size_t)w * bits_stride(K) : nullptr, m.A + w, m.shares ? sh_shares : nullptr,
-                   m.nnz + w, sm.all_vals, sm.all_idx, smem_items, g_vals, g_idx, sh);
-      }
+      for (u64 w = w0; w < min((u64)m.V, w0 + nw); ++w)
+        if (m.nnz[w] == kNnzWide) alias_word_of(m, w, m.shares ? sh_shares : nullptr, sm.all, most, nullptr, sh);
     __syncthreads();
   }
   if (m.shares && threadIdx.x < 2)
+    atomicAdd((unsigned long long*)m.shares + threadIdx.x, (unsigned long long)sh_shares[threadIdx.x]);
+}
+
+// The words that alias_build_kernel's warps left, a block to each.  Words are
+// ranked by frequency, so the wide ones are neighbours: as part of that kernel,
+// four to a block of half the threads, one block's words waited for each other
+// (K=4096, 2,000 words of 320 topics: 404 us, 99 before that kernel; K=12000,
+// 1,000 words of 750: 890 and 171).  Blocks take every gridDim-th word.
+__global__ void __launch_bounds__(256) alias_wide_kernel(ModelDev m, unsigned char* gscratch, size_t slice,
+                                                         u32 smem_items) {
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  __shared__ u64 sh[33], sh_shares[2];
+  if (threadIdx.x < 2) sh_shares[threadIdx.x] = 0;
+  __syncthreads();
+  const AliasScratch all = alias_scratch_at(s_raw, smem_items);
+  unsigned char* g = gscratch ? gscratch + (size_t)blockIdx.x * slice : nullptr;
+  for_wide_words(m.nnz, 0, m.V, [&](u64 w) {
+    alias_word_of(m, w, m.shares ? sh_shares : nullptr, all, smem_items, g, sh);
+  });
+  __syncthreads();
+  if (m.shares && threadIdx.x < 2 && sh_shares[threadIdx.x])
     atomicAdd((unsigned long long*)m.shares + threadIdx.x, (unsigned long long)sh_shares[threadIdx.x]);
 }
 
@@ -650,7 +711,7 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_batch_kernel(
   if (threadIdx.x < 2) sh_shares[threadIdx.x] = 0;
   if (threadIdx.x == 0) wide = 0;
   __syncthreads();
-  const AliasSmem sm = alias_smem(s_raw, most, Kmax);
+  const AliasSmem sm = alias_smem(s_raw, most);
   u64 x_all = 0, x_long = 0;
   const u64 step = (u64)gridDim.x * nw, first = (u64)w0 + (u64)blockIdx.x * nw;
   for (u64 w = first + warp; w < w1; w += step) {
@@ -672,18 +733,26 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_batch_kernel(
     atomicAdd((unsigned long long*)sh_shares + 1, (unsigned long long)x_long);
   }
   __syncthreads();
-  if (wide) {
+  if (wide && Kmax <= most) {  // as alias_build_kernel
     for (u64 wb = first; wb < w1; wb += step)
-      for (u64 w = wb; w < min((u64)w1, wb + nw); ++w) {
-        if (ar.nnz[w] != kNnzWide) continue;
-        const u32 pb = bp.wpid[w], K = bp.K[pb];
-        const size_t row = bp.row_off[w];
-        alias_word(K, ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row, ar.lists + bp.list_off[w], nullptr,
-                   ar.A + w, sh_shares, ar.nnz + w, sm.all_vals, sm.all_idx, Kmax, nullptr, nullptr, sh);
-      }
+      for (u64 w = wb; w < min((u64)w1, wb + nw); ++w)
+        if (ar.nnz[w] == kNnzWide) alias_word_of(ar, bp, w, sh_shares, sm.all, most, sh);
     __syncthreads();
   }
   if (threadIdx.x < 2)
+    atomicAdd((unsigned long long*)ar.shares + threadIdx.x, (unsigned long long)sh_shares[threadIdx.x]);
+}
+
+// alias_wide_kernel for a batch.
+__global__ void __launch_bounds__(256) alias_wide_batch_kernel(ModelDev ar, BatchPhiDev bp, u32 Kmax, u32 w0, u32 w1) {
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  __shared__ u64 sh[33], sh_shares[2];
+  if (threadIdx.x < 2) sh_shares[threadIdx.x] = 0;
+  __syncthreads();
+  const AliasScratch all = alias_scratch_at(s_raw, Kmax);
+  for_wide_words(ar.nnz, w0, w1, [&](u64 w) { alias_word_of(ar, bp, w, sh_shares, all, Kmax, sh); });
+  __syncthreads();
+  if (threadIdx.x < 2 && sh_shares[threadIdx.x])
     atomicAdd((unsigned long long*)ar.shares + threadIdx.x, (unsigned long long)sh_shares[threadIdx.x]);
 }
 
@@ -933,13 +1002,20 @@ void launch_phi_draw_batch(const ModelDev& ar, const BatchPhiDev& bp, u32 n_bloc
 void launch_alias_build_batch(const ModelDev& ar, const BatchPhiDev& bp, u32 Kmax, u32 w0, u32 w1, cudaStream_t s) {
   if (w1 <= w0) return;
   const u32 most = alias_items(Kmax);
-  const size_t need = std::max(kAliasWarps * alias_warp_bytes(most), alias_scratch_item_bytes(Kmax));
-  if (need > 47 * 1024) cudaFuncSetAttribute(alias_build_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);
+  const size_t need = kAliasWarps * alias_warp_bytes(most);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, alias_build_batch_kernel, 32 * kAliasWarps, need);
   if (per_sm < 1) per_sm = 1;
   const u32 blocks = std::min<u32>((w1 - w0 + kAliasWarps - 1) / kAliasWarps, (u32)(device_sm_count() * per_sm * 4));
   alias_build_batch_kernel<<<blocks, 32 * kAliasWarps, need, s>>>(ar, bp, most, Kmax, w0, w1);
+  if (Kmax <= most) return;
+  const size_t smem = alias_scratch_item_bytes(Kmax);
+  const u32 nt = alias_threads(Kmax);
+  per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, alias_wide_batch_kernel, nt, smem);
+  if (per_sm < 1) per_sm = 1;
+  alias_wide_batch_kernel<<<std::min<u32>(w1 - w0, (u32)(device_sm_count() * per_sm)), nt, smem, s>>>(ar, bp, Kmax, w0,
+                                                                                                      w1);
 }
 
 void launch_bump(u32* t, cudaStream_t s) { bump_kernel<<<1, 1, 0, s>>>(t); }
@@ -994,24 +1070,27 @@ size_t alias_build_scratch_bytes(u32 K) {
   return alias_slice_bytes(K) * (size_t)device_sm_count() * kAliasBlocksPerSm;
 }
 
-void launch_alias_build(const ModelDev& m, cudaStream_t s, void* scratch, size_t scratch_bytes) {
+u32 launch_alias_build(const ModelDev& m, cudaStream_t s, void* scratch, size_t scratch_bytes) {
   if (m.Sinv) topic_recip_kernel<<<(m.K + 255) / 256, 256, 0, s>>>(m.S, m.Sinv, m.K);
-  const u32 items = std::min(m.K, kAliasSmemItems), most = alias_items(m.K);
-  const size_t smem = std::max(kAliasWarps * alias_warp_bytes(most), alias_scratch_item_bytes(items));
-  if (smem > 47 * 1024) cudaFuncSetAttribute(alias_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const u32 most = alias_items(m.K), recip = m.Sinv ? 1u : 0u;
+  const size_t need = kAliasWarps * alias_warp_bytes(most);
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, alias_build_kernel, 32 * kAliasWarps, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, alias_build_kernel, 32 * kAliasWarps, need);
   if (per_sm < 1) per_sm = 1;
-  u32 blocks = std::min<u32>((m.V + kAliasWarps - 1) / kAliasWarps,
-                             (u32)(device_sm_count() * per_sm * (m.K <= kAliasSmemItems ? 4 : 1)));
-  if (m.K > kAliasSmemItems) {
-    const size_t slice = alias_slice_bytes(m.K);
-    blocks = std::min<u32>(blocks, (u32)(scratch_bytes / slice));
-    if (!blocks) return;  // no scratch: the caller allocates alias_build_scratch_bytes(K)
-    alias_build_kernel<<<blocks, 32 * kAliasWarps, smem, s>>>(m, (unsigned char*)scratch, slice, most, items);
-  } else {
-    alias_build_kernel<<<blocks, 32 * kAliasWarps, smem, s>>>(m, nullptr, 0, most, items);
-  }
+  const u32 blocks = std::min<u32>((m.V + kAliasWarps - 1) / kAliasWarps,
+                                   (u32)(device_sm_count() * per_sm * (m.K <= kAliasSmemItems ? 4 : 1)));
+  alias_build_kernel<<<blocks, 32 * kAliasWarps, need, s>>>(m, most);
+  if (m.K <= most) return recip + 1;
+  const u32 items = std::min(m.K, kAliasSmemItems), nt = alias_threads(m.K);
+  const size_t smem = alias_scratch_item_bytes(items), slice = m.K > kAliasSmemItems ? alias_slice_bytes(m.K) : 0;
+  per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, alias_wide_kernel, nt, smem);
+  if (per_sm < 1) per_sm = 1;
+  u32 wide = std::min<u32>(m.V, (u32)(device_sm_count() * per_sm));
+  if (slice) wide = std::min<u32>(wide, (u32)(scratch_bytes / slice));
+  if (!wide) return recip + 1;  // no scratch: the caller allocates alias_build_scratch_bytes(K)
+  alias_wide_kernel<<<wide, nt, smem, s>>>(m, slice ? (unsigned char*)scratch : nullptr, slice, items);
+  return recip + 2;
 }
 
 void launch_count_rebuild(u32* n, const u32* w, const u32* z, u64 n_tokens, u32 K, u32 V, u32* status,

@@ -188,7 +188,8 @@ void launch_bump(u32* t, cudaStream_t s);
 // x ~ Poisson(beta + n) into q (raw), n <- 0, S[k] += x.  S must be zeroed first.
 void launch_phi_draw(const ModelDev& m, u32 t, cudaStream_t s);
 // Per word: q from x and S, A, nnz and the alias table.
-void launch_alias_build(const ModelDev& m, cudaStream_t s, void* scratch, size_t scratch_bytes);
+// Returns the number of launches.
+u32 launch_alias_build(const ModelDev& m, cudaStream_t s, void* scratch, size_t scratch_bytes);
 size_t alias_build_scratch_bytes(u32 K);
 // n[w[i]][z[i]] += 1 for every token (warp-aggregated atomics); w and z
 // 16-byte aligned.
