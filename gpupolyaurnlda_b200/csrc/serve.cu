@@ -325,8 +325,13 @@ __device__ __forceinline__ u64 global_timer_ns() {
 
 // Persistent mode: every block is one warp that serves requests until it has
 // been idle for kIdleNs or the stop flag is up.  Every wait is bounded.
+// Resident blocks, by what their registers cost: over long lists (K=1000, lists
+// of 990 entries, 50 iterations) 32 blocks an SM, 64 registers each, take 169,
+// 204 and 283 ms for 100, 3,000 and 20,000 requests, 28 take 150, 179 and 262, 24
+// take 150, 174 and 268.  Over the words' lists (19 entries) 24 take 55, 67 and 141
+// (the walk over the shorter side there 70, 87 and 155).
 template <bool WORDS>
-__global__ void __launch_bounds__(32, WORDS ? 24 : 32) fold_persistent_kernel(FoldCommon a, RingDev q) {
+__global__ void __launch_bounds__(32, WORDS ? 24 : 28) fold_persistent_kernel(FoldCommon a, RingDev q) {
   extern __shared__ __align__(16) unsigned char fsm[];
   const u32 lane = threadIdx.x;
   while (true) {
