@@ -47,23 +47,31 @@ constexpr u32 kMaxDocLen = 65535u;
 constexpr u32 kStatusListFull = 32;  // a list sized for its document was too small (cannot happen)
 constexpr u32 kNone = 0xffffu;     // no topic (topics are below 32768)
 constexpr u32 kSparseBit = 0x8000u;
+constexpr u32 kLongAhead = 4;  // entries of a word's list that a lane reads ahead (2: up to a third slower)
+// Lists in shared memory have their q values there if that leaves a block this
+// many warps (three times the memory): K=9000, 2,000 documents of 1,000 tokens of
+// which the lengths are on the device only, 40 ms with one, 20 with two or three.
+constexpr u32 kStagedWarps = 2;
 constexpr u32 kBitsAhead = 4;  // tokens whose words' bits are loaded at a time (1: 11.3 ms, 2: 10.3, 8: 10.0)
 constexpr u32 kBitsMost = 8;   // entries a lane with room for the bits in registers
 
 // Shared memory per warp: the list (topic << 16 | count, `cap` entries), the
 // positions of a merge's new entries, the chunk's staged tokens (32 bytes each,
-// and one behind them), and for lists that stay there, if they fit, the q values
-// of the current token's and the next one's word at the list's topics.
+// and one behind them), and for lists that stay there an index of the list by
+// topic and, if they fit, the q values of the current token's and the next one's
+// word at the list's topics.
 struct WarpMem {
   u32* list;
-  u32* q;  // 2 x cap, or null
+  uint16_t* index;  // K: a topic's place in the list if it is there, else anything
+  u32* q;           // 2 x cap, or null
   u32* at;
   uint4* stage;
   u32 cap;
 };
 
-__host__ __device__ constexpr size_t warp_mem_bytes(u32 cap, bool with_q) {
-  return (((size_t)cap * (with_q ? 12 : 4) + 15) & ~(size_t)15) + 32 * 4 + 66 * 16;
+// Of a list of `cap` entries; index: topics of its index (0: none).
+__host__ __device__ constexpr size_t warp_mem_bytes(u32 cap, u32 index, bool with_q) {
+  return (((size_t)cap * (with_q ? 12 : 4) + (size_t)index * 2 + 15) & ~(size_t)15) + 32 * 4 + 66 * 16;
 }
 
 __device__ __forceinline__ WarpMem warp_mem_at(unsigned char* base, u32 cap, bool with_q) {
@@ -72,6 +80,7 @@ __device__ __forceinline__ WarpMem warp_mem_at(unsigned char* base, u32 cap, boo
   wm.at = (u32*)(wm.stage + 66);
   wm.list = wm.at + 32;
   wm.q = with_q ? wm.list + cap : nullptr;
+  wm.index = (uint16_t*)(wm.list + (with_q ? 3 : 1) * cap);
   wm.cap = cap;
   return wm;
 }
@@ -309,39 +318,35 @@ __device__ __forceinline__ u32 list_chunk(const WarpMem& wm, const u32* __restri
   return nz;
 }
 
-// Position of topic k in the sorted list (it is there).
-__device__ __forceinline__ u32 position(const u32* list, u32 n, u32 k) {
-  u32 lo = 0, hi = n;
-  while (lo < hi) {
-    const u32 mid = (lo + hi) >> 1;
-    if (list[mid] >> 16 < k)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  return lo;
-}
-
 __device__ __forceinline__ void copy_word_async(u32* to, const u32* from) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((u32)__cvta_generic_to_shared(to)), "l"(from)
                : "memory");
 }
 
-// list_chunk with the list left in shared memory, of any length.  The gathers of
-// q for the next token are asynchronous copies, so a long list's gathers are all
-// in flight at once (waiting for eight at a time, a token of a list of about
-// 700 entries took 5 us).  Where there is no room for them they are loaded, eight
-// at a time, as they are summed.
-static __device__ __noinline__ u32 long_chunk(const WarpMem wm, u32 n, u32 nt, u32 nz, u32 lane) {
+// list_chunk with the list left in shared memory, of any length.  A token's
+// masses come from the shorter of two sides.  The document's: q is gathered at
+// the list's topics, the next token's by asynchronous copies, so that a long
+// list's gathers are all in flight at once; where there is no room for them they
+// are loaded, eight at a time, as they are summed.  The word's: its list of
+// nonzero q is read, the first entries of the next token's ahead, and its topics
+// are looked up in the document's list through an index by topic.  Bound by the
+// steps from one token to the next.  The side by length: twice or four times the
+// word's entries for one of the document's 1.3 times slower (K=9000, 1,000
+// documents of 2,000 tokens from a random start: 101, 133 and 138 ms).  The same
+// documents with the document's side alone 165 ms; one of 13,000 tokens 203 -> 48
+// (3.7 us a token), 41 of 5,000 143 -> 47.  A binary search in the list in place of
+// the index: 300, 102 and 147 ms.
+static __device__ __noinline__ u32 long_chunk(const WarpMem wm, const u32* q0, const u64* csr, u32 n, u32 nt, u32 nz,
+                                              u32 lane) {
   u32* list = wm.list;
+  uint16_t* index = wm.index;
+  for (u32 e = lane; e < n; e += 32) index[list[e] >> 16] = (uint16_t)e;
+  __syncwarp();
   if (lane < nt) {  // the staged topics become positions
     const u32 v = wm.stage[2 * lane].x;
-    const u32 pz = position(list, n, v & 0xffffu), pk = position(list, n, v >> 16);
-    wm.stage[2 * lane].x = pz | (pk << 16);
+    wm.stage[2 * lane].x = index[v & 0xffffu] | ((u32)index[v >> 16] << 16);
   }
   __syncwarp();
-  const u32 per = (n + 31) >> 5;
-  const u32 e0 = min(n, lane * per), e1 = min(n, e0 + per);
   // one token into entry `in` and one out of entry `out` (lanes 0 and 1)
   auto move = [&](bool add, u32 in, bool del, u32 out) {
     const bool act = !(add && del && in == out) && (lane == 0 ? add : lane == 1 && del);
@@ -355,18 +360,41 @@ static __device__ __noinline__ u32 long_chunk(const WarpMem wm, u32 n, u32 nt, u
     nz += (b & 1u) - ((b >> 1) & 1u);
     __syncwarp();
   };
-  // Copies token j's q values: entries without a count are left out, but for
-  // the one that the draw in flight may fill.
-  auto fetch = [&](u32 j, u32 pending) {
-    if (!wm.q) return;
+  auto row_of = [&](u32 j) {
     const uint4 b = wm.stage[2 * j + 1];
-    const u32* row = (const u32*)(((u64)b.y << 32) | b.x);
-    u32* q = wm.q + (j & 1) * wm.cap;
-    for (u32 e = lane; e < n; e += 32) {
-      const u32 v = list[e];
-      if ((v & 0xffffu) || e == pending) copy_word_async(q + e, row + (v >> 16));
+    return (const u32*)(((u64)b.y << 32) | b.x);
+  };
+  auto word_side = [&](u32 nw) { return nw < n; };
+  constexpr u32 U = kLongAhead;
+  u64 ent[U];  // the lane's first entries of a word's list
+  auto read = [&](const u64* crow, u32 e, u32 end) {
+#pragma unroll
+    for (u32 u = 0; u < U; ++u) ent[u] = e + u < end ? __ldg(crow + e + u) : 0ull;
+  };
+  // What token j needs and does not depend on the counts.  Of the list's q values
+  // those of entries without a count are left out, but for the one that the draw
+  // in flight may fill.
+  auto fetch = [&](u32 j, u32 pending) {
+    const u32* row = row_of(j);
+    const u32 nw = wm.stage[2 * j].w;
+    if (word_side(nw)) {
+      const u32 per = (nw + 31) >> 5, e0 = min(nw, lane * per);
+      read(csr + (row - q0), e0, min(nw, e0 + per));
+    } else if (wm.q) {
+      u32* q = wm.q + (j & 1) * wm.cap;
+      for (u32 e = lane; e < n; e += 32) {
+        const u32 v = list[e];
+        if ((v & 0xffffu) || e == pending) copy_word_async(q + e, row + (v >> 16));
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // an entry of a word's list: its topic's place in the document's, and its mass
+  // (a topic that is not there has any place)
+  auto look_up = [&](u64 en, u32* at) {
+    const u32 p = index[(u32)en & 0xffffu], v = p < n ? list[p] : 0u;
+    *at = p;
+    return v >> 16 == ((u32)en & 0xffffu) ? (u64)(v & 0xffffu) * (u32)(en >> 32) : 0ull;
   };
   fetch(0, n);
   __syncwarp();  // every lane has read the list before the move writes it
@@ -374,51 +402,103 @@ static __device__ __noinline__ u32 long_chunk(const WarpMem wm, u32 n, u32 nt, u
   for (u32 j = 0; j < nt; ++j) {
     const uint4 a = wm.stage[2 * j], b = wm.stage[2 * j + 1];
     const double aA = __hiloint2double((int)b.w, (int)b.z);
-    const u32* row = (const u32*)(((u64)b.y << 32) | b.x);
-    const u32* q = wm.q + (j & 1) * wm.cap;
-    // entry e's mass, v its topic and count
-    auto mass = [&](u32 e, u32 v) {
-      return v & 0xffffu ? (u64)(v & 0xffffu) * (wm.q ? q[e] : __ldg(row + (v >> 16))) : 0ull;
-    };
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncwarp();
-    if (j + 1 < nt) fetch(j + 1, a.x >> 16);
-    u64 x = 0;
-    if (wm.q) {
-#pragma unroll 4
-      for (u32 e = e0; e < e1; ++e) {
-        const u32 c = list[e] & 0xffffu;
-        if (c) x += (u64)c * q[e];
+    const u32* row = row_of(j);
+    const bool more = j + 1 < nt;
+    u32 pos = a.x >> 16;
+    bool sp;
+    if (word_side(a.w)) {
+      const u64* crow = csr + (row - q0);
+      const u32 nw = a.w, per = (nw + 31) >> 5, e0 = min(nw, lane * per), e1 = min(nw, e0 + per);
+      u64 P[U];  // sums over the lane's first entries
+      u32 at[U];
+      u64 x = 0;
+#pragma unroll
+      for (u32 u = 0; u < U; ++u) P[u] = x += look_up(ent[u], at + u);
+      for (u32 e = e0 + U; e < e1; e += U) {
+        read(crow, e, e1);
+        u32 other;
+#pragma unroll
+        for (u32 u = 0; u < U; ++u) x += look_up(ent[u], &other);
+      }
+      __syncwarp();
+      if (more) fetch(j + 1, pos);
+      const u64 incl = scan64(x);
+      const u64 B = __shfl_sync(kFullMask, incl, 31);
+      sp = sparse_test(a.y, aA, B);
+      if (sp) {
+        u64 t = scale_u32(a.z, B);
+        const u32 f = __popc(__ballot_sync(kFullMask, incl <= t)) & 31u;
+        t -= __shfl_sync(kFullMask, incl - x, f);
+        if (per <= U) {
+          u32 p = at[U - 1];
+#pragma unroll
+          for (u32 u = U - 1; u-- > 0;)
+            if (P[u] > t) p = at[u];
+          pos = __shfl_sync(kFullMask, p, f);
+        } else {  // the crossing lane's run, 32 entries at a time
+          const u32 f1 = min(nw, f * per + per);
+          for (u32 e = f * per; e < f1; e += 32) {
+            u32 p;
+            const u64 in2 = scan64(look_up(e + lane < f1 ? __ldg(crow + e + lane) : 0ull, &p));
+            const u64 all = __shfl_sync(kFullMask, in2, 31);
+            if (all > t) {
+              pos = __shfl_sync(kFullMask, p, __popc(__ballot_sync(kFullMask, in2 <= t)));
+              break;
+            }
+            t -= all;
+          }
+        }
       }
     } else {
-#pragma unroll 8
-      for (u32 e = e0; e < e1; ++e) x += mass(e, list[e]);
-    }
-    __syncwarp();
-    const u64 incl = scan64(x);
-    const u64 B = __shfl_sync(kFullMask, incl, 31);
-    const bool sp = sparse_test(a.y, aA, B);
-    u32 pos = a.x >> 16;
-    if (sp) {
-      u64 t = scale_u32(a.z, B);
-      const u32 f = __popc(__ballot_sync(kFullMask, incl <= t)) & 31u;
-      t -= __shfl_sync(kFullMask, incl - x, f);
-      // the crossing lane's run, 32 entries at a time
-      const u32 f1 = min(n, f * per + per);
-      for (u32 e = f * per; e < f1; e += 32) {
-        const u32 v = e + lane < f1 ? list[e + lane] : 0u;
-        const u64 in2 = scan64(mass(e + lane, v));
-        const u64 all = __shfl_sync(kFullMask, in2, 31);
-        if (all > t) {
-          pos = e + __popc(__ballot_sync(kFullMask, in2 <= t));
-          break;
+      const u32* q = wm.q + (j & 1) * wm.cap;
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncwarp();
+      if (more) fetch(j + 1, pos);
+      const u32 per = (n + 31) >> 5, e0 = min(n, lane * per), e1 = min(n, e0 + per);
+      u64 x = 0;
+      if (wm.q) {
+#pragma unroll 4
+        for (u32 e = e0; e < e1; ++e) {
+          const u32 c = list[e] & 0xffffu;
+          if (c) x += (u64)c * q[e];
         }
-        t -= all;
+      } else {
+        for (u32 e = e0; e < e1; e += 8) {
+          u32 v[8], y[8];
+#pragma unroll
+          for (u32 u = 0; u < 8; ++u) v[u] = e + u < e1 ? list[e + u] : 0u;
+#pragma unroll
+          for (u32 u = 0; u < 8; ++u) y[u] = v[u] & 0xffffu ? __ldg(row + (v[u] >> 16)) : 0u;
+#pragma unroll
+          for (u32 u = 0; u < 8; ++u) x += (u64)(v[u] & 0xffffu) * y[u];
+        }
+      }
+      __syncwarp();
+      const u64 incl = scan64(x);
+      const u64 B = __shfl_sync(kFullMask, incl, 31);
+      sp = sparse_test(a.y, aA, B);
+      if (sp) {
+        u64 t = scale_u32(a.z, B);
+        const u32 f = __popc(__ballot_sync(kFullMask, incl <= t)) & 31u;
+        t -= __shfl_sync(kFullMask, incl - x, f);
+        // the crossing lane's run, 32 entries at a time
+        const u32 f1 = min(n, f * per + per);
+        for (u32 e = f * per; e < f1; e += 32) {
+          const u32 v = e + lane < f1 ? list[e + lane] : 0u;
+          const u32 y = v & 0xffffu ? (wm.q ? q[e + lane] : __ldg(row + (v >> 16))) : 0u;
+          const u64 in2 = scan64((u64)(v & 0xffffu) * y);
+          const u64 all = __shfl_sync(kFullMask, in2, 31);
+          if (all > t) {
+            pos = e + __popc(__ballot_sync(kFullMask, in2 <= t));
+            break;
+          }
+          t -= all;
+        }
       }
     }
-    const bool more = j + 1 < nt;
     if (lane == 0) wm.stage[2 * j].x = (list[pos] >> 16) | (sp ? kSparseBit : 0u);
     if (lane == 0) wm.stage[2 * j].y = nz;
+    __syncwarp();  // every lane has read the list
     move(true, pos, more, more ? wm.stage[2 * (j + 1)].x & 0xffffu : 0u);
   }
   // the live entries, in order
@@ -437,7 +517,7 @@ static __device__ __noinline__ u32 long_chunk(const WarpMem wm, u32 n, u32 nt, u
 // LONG: the documents of z.rest, from the token each stands at, lists in shared
 // memory.
 template <bool LL, bool LONG, bool FEW>
-__global__ void __launch_bounds__(256, LONG ? 3 : 2) z_sweep_pairs_kernel(ListArgs a) {
+__global__ void __launch_bounds__(256, 2) z_sweep_pairs_kernel(ListArgs a) {
   extern __shared__ __align__(16) unsigned char zsm[];
   __shared__ unsigned long long blk_stats[4];  // tokens, documents, sparse work, sparse draws
   if (threadIdx.x < 4) blk_stats[threadIdx.x] = 0;
@@ -446,7 +526,7 @@ __global__ void __launch_bounds__(256, LONG ? 3 : 2) z_sweep_pairs_kernel(ListAr
   const ZLaunch& p = a.z;
   const u32 lane = threadIdx.x & 31;
   const u32 K = m.K, V = m.V, stride = bits_stride(m.K);
-  const WarpMem wm = warp_mem_at(zsm + (threadIdx.x >> 5) * warp_mem_bytes(a.cap, LONG && a.with_q), a.cap,
+  const WarpMem wm = warp_mem_at(zsm + (threadIdx.x >> 5) * warp_mem_bytes(a.cap, LONG ? K : 0u, LONG && a.with_q), a.cap,
                                  LONG && a.with_q);
   const u32 n_items = LONG ? *p.n_rest : p.n_docs;
   double ll_acc = 0.0, ll_skip = 0.0;
@@ -525,7 +605,7 @@ __global__ void __launch_bounds__(256, LONG ? 3 : 2) z_sweep_pairs_kernel(ListAr
       {
         const u64 aA = (u64)__double_as_longlong(__dmul_rn((double)m.alpha, exact_double(A1)));
         const u64 row = (u64)(m.q + my_row);
-        wm.stage[2 * lane] = make_uint4(z1 | (kd << 16), r.x, r.y, FEW ? w1 : 0u);
+        wm.stage[2 * lane] = make_uint4(z1 | (kd << 16), r.x, r.y, LONG ? my_nw : w1);
         wm.stage[2 * lane + 1] = make_uint4((u32)row, (u32)(row >> 32), (u32)aA, (u32)(aA >> 32));
       }
       __syncwarp();
@@ -542,7 +622,7 @@ __global__ void __launch_bounds__(256, LONG ? 3 : 2) z_sweep_pairs_kernel(ListAr
       w3 = word(base + 96);
       const u32 per = (n + 31) >> 5;
       if (LONG)
-        n = long_chunk(wm, n, nt, nz, lane);
+        n = long_chunk(wm, m.q, m.csr, n, nt, nz, lane);
       else if (per <= 2)
         n = list_chunk<2, FEW>(wm, m.bits, stride, n, nt, nz, lane);
       else if (per == 3)
@@ -634,11 +714,12 @@ void launch_lists(const ModelDev& m, const ZLaunch& z, cudaStream_t s, u32 cap) 
   auto kern = (z.flags & kZFlagLoglik) && z.ll ? z_sweep_pairs_kernel<true, LONG, FEW>
                                                    : z_sweep_pairs_kernel<false, LONG, FEW>;
   constexpr size_t kBudget = 200 * 1024;
-  static_assert(warp_mem_bytes(GPULDA_MAX_K + 32, false) <= kBudget, "a list of every topic fits");
-  a.with_q = LONG && warp_mem_bytes(cap, true) <= kBudget;
-  u32 warps = 8;
-  while (warps > 1 && warps * warp_mem_bytes(cap, a.with_q) > kBudget) --warps;
-  const size_t smem = warps * warp_mem_bytes(cap, a.with_q);
+  static_assert(warp_mem_bytes(GPULDA_MAX_K + 32, GPULDA_MAX_K, false) <= kBudget, "a list of every topic fits");
+  const u32 index = LONG ? m.K : 0u;
+  a.with_q = LONG && kStagedWarps * warp_mem_bytes(cap, index, true) <= kBudget;
+  const size_t per_warp = warp_mem_bytes(cap, index, a.with_q);
+  const u32 warps = (u32)std::min<size_t>(8, kBudget / per_warp);
+  const size_t smem = warps * per_warp;
   if (smem > 47 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBudget);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem);
