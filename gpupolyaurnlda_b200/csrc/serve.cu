@@ -106,18 +106,23 @@ struct FoldCommon {
 // records (the request is skipped).
 constexpr u32 kStatusBadRequest = 16;
 
-// A request as sweep_doc's source of tokens: n_iter passes over its nc chunks.
-// A chunk's topics are read a chunk ahead: with one chunk they are those just
-// drawn.
+// Chunks of a request that one call of sweep_doc goes through (at least a pass
+// over the longest request): it numbers them, and the three ahead, in 32 bits.
+constexpr u32 kFoldRun = 1u << 16;
+static_assert(kFoldRun >= 65535 / 32 + 1 && (u64)kFoldRun + 3 <= 0xffffffffull, "chunk numbers");
+
+// A request as sweep_doc's source of tokens: passes first .. over its nc chunks,
+// `chunks` in all.  A chunk's topics are read a chunk ahead: with one chunk they
+// are those just drawn.
 struct FoldSource {
   const u32* w_;
   const u32* z_;
-  u32 L, V, lane, nc, n_iter;
+  u32 L, V, lane, nc, first, chunks;
   u64 ridx;
   u32 k0, k1;
   u32 status;
   __device__ __forceinline__ u32 at(u32 c) const { return (c % nc) * 32 + lane; }
-  __device__ __forceinline__ bool valid(u32 c) const { return c < nc * n_iter && at(c) < L; }
+  __device__ __forceinline__ bool valid(u32 c) const { return c < chunks && at(c) < L; }
   __device__ __forceinline__ u32 word(u32 c) {
     u32 w = valid(c) ? __ldcg(w_ + at(c)) : 0u;
     if (w >= V) {
@@ -128,7 +133,7 @@ struct FoldSource {
   }
   __device__ __forceinline__ u32 topic(u32 c) const { return z_[at(c)]; }
   __device__ __forceinline__ U4 words(u32 c) const {
-    return draw4(ridx | at(c), c / nc, kStreamFold, 0, k0, k1);
+    return draw4(ridx | at(c), first + c / nc, kStreamFold, 0, k0, k1);
   }
   __device__ __forceinline__ void chunk_done(u32 c, u32 k, u32* z_next) const {
     if (nc == 1 && valid(c)) *z_next = valid(c + 1) ? k : *z_next;
@@ -168,10 +173,11 @@ __device__ __forceinline__ void fold_request(const FoldCommon& a, unsigned char*
     uint4* stage = reinterpret_cast<uint4*>(fsm + word_doc_bytes(K));
     word_doc_build<32>(wd, z, L, K, lane, &status, kStatusBadTopic);
 
-    {
-      const u32 nc = (L + 31) / 32;
-      FoldSource src{w, z, L, V, lane, nc ? nc : 1u, a.n_iter, ridx, k0, k1, 0u};
-      sweep_doc<32>(wd, stage, m, Rows{nullptr, nullptr}, K, alpha, nc * a.n_iter, lane, src,
+    const u32 nc = (L + 31) / 32, run = nc ? kFoldRun / nc : 0u;
+    for (u32 t = 0, n; nc && t < a.n_iter; t += n) {
+      n = min(run, a.n_iter - t);
+      FoldSource src{w, z, L, V, lane, nc, t, nc * n, ridx, k0, k1, 0u};
+      sweep_doc<32>(wd, stage, m, Rows{nullptr, nullptr}, K, alpha, nc * n, lane, src,
                     [&](u32 c, u32 new_z, bool, u32, u64, u32) {
                       const u32 i = (c % nc) * 32 + lane;
                       if (i < L) z[i] = new_z;
