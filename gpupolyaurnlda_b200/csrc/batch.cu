@@ -132,7 +132,7 @@ struct Batch {
   u32* order_all = nullptr;          // every document, longest first
   u64 cells = 0, N = 0, S_total = 0;
   u32 D = 0, Vtot = 0;
-  u64 bytes = 0;
+  u64 bytes = 0, lists_bytes = 0;
   u64 iters = 0;
   int t = -1;
 
@@ -186,6 +186,21 @@ struct Batch {
     ModelDev m = ar;
     m.shares = ar.S + S_total + 2 * j;
     return m;
+  }
+
+  // Memory for the time of a call, for which the words' lists are given up if
+  // need be (sweeps work without them).
+  cudaError_t scratch(u32** p, u64 count) {
+    const u64 n = std::max<u64>(1, count) * sizeof(u32);
+    cudaError_t e = cudaMalloc((void**)p, n);
+    if (e != cudaErrorMemoryAllocation || !ar.lists || cudaDeviceSynchronize() != cudaSuccess) return e;
+    cudaGetLastError();
+    drop_graph();
+    cudaFree(ar.lists);
+    allocs.erase(std::find(allocs.begin(), allocs.end(), (void*)ar.lists));
+    bytes -= lists_bytes;
+    ar.lists = nullptr;
+    return cudaMalloc((void**)p, n);
   }
 
   void drop_graph() {
@@ -493,7 +508,7 @@ int create_impl(const GpuldaProblem* probs, u32 P, Batch** out) {
   ModelDev& ar = b.ar;
   ar.V = b.Vtot;
   if ((rc = b.alloc(&ar.n, cells)) || (rc = b.alloc(&ar.q, cells)) || (rc = b.alloc(&ar.al, cells)) ||
-      (rc = b.alloc(&ar.csr, cells)) || (rc = b.alloc(&ar.lists, lists)) || (rc = b.alloc(&ar.A, W)) || (rc = b.alloc(&ar.S, S + kShares)) ||
+      (rc = b.alloc(&ar.csr, cells)) || (rc = b.alloc(&ar.A, W)) || (rc = b.alloc(&ar.S, S + kShares)) ||
       (rc = b.alloc(&ar.nnz, W)) || (rc = b.alloc(&b.z, N)) || (rc = b.alloc(&b.w, N)) ||
       (rc = b.alloc(&b.d_len, D)) || (rc = b.alloc(&b.d_idx, D)) || (rc = b.alloc(&b.order, D)) ||
       (rc = b.alloc(&b.order_all, D)) ||
@@ -623,6 +638,12 @@ int create_impl(const GpuldaProblem* probs, u32 P, Batch** out) {
   b.allocs.erase(std::find(b.allocs.begin(), b.allocs.end(), (void*)Cdev));
   b.bytes -= (u64)W * 4;
   if ((rc = upload_block_tables(b))) return rc;
+  ar.lists = try_alloc<u64>(lists);
+  if (ar.lists) {
+    b.allocs.push_back(ar.lists);
+    b.bytes += lists * 8;
+    b.lists_bytes = lists * 8;
+  }
   *out = holder.release();
   return GPULDA_OK;
 }
@@ -725,8 +746,8 @@ int tune_bucket(Batch& b, u32 j) {
   u32 *n_save = nullptr, *z_save = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   int rc = GPULDA_OK;
-  BCK(cudaMalloc(&n_save, std::max<u64>(1, cells) * 4));
-  if (cudaMalloc(&z_save, std::max<u64>(1, toks) * 4) != cudaSuccess) {
+  BCK(b.scratch(&n_save, cells));
+  if (b.scratch(&z_save, toks) != cudaSuccess) {
     cudaFree(n_save);
     return report_error(GPULDA_ERR_NOMEM, "autotuner snapshot");
   }
@@ -807,8 +828,8 @@ int tune_merged(Batch& b) {
   u32 *n_save = nullptr, *z_save = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   int rc = GPULDA_OK;
-  BCK(cudaMalloc(&n_save, std::max<u64>(1, b.cells) * 4));
-  if (cudaMalloc(&z_save, std::max<u64>(1, b.N) * 4) != cudaSuccess) {
+  BCK(b.scratch(&n_save, b.cells));
+  if (b.scratch(&z_save, b.N) != cudaSuccess) {
     cudaFree(n_save);
     return report_error(GPULDA_ERR_NOMEM, "autotuner snapshot");
   }

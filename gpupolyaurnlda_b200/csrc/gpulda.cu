@@ -166,6 +166,7 @@ struct Model {
   // (counts, statistics, log-likelihood) waits for it.
   cudaEvent_t noalloc_done = nullptr;
   bool noalloc_pending = false;
+  bool captured = false;  // an allocation-free sweep was issued on a capturing stream
 
   // device-resident corpus
   u64* crest = nullptr;  // documents that sweeps hand on (K > kMapMinK)
@@ -230,17 +231,33 @@ int cuda_fail(cudaError_t e, const char* where) {
 
 cudaStream_t main_stream() { return g.user_stream ? g.user_stream : g.stream; }
 
+void dfree(void* p) {
+  if (p) cudaFree(p);
+}
+
+// Gives back the tables that the model works without; false if there are none
+// (or a captured sweep may still read them).
+bool release_tables() {
+  if ((!g.dev.lists && !g.dev.bits) || g.captured || cudaDeviceSynchronize() != cudaSuccess) return false;
+  dfree(g.dev.lists);
+  dfree(g.dev.bits);
+  g.dev.lists = nullptr;
+  g.dev.shares = nullptr;
+  g.dev.bits = nullptr;
+  return true;
+}
+
 template <class T>
 int dalloc(T** p, size_t count) {
   *p = nullptr;
   if (!count) count = 1;
   cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
+  if (e == cudaErrorMemoryAllocation && release_tables()) {
+    cudaGetLastError();
+    e = cudaMalloc((void**)p, count * sizeof(T));
+  }
   if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc");
   return GPULDA_OK;
-}
-
-void dfree(void* p) {
-  if (p) cudaFree(p);
 }
 
 int check_status() {
@@ -330,8 +347,6 @@ int init_impl(const Args* args, Buffer* buffers, u32 n_buffers, const GpuldaExAr
   for (auto& e : g.z_ev) CK(cudaEventCreate(&e));
   if ((rc = dalloc(&g.dev.n, cells)) || (rc = dalloc(&g.dev.q, cells)) || (rc = dalloc(&g.dev.al, cells)) ||
       (rc = dalloc(&g.dev.csr, cells)) ||
-      (g.K <= kMapMinK && (rc = dalloc(&g.dev.lists, (size_t)g.V * list_stride(g.K)))) ||
-      (bits_pay(g.K, g.V) && (rc = dalloc(&g.dev.bits, (size_t)g.V * bits_stride(g.K)))) ||
       (rc = dalloc(&g.dev.A, g.V)) || (rc = dalloc(&g.dev.S, g.K + 2)) || (rc = dalloc(&g.dev.Sinv, g.K)) ||
       (rc = dalloc(&g.dev.nnz, g.V)) ||
       (rc = dalloc(&g.C, g.V)) || (rc = dalloc(&g.cdf, (size_t)kPoisN * kPoisW)) ||
@@ -368,7 +383,6 @@ int init_impl(const Args* args, Buffer* buffers, u32 n_buffers, const GpuldaExAr
   g.dev.beta = g.beta;
   g.dev.key0 = g.key0;
   g.dev.key1 = g.key1;
-  g.dev.shares = g.K <= kMapMinK ? g.dev.S + g.K : nullptr;
   g.dev.tables = PoisTables{g.cdf, g.guide, g.lfac};
 
   for (u32 i = 0; i < n_buffers; ++i) {
@@ -406,6 +420,9 @@ int init_impl(const Args* args, Buffer* buffers, u32 n_buffers, const GpuldaExAr
   launch_init_counts(g.dev, g.C, g.stream);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(g.stream));
+  if (g.K <= kMapMinK) g.dev.lists = try_alloc<u64>((size_t)g.V * list_stride(g.K));
+  if (g.dev.lists) g.dev.shares = g.dev.S + g.K;
+  if (bits_pay(g.K, g.V)) g.dev.bits = try_alloc<u32>((size_t)g.V * bits_stride(g.K));
   g.live = true;
   return GPULDA_OK;
 }
@@ -1120,6 +1137,8 @@ extern "C" int gpulda_sample_z_device_noalloc(uint32_t* z, const uint32_t* w, co
   u32* d_idx = g_noalloc_addr[dev];
   u32* work = d_idx + kNoAllocMaxDocs;
   cudaStream_t s = stream ? (cudaStream_t)stream : main_stream();
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture != cudaStreamCaptureStatusNone) g.captured = true;
   // the previous call's use of the shared scratch ends before this one's begins
   if (int rc = after_noalloc(s)) return rc;
   const int rc = noalloc_launches(s, z, w, d_len, n_docs, n_tokens, d_idx, work);

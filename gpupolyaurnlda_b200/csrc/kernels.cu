@@ -632,7 +632,7 @@ __device__ __forceinline__ void alias_word_of(const ModelDev& ar, const BatchPhi
                                               const AliasScratch& all, u32 smem_items, u64* sh) {
   const u32 pb = bp.wpid[w];
   const size_t row = bp.row_off[w];
-  alias_word(bp.K[pb], ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row, ar.lists + bp.list_off[w],
+  alias_word(bp.K[pb], ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row, ar.lists ? ar.lists + bp.list_off[w] : nullptr,
              nullptr, ar.A + w, s_shares, ar.nnz + w, all.vals, all.idx, smem_items, nullptr, nullptr, sh);
 }
 
@@ -718,7 +718,7 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_batch_kernel(
     const u32 pb = bp.wpid[w], K = bp.K[pb];
     const size_t row = bp.row_off[w];
     if (alias_word_warp(K, ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row,
-                        ar.lists + bp.list_off[w], nullptr, ar.A + w, ar.nnz + w, x_all, x_long, sm.ent, sm.vals, sm.idx, most))
+                        ar.lists ? ar.lists + bp.list_off[w] : nullptr, nullptr, ar.A + w, ar.nnz + w, x_all, x_long, sm.ent, sm.vals, sm.idx, most))
       continue;
     if ((threadIdx.x & 31) == 0) {
       ar.nnz[w] = kNnzWide;

@@ -87,13 +87,14 @@ struct ModelDev {
   u32* q;      // V*K fixed-point Phi (raw x between the two Phi kernels)
   u64* al;     // V*K alias entries
   u64* csr;    // V*K per-word lists of (q << 32 | k) for q > 0, ascending k, nnz[w] used
-  u64* lists;  // the same lists by eighths, list_stride(K) entries apart (K <= kMapMinK, else null)
-  u32* bits;   // a bit for each of a word's topics with q > 0, bits_stride(K) words a row (training, if bits_pay, else null)
+  u64* lists;  // the same lists by eighths, list_stride(K) entries apart (K <= kMapMinK and memory allowing, else null)
+  u32* bits;   // a bit for each of a word's topics with q > 0, bits_stride(K) words a row (training, if bits_pay and
+               // memory allowing, else null)
   u64* A;      // V   dense mass per word
   u64* S;      // K   per-topic normalisers
   u64* Sinv;   // K   floor((2^64 - 1) / S[k]), written by the alias build's launch (null: divide)
   u32* nnz;    // V   nonzero x per word
-  u64* shares; // 2   sum of x, and that of the words with long lists (K <= kMapMinK, else null)
+  u64* shares; // 2   sum of x, and that of the words with long lists (with `lists`, else null)
   PoisTables tables;
 };
 
@@ -162,6 +163,19 @@ struct ZLaunch {
   u64* rest = nullptr;
   u32* n_rest = nullptr;
 };
+
+// Memory for a table that sweeps are faster with and work without: `count`
+// elements, or null where they would take more than half of what is free.  (The
+// words' lists are another 9 bytes a cell at K=1000, beside 24.)
+template <class T>
+T* try_alloc(size_t count) {
+  size_t free = 0, total = 0;
+  void* p = nullptr;
+  if (cudaMemGetInfo(&free, &total) == cudaSuccess && count * sizeof(T) > free / 2) return nullptr;
+  if (cudaMalloc(&p, count * sizeof(T)) != cudaSuccess) p = nullptr;
+  if (!p) cudaGetLastError();
+  return (T*)p;
+}
 
 // Grid sizing helpers need the device's SM count.
 int device_sm_count();

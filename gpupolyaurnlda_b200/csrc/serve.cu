@@ -558,7 +558,7 @@ struct Server {
   }
 };
 
-int create_common(const GpuldaServeArgs* a, u32 K, u32 V, float alpha, std::unique_ptr<Server>& sv) {
+int create_common(const GpuldaServeArgs* a, u32 K, u32 V, float alpha, bool lists, std::unique_ptr<Server>& sv) {
   if (!a) return report_error(GPULDA_ERR_ARGS, "null GpuldaServeArgs");
   if (a->mode != GPULDA_SERVE_PERSISTENT && a->mode != GPULDA_SERVE_LAUNCH)
     return report_error(GPULDA_ERR_ARGS, "unknown serving mode");
@@ -583,7 +583,6 @@ int create_common(const GpuldaServeArgs* a, u32 K, u32 V, float alpha, std::uniq
   FoldCommon& fc = s.fc;
   int rc;
   if ((rc = s.alloc(&fc.m.q, cells)) || (rc = s.alloc(&fc.m.al, cells)) || (rc = s.alloc(&fc.m.csr, cells)) ||
-      (rc = s.alloc(&fc.m.lists, (size_t)V * list_stride(K))) ||
       (rc = s.alloc(&fc.m.A, V)) || (rc = s.alloc(&fc.m.nnz, V)) || (rc = s.alloc(&fc.status, 1)))
     return rc;
   fc.m.K = K;
@@ -634,13 +633,16 @@ int create_common(const GpuldaServeArgs* a, u32 K, u32 V, float alpha, std::uniq
       if ((rc = sl.st.init(kSlotStagingBytes))) return rc;
     }
   }
+  if (lists) fc.m.lists = try_alloc<u64>((size_t)V * list_stride(K));
+  if (fc.m.lists) s.allocs.push_back(fc.m.lists);
   SCK(cudaDeviceSynchronize());
   return GPULDA_OK;
 }
 
-// The walk for the model's requests: over the words' lists unless more than one
-// in 12 of a uniform mixture's tokens has a word with a long list (the training
-// sweep's rule, with the dense masses for the words' tokens).
+// The walk for the model's requests: over the words' lists, if there was memory
+// for them, unless more than one in 12 of a uniform mixture's tokens has a word
+// with a long list (the training sweep's rule, with the dense masses for the
+// words' tokens).
 int choose_walk(Server& s) {
   std::vector<u32> nnz(s.V);
   std::vector<u64> A(s.V);
@@ -651,7 +653,7 @@ int choose_walk(Server& s) {
     all += (double)A[w];
     if (nnz[w] > kShortList) in_long += (double)A[w];
   }
-  s.words = 12.0 * in_long <= all;
+  s.words = s.fc.m.lists && 12.0 * in_long <= all;
   return GPULDA_OK;
 }
 
@@ -860,14 +862,15 @@ extern "C" int gpulda_serve_create(const GpuldaServeArgs* args, void** handle) {
   if (!current_model(&src, &t)) return report_error(GPULDA_ERR_STATE, "no initialized model to serve");
   if (t < 0) return report_error(GPULDA_ERR_STATE, "the model has no Phi yet (no sample_phi)");
   std::unique_ptr<Server> sv;
-  int rc = create_common(args, src.K, src.V, src.alpha, sv);
+  int rc = create_common(args, src.K, src.V, src.alpha, src.lists != nullptr, sv);
   if (rc) return rc;
   Server& s = *sv;
   const size_t cells = (size_t)src.K * src.V;
   SCK(cudaMemcpy(s.fc.m.q, src.q, cells * 4, cudaMemcpyDeviceToDevice));
   SCK(cudaMemcpy(s.fc.m.al, src.al, cells * 8, cudaMemcpyDeviceToDevice));
   SCK(cudaMemcpy(s.fc.m.csr, src.csr, cells * 8, cudaMemcpyDeviceToDevice));
-  SCK(cudaMemcpy(s.fc.m.lists, src.lists, (size_t)src.V * list_stride(src.K) * 8, cudaMemcpyDeviceToDevice));
+  if (s.fc.m.lists)
+    SCK(cudaMemcpy(s.fc.m.lists, src.lists, (size_t)src.V * list_stride(src.K) * 8, cudaMemcpyDeviceToDevice));
   SCK(cudaMemcpy(s.fc.m.A, src.A, (size_t)src.V * 8, cudaMemcpyDeviceToDevice));
   SCK(cudaMemcpy(s.fc.m.nnz, src.nnz, (size_t)src.V * 4, cudaMemcpyDeviceToDevice));
   SCK(cudaDeviceSynchronize());
@@ -882,7 +885,7 @@ extern "C" int gpulda_serve_create_from_phi(const GpuldaServeArgs* args, uint32_
   *handle = nullptr;
   if (!q) return report_error(GPULDA_ERR_ARGS, "null Phi");
   std::unique_ptr<Server> sv;
-  int rc = create_common(args, K, V, alpha, sv);
+  int rc = create_common(args, K, V, alpha, true, sv);
   if (rc) return rc;
   Server& s = *sv;
   const size_t cells = (size_t)K * V;

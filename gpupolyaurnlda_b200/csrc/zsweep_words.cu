@@ -271,6 +271,14 @@ u32 launch_sweep(const ModelDev& m, const BatchDev* b, u32 Kmax, ZLaunch zl, con
                  u32 warps_per_block, u32 blocks_per_sm) {
   if (!zl.n_docs) return 0;
   zl.work = x.ctrs + kCtrWork;
+  if (Kmax <= kMapMinK && !m.lists) {  // (no memory for them)
+    zl.shares = nullptr;
+    if (b)
+      launch_z_sweep_batch(m, *b, Kmax, zl, s, warps_per_block, blocks_per_sm);
+    else
+      launch_z_sweep(m, zl, s);
+    return 1;
+  }
   if (Kmax <= kMapMinK) {
     // Both sweeps are launched where the words' lists may be long, and one of
     // them returns at once (3 us): which is known on the device only.
