@@ -422,7 +422,8 @@ int init_impl(const Args* args, Buffer* buffers, u32 n_buffers, const GpuldaExAr
   CK(cudaStreamSynchronize(g.stream));
   if (g.K <= kMapMinK) g.dev.lists = try_alloc<u64>((size_t)g.V * list_stride(g.K));
   if (g.dev.lists) g.dev.shares = g.dev.S + g.K;
-  if (bits_pay(g.K, g.V)) g.dev.bits = try_alloc<u32>((size_t)g.V * bits_stride(g.K));
+  if (bits_pay(g.K, g.V) && !(g.flags & GPULDA_FLAG_HASHMAP))
+    g.dev.bits = try_alloc<u32>((size_t)g.V * bits_stride(g.K));
   g.live = true;
   return GPULDA_OK;
 }

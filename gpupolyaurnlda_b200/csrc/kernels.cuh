@@ -42,7 +42,8 @@ __host__ __device__ inline u32 list_stride(u32 K) { return 16 * list_pairs(K); }
 // Words from one word's bits to the next: whole sectors.
 __host__ __device__ inline u32 bits_stride(u32 K) { return (K + 255) / 256 * 8; }
 
-// Whether a large-K model keeps them: where q takes several times the 126 MB of
+// Whether a large-K model keeps them (unless its sweeps are the hash map's, which
+// do not read them): where q takes several times the 126 MB of
 // L2, a gather of q mostly goes to HBM.  At 233 MB (K=7275) the bits made the
 // sweep 2.23 -> 2.44 ms and the alias build 0.36 -> 0.46; at 1.2 GB 13.7 -> 9.6
 // and 0.73 -> 0.78.
