@@ -398,7 +398,8 @@ __device__ __forceinline__ void alias_word(u32 K, u32* __restrict__ qrow, const 
     xsum = __reduce_add_sync(kFullMask, xsum);
     if ((threadIdx.x & 31) == 0) {
       atomicAdd((unsigned long long*)s_shares, (unsigned long long)xsum);
-      if (n > kShortList) atomicAdd((unsigned long long*)s_shares + 1, (unsigned long long)xsum);
+      if (n > kShortList)
+        atomicAdd((unsigned long long*)s_shares + 1, (unsigned long long)xsum * long_list_weight(n));
     }
   }
   if (eighths && n) {  // the list again, by eighths, with zeros to the end of the last
@@ -481,7 +482,7 @@ __device__ __forceinline__ bool alias_word_warp(u32 K, u32* qrow, const u64* __r
   __syncwarp();
   const u64 A = warp_sum_u64(part);
   x_all += xsum;
-  if (n > kShortList) x_long += xsum;
+  x_long += xsum * long_list_weight(n);
   for (u32 i = lane; i < n; i += 32) {
     const u64 e = ent[i];
     qrow[(u32)e] = (u32)(e >> 32);

@@ -80,6 +80,10 @@ __device__ __forceinline__ Run lane_run(u32 nw, u32 l) {
 // A word's list is short up to this many entries.
 constexpr u32 kShortList = 160;
 
+// How many tokens of words with short lists make up for one whose word has a list
+// of nw entries (mostly_long_lists).
+__host__ __device__ inline u32 long_list_weight(u32 nw) { return nw > kShortList ? 11 + nw * nw / 100000 : 0; }
+
 struct ModelDev {
   u32 K, V;
   float alpha, beta;
@@ -95,7 +99,7 @@ struct ModelDev {
   u64* S;      // K   per-topic normalisers
   u64* Sinv;   // K   floor((2^64 - 1) / S[k]), written by the alias build's launch (null: divide)
   u32* nnz;    // V   nonzero x per word
-  u64* shares; // 2   sum of x, and that of the words with long lists (with `lists`, else null)
+  u64* shares; // 2   sum of x, and that of x * long_list_weight(nnz) (with `lists`, else null)
   PoisTables tables;
 };
 
@@ -241,10 +245,14 @@ void launch_z_sweep_batch(const ModelDev& arenas, const BatchDev& b, u32 Kmax, c
 void launch_z_sweep_words(const ModelDev& m, const BatchDev* b, u32 Kmax, const ZLaunch& z, u32 n_long, cudaStream_t s,
                           u32 warps_per_block, u32 blocks_per_sm);
 // Whether so many tokens' words have long lists that the sweep over the
-// documents' topics and the words' lists is the faster: above one in 12 a step
-// of the other's four documents to a warp is a long one too often (0.17 ns a
-// token with none, 1.8 with mostly long lists, against 0.28 and 0.5).
-__device__ __forceinline__ bool mostly_long_lists(const u64* shares) { return 12 * shares[1] > shares[0]; }
+// documents' topics and the words' lists is the faster.  That one takes 0.27 to
+// 0.34 ns a token (3e6 tokens in documents of 100, K=200 to 2000), the other 0.14 to
+// 0.21 and, for a token whose word has a list of 200, 500, 1000 or 2000 entries,
+// 1.0, 1.5, 2.5 or 6.3 ns more (its warp's other documents wait): they are even
+// with one such token in 9, 10, 17 or 50; with documents of 400 in 20 or 70 of the
+// last two.  (One in 12 whatever the lengths: 2.15 for 1.03 ms with 8 % of the
+// tokens in lists of 2000 entries.)
+__device__ __forceinline__ bool mostly_long_lists(const u64* shares) { return shares[1] > shares[0]; }
 // The same sweep with each document's counts in a shared-memory hash map
 // (large K).  Documents longer than lmax are reported, not swept.  Returns
 // false without launching when lmax needs more shared memory than a block has.

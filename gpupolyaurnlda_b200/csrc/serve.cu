@@ -640,9 +640,8 @@ int create_common(const GpuldaServeArgs* a, u32 K, u32 V, float alpha, bool list
 }
 
 // The walk for the model's requests: over the words' lists, if there was memory
-// for them, unless more than one in 12 of a uniform mixture's tokens has a word
-// with a long list (the training sweep's rule, with the dense masses for the
-// words' tokens).
+// for them, unless too many of a uniform mixture's tokens have a word with a long
+// list (the training sweep's rule, with the dense masses for the words' tokens).
 int choose_walk(Server& s) {
   std::vector<u32> nnz(s.V);
   std::vector<u64> A(s.V);
@@ -651,9 +650,9 @@ int choose_walk(Server& s) {
   double all = 0.0, in_long = 0.0;
   for (u32 w = 0; w < s.V; ++w) {
     all += (double)A[w];
-    if (nnz[w] > kShortList) in_long += (double)A[w];
+    in_long += (double)A[w] * long_list_weight(nnz[w]);
   }
-  s.words = s.fc.m.lists && 12.0 * in_long <= all;
+  s.words = s.fc.m.lists && in_long <= all;
   return GPULDA_OK;
 }
 
