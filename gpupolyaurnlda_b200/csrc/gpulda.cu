@@ -266,9 +266,10 @@ int check_status() {
   if (st) {
     CK(cudaMemset(g.status, 0, sizeof(u32)));
     char buf[200];
-    snprintf(buf, sizeof buf, "device status 0x%x (%s%s%s%s)", st, (st & kStatusBadTopic) ? "topic>=K " : "",
+    snprintf(buf, sizeof buf, "device status 0x%x (%s%s%s%s%s)", st, (st & kStatusBadTopic) ? "topic>=K " : "",
              (st & kStatusBadWord) ? "word>=V " : "", (st & kStatusDocRange) ? "document past n_tokens " : "",
-             (st & kStatusDocTooLong) ? "document too long " : "");
+             (st & kStatusDocTooLong) ? "document too long " : "",
+             (st & kStatusListFull) ? "document's list too small " : "");
     return fail(GPULDA_ERR_DEVICE, buf);
   }
   return GPULDA_OK;

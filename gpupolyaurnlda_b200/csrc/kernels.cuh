@@ -14,6 +14,7 @@ enum StatusBits : u32 {
   kStatusBadWord = 2,     // a w value >= V (used modulo V)
   kStatusDocRange = 4,    // a document runs past n_tokens (skipped)
   kStatusDocTooLong = 8,  // a document longer than the count width allows (skipped)
+  kStatusListFull = 32,   // a list sized for its document was too small (cannot happen; the rest is skipped)
 };
 
 // Counter slots written by the z sweep.

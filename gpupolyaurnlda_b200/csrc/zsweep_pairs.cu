@@ -44,7 +44,6 @@ namespace gpulda {
 namespace {
 
 constexpr u32 kMaxDocLen = 65535u;
-constexpr u32 kStatusListFull = 32;  // a list sized for its document was too small (cannot happen)
 constexpr u32 kNone = 0xffffu;     // no topic (topics are below 32768)
 constexpr u32 kSparseBit = 0x8000u;
 constexpr u32 kLongAhead = 4;  // entries of a word's list that a lane reads ahead (2: up to a third slower)
