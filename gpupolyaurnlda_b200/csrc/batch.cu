@@ -141,7 +141,6 @@ struct Batch {
   u32 *z = nullptr, *w = nullptr, *d_len = nullptr, *d_idx = nullptr, *order = nullptr;
   u32 *pid = nullptr, *wpid = nullptr;
   u64 *row_off = nullptr, *list_off = nullptr;
-  u32 lmax = 0;         // longest document
   u32 n_chain = 0;      // documents of order_all that take a warp each
   u32 *K = nullptr, *key0 = nullptr, *key1 = nullptr;
   float *alpha = nullptr, *beta = nullptr;
@@ -178,7 +177,8 @@ struct Batch {
     return BatchDev{pid, row_off, list_off, K, alpha, key0, key1, tok_base, lg_a, lg_Ka};
   }
   BatchPhiDev phidev(u32 block0) const {
-    return BatchPhiDev{blocks + block0, K, cell_base, S_off, beta, key0, key1, wpid, row_off, list_off, cdf, guide, lfac};
+    return BatchPhiDev{blocks + block0, K,       cell_base, S_off, beta,  key0, key1,
+                       wpid,            row_off, list_off,  cdf,   guide, lfac};
   }
 
   // The arenas with the shares of bucket j's (or the merged) launches.
@@ -306,7 +306,7 @@ void bucket_sweep(const Batch& b, u32 j, unsigned long long* counters, double* l
   const Bucket& bu = b.bk[j];
   const BatchDev bd = b.zdev();
   launch_sweep(b.arena(j), &bd, bu.Kmax, z_args(b, j, counters, ll),
-               SweepAux{b.work + j * kSweepCtrs, nullptr, b.lmax, bu.n_chain}, s, shape.z_warps_per_block,
+               SweepAux{b.work + j * kSweepCtrs, nullptr, 0, bu.n_chain}, s, shape.z_warps_per_block,
                shape.z_blocks_per_sm);
 }
 
@@ -314,7 +314,7 @@ void merged_sweep(const Batch& b, unsigned long long* counters, double* ll, cons
                   cudaStream_t s) {
   const BatchDev bd = b.zdev();
   launch_sweep(b.arena(kMergedWork), &bd, b.Kmax_all, z_args_merged(b, counters, ll),
-               SweepAux{b.work + kMergedWork * kSweepCtrs, nullptr, b.lmax, b.n_chain}, s, shape.z_warps_per_block,
+               SweepAux{b.work + kMergedWork * kSweepCtrs, nullptr, 0, b.n_chain}, s, shape.z_warps_per_block,
                shape.z_blocks_per_sm);
 }
 
@@ -512,7 +512,8 @@ int create_impl(const GpuldaProblem* probs, u32 P, Batch** out) {
       (rc = b.alloc(&ar.nnz, W)) || (rc = b.alloc(&b.z, N)) || (rc = b.alloc(&b.w, N)) ||
       (rc = b.alloc(&b.d_len, D)) || (rc = b.alloc(&b.d_idx, D)) || (rc = b.alloc(&b.order, D)) ||
       (rc = b.alloc(&b.order_all, D)) ||
-      (rc = b.alloc(&b.pid, D)) || (rc = b.alloc(&b.wpid, W)) || (rc = b.alloc(&b.row_off, W)) || (rc = b.alloc(&b.list_off, W)) ||
+      (rc = b.alloc(&b.pid, D)) || (rc = b.alloc(&b.wpid, W)) || (rc = b.alloc(&b.row_off, W)) ||
+      (rc = b.alloc(&b.list_off, W)) ||
       (rc = b.alloc(&b.K, P)) || (rc = b.alloc(&b.key0, P)) || (rc = b.alloc(&b.key1, P)) ||
       (rc = b.alloc(&b.alpha, P)) || (rc = b.alloc(&b.beta, P)) || (rc = b.alloc(&b.tok_base, P)) ||
       (rc = b.alloc(&b.cell_base, P)) || (rc = b.alloc(&b.S_off, P)) || (rc = b.alloc(&b.lg_a, P)) ||
@@ -622,7 +623,6 @@ int create_impl(const GpuldaProblem* probs, u32 P, Batch** out) {
     }
     for (u32 d = 0; d < D; ++d) order_all[d] = d;
     std::stable_sort(order_all.begin(), order_all.end(), [&](u32 x, u32 y) { return lens[x] > lens[y]; });
-    if (D) b.lmax = lens[order_all[0]];
     const u32 chain = long_document(N);
     while (b.n_chain < D && lens[order_all[b.n_chain]] >= chain) ++b.n_chain;
   }

@@ -459,7 +459,7 @@ int phi_step_async(cudaStream_t s) {
 }
 
 ZLaunch z_args(u32* z, const u32* w, const u32* d_len, const u32* d_idx, const u32* order, u32* K_d, u32 n_docs,
-               u64 n_tokens, u64 tok_base, u32* work) {
+               u64 n_tokens, u64 tok_base) {
   ZLaunch zl;
   zl.w = w;
   zl.z = z;
@@ -474,7 +474,7 @@ ZLaunch z_args(u32* z, const u32* w, const u32* d_len, const u32* d_idx, const u
   zl.flags = (g.flags & GPULDA_FLAG_LOGLIK) ? kZFlagLoglik : 0u;
   zl.counters = g.counters;
   zl.ll = g.ll;
-  zl.work = work;
+  zl.work = nullptr;  // set with the launch's counters
   zl.status = g.status;
   return zl;
 }
@@ -510,7 +510,7 @@ int z_step_async(cudaStream_t s, u32* z, const u32* w, const u32* d_len, u32* d_
   auto section = [&](u32 a, u32 b, u32 lmax) {
     if (a == b || rc) return;
     const ZLaunch zl =
-        z_args(z, w, d_len, d_idx, order + a, K_d, b - a, n_tokens, g.tok_offset, nullptr);
+        z_args(z, w, d_len, d_idx, order + a, K_d, b - a, n_tokens, g.tok_offset);
     rc = z_launch(s, zl, SweepAux{work, rest, lmax, split.n_chain});
   };
   if (g.K > kMapMinK && (g.flags & GPULDA_FLAG_HASHMAP)) {
@@ -607,7 +607,7 @@ int pipelined_sweep(Buffer* b, BufCtx* ctx) {
     const u32 d0 = dcut[p];
     const u32* order = ctx->order + d0 + a;
     const ZLaunch zl =
-        z_args(gz, gw, gdl + d0, gdi + d0, order, gkd + d0, b2 - a, b->n_tokens, tok_base, nullptr);
+        z_args(gz, gw, gdl + d0, gdi + d0, order, gkd + d0, b2 - a, b->n_tokens, tok_base);
     return z_launch(st, zl, SweepAux{ctx->work + slot * kSweepCtrs, nullptr, b->d[d0 + ctx->order_host[d0 + a]],
                                      n_chain[p] > a ? n_chain[p] - a : 0u});
   };
@@ -1098,7 +1098,7 @@ int noalloc_launches(cudaStream_t s, u32* z, const u32* w, const u32* d_len, u32
   // first, which the device finds out: 60,000 of 340 tokens' mean from a random
   // start 17.5 -> 13.2 ms an iteration.  Fewer start at once, a warp each,
   // in any order, and the three launches (9 us) would be lost on them.
-  ZLaunch zl = z_args(z, w, d_len, d_idx, nullptr, nullptr, n_docs, n_tokens, g.tok_offset, nullptr);
+  ZLaunch zl = z_args(z, w, d_len, d_idx, nullptr, nullptr, n_docs, n_tokens, g.tok_offset);
   u32 n_long = n_docs;
   if (n_docs > 16u * (u32)device_sm_count()) {
     const DocPlan plan = doc_plan_at(order + kNoAllocMaxDocs);

@@ -355,10 +355,9 @@ __device__ __forceinline__ void list_bits(const u64* ent, u32 n, u32* bits, u32 
 }
 
 __device__ __forceinline__ void alias_word(u32 K, u32* __restrict__ qrow, const u64* __restrict__ S,
-                                           const u64* __restrict__ Sinv, u64* alrow, u64* csrrow, u64* eighths, u32* bits, u64* A_out,
-                                           u64* s_shares,
-                                           u32* nnz_out, u64* s_vals, uint16_t* s_idx, u32 smem_items, u64* g_vals,
-                                           uint16_t* g_idx, u64* sh) {
+                                           const u64* __restrict__ Sinv, u64* alrow, u64* csrrow, u64* eighths,
+                                           u32* bits, u64* A_out, u64* s_shares, u32* nnz_out, u64* s_vals,
+                                           uint16_t* s_idx, u32 smem_items, u64* g_vals, uint16_t* g_idx, u64* sh) {
   u64 part = 0, nz = 0;
   u32 xsum = 0;
   if (bits)
@@ -432,8 +431,8 @@ __device__ __forceinline__ void alias_word(u32 K, u32* __restrict__ qrow, const 
 // to 1000 topics) 337 -> 146.
 __device__ __forceinline__ bool alias_word_warp(u32 K, u32* qrow, const u64* __restrict__ S,
                                                 const u64* __restrict__ Sinv, u64* alrow, u64* csrrow, u64* eighths,
-                                                u32* bits, u64* A_out, u32* nnz_out, u64& x_all, u64& x_long, u64* ent, u64* vals,
-                                                uint16_t* idx, u32 most) {
+                                                u32* bits, u64* A_out, u32* nnz_out, u64& x_all, u64& x_long,
+                                                u64* ent, u64* vals, uint16_t* idx, u32 most) {
   constexpr u32 kInFlight = 4;  // loads of 512 bytes; 8 take registers and a resident block (mid 212 -> 239 us)
   const u32 lane = threadIdx.x & 31, before = (1u << lane) - 1;
   const u32 head = (u32)((uintptr_t)qrow >> 2) & 3;  // the row starts inside an aligned group of four
@@ -633,8 +632,9 @@ __device__ __forceinline__ void alias_word_of(const ModelDev& ar, const BatchPhi
                                               const AliasScratch& all, u32 smem_items, u64* sh) {
   const u32 pb = bp.wpid[w];
   const size_t row = bp.row_off[w];
-  alias_word(bp.K[pb], ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row, ar.lists ? ar.lists + bp.list_off[w] : nullptr,
-             nullptr, ar.A + w, s_shares, ar.nnz + w, all.vals, all.idx, smem_items, nullptr, nullptr, sh);
+  alias_word(bp.K[pb], ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row,
+             ar.lists ? ar.lists + bp.list_off[w] : nullptr, nullptr, ar.A + w, s_shares, ar.nnz + w, all.vals, all.idx,
+             smem_items, nullptr, nullptr, sh);
 }
 
 __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_kernel(ModelDev m, u32 most) {
@@ -719,7 +719,8 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_batch_kernel(
     const u32 pb = bp.wpid[w], K = bp.K[pb];
     const size_t row = bp.row_off[w];
     if (alias_word_warp(K, ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row,
-                        ar.lists ? ar.lists + bp.list_off[w] : nullptr, nullptr, ar.A + w, ar.nnz + w, x_all, x_long, sm.ent, sm.vals, sm.idx, most))
+                        ar.lists ? ar.lists + bp.list_off[w] : nullptr, nullptr, ar.A + w, ar.nnz + w, x_all, x_long,
+                        sm.ent, sm.vals, sm.idx, most))
       continue;
     if ((threadIdx.x & 31) == 0) {
       ar.nnz[w] = kNnzWide;

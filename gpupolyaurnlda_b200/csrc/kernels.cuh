@@ -276,7 +276,7 @@ enum SweepCtrSlots { kCtrWork = 0, kCtrRestWork = 1, kCtrRest = 2 };
 struct SweepAux {
   u32* ctrs;   // kSweepCtrs
   u64* queue;  // a document each (K > kMapMinK)
-  u32 lmax;    // longest document
+  u32 lmax;    // longest document (K > kMapMinK)
   u32 n_long;  // documents to take a warp each (K <= kMapMinK; long_document)
 };
 u32 launch_sweep(const ModelDev& m, const BatchDev* b, u32 Kmax, ZLaunch zl, const SweepAux& x, cudaStream_t s,

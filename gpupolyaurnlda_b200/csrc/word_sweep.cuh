@@ -42,8 +42,12 @@ __host__ __device__ __forceinline__ size_t word_doc_bytes(u32 Kmax) { return (si
 __host__ __device__ constexpr size_t stage_bytes(u32 W) { return (32 / W) * (W + 1) * 32; }
 
 // Shared memory per warp, with four documents or one.
-__host__ __device__ __forceinline__ size_t word_warp_bytes(u32 Kmax) { return word_doc_bytes(Kmax) * 4 + stage_bytes(8); }
-__host__ __device__ __forceinline__ size_t word_warp_bytes_one(u32 Kmax) { return word_doc_bytes(Kmax) + stage_bytes(32); }
+__host__ __device__ __forceinline__ size_t word_warp_bytes(u32 Kmax) {
+  return word_doc_bytes(Kmax) * 4 + stage_bytes(8);
+}
+__host__ __device__ __forceinline__ size_t word_warp_bytes_one(u32 Kmax) {
+  return word_doc_bytes(Kmax) + stage_bytes(32);
+}
 
 // Flag beside a drawn topic: the sparse branch drew it.
 constexpr u32 kWordSparse = 0x10000u;
@@ -58,38 +62,6 @@ template <u32 W>
 __device__ __forceinline__ u32 group_ballot(bool p, u32 lane) {
   const u32 b = __ballot_sync(kFullMask, p);
   return W == 32 ? b : (b >> (lane & (32 - W))) & ((1u << (W & 31)) - 1u);
-}
-
-// Inclusive scan over the group's lanes: the shuffle's own predicate guards the
-// two-word add.
-template <u32 W>
-__device__ __forceinline__ u64 group_scan(u64 x) {
-#pragma unroll
-  for (u32 o = 1; o < W; o <<= 1)
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        ".reg .u32 a0, a1, b0, b1;\n\t"
-        "mov.b64 {a0, a1}, %0;\n\t"
-        "shfl.sync.up.b32 b0|p, a0, %1, %2, 0xffffffff;\n\t"
-        "shfl.sync.up.b32 b1, a1, %1, %2, 0xffffffff;\n\t"
-        "@p add.cc.u32 a0, a0, b0;\n\t"
-        "@p addc.u32 a1, a1, b1;\n\t"
-        "mov.b64 %0, {a0, a1};\n\t"
-        "}"
-        : "+l"(x)
-        : "r"(o), "r"((32 - W) << 8));
-  return x;
-}
-
-template <u32 W>
-__device__ __forceinline__ u32 group_scan32(u32 x, u32 l) {
-#pragma unroll
-  for (u32 o = 1; o < W; o <<= 1) {
-    const u32 y = __shfl_up_sync(kFullMask, x, o, W);
-    x += l >= o ? y : 0u;
-  }
-  return x;
 }
 
 template <u32 W, class T>
@@ -163,26 +135,6 @@ __device__ __forceinline__ bool counts_move(const WordDoc& dc, u32 k, u32 z, u32
 
 // --- draws -------------------------------------------------------------------------
 
-// Integers below 2^52 as doubles, exactly: the integer is the low mantissa of
-// 2^52, which is subtracted again.
-__device__ __forceinline__ double exact_double(u64 x) {
-  return __dadd_rn(__hiloint2double((int)(0x43300000u | (u32)(x >> 32)), (int)(u32)x), -4503599627370496.0);
-}
-
-// r / 2^32, exactly, the same way from 2^20.
-__device__ __forceinline__ double exact_unit(u32 r) {
-  return __dadd_rn(__hiloint2double(0x41300000, (int)r), -1048576.0);
-}
-
-// The mixture test: u * (alpha A + B) < B in double, alpha A rounded once.  B is
-// below 2^48 (65535 tokens of mass below 2^32).
-__device__ __forceinline__ bool sparse_test(u32 r, double aA, u64 B) {
-  const double b = exact_double(B);
-  return __dmul_rn(exact_unit(r), __dadd_rn(aA, b)) < b;
-}
-
-__device__ __forceinline__ ulonglong2 ld_pair(const u64* p) { return __ldg(reinterpret_cast<const ulonglong2*>(p)); }
-
 __device__ __forceinline__ u64 mass_of(const uint16_t* cnt, u64 ent) {
   return (u64)cnt[(u32)ent] * (u32)(ent >> 32);
 }
@@ -206,8 +158,9 @@ struct Staged {  // a token's data, read back by its group
 
 __device__ __forceinline__ Staged staged(const uint4* gs, u32 j) { return Staged{gs[2 * j], gs[2 * j + 1]}; }
 
-// The draw of one token of each group over lists of any length.  Out of line: the common draws' loop stays small enough for the
-// instruction cache.  Returns the topic, with kWordSparse.
+// The draw of one token of each group over lists of any length.  Out of line:
+// the common draws' loop stays small enough for the instruction cache.  Returns
+// the topic, with kWordSparse.
 template <u32 W>
 static __device__ __noinline__ u32 long_draw(const uint16_t* cnt, Staged c, u32 lane) {
   const u32 l = group_lane<W>(lane);

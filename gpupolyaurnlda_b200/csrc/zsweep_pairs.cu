@@ -93,42 +93,6 @@ struct ListArgs {
   double lg_a;   // lgamma(alpha)
 };
 
-// Inclusive scan of u64 over the warp: the shuffle's own predicate guards the
-// two-word add.
-__device__ __forceinline__ u64 scan64(u64 x) {
-#pragma unroll
-  for (u32 o = 1; o < 32; o <<= 1)
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        ".reg .u32 a0, a1, b0, b1;\n\t"
-        "mov.b64 {a0, a1}, %0;\n\t"
-        "shfl.sync.up.b32 b0|p, a0, %1, 0, 0xffffffff;\n\t"
-        "shfl.sync.up.b32 b1, a1, %1, 0, 0xffffffff;\n\t"
-        "@p add.cc.u32 a0, a0, b0;\n\t"
-        "@p addc.u32 a1, a1, b1;\n\t"
-        "mov.b64 %0, {a0, a1};\n\t"
-        "}"
-        : "+l"(x)
-        : "r"(o));
-  return x;
-}
-
-// Integers below 2^52 as doubles, exactly: the integer is the low mantissa of
-// 2^52, which is subtracted again.
-__device__ __forceinline__ double exact_double(u64 x) {
-  return __dadd_rn(__hiloint2double((int)(0x43300000u | (u32)(x >> 32)), (int)(u32)x), -4503599627370496.0);
-}
-
-// The mixture test u * (alpha A + B) < B in double, alpha A rounded once; u = r /
-// 2^32, exactly, by the same way from 2^20.  B is below 2^48 (65535 tokens of
-// mass below 2^32).
-__device__ __forceinline__ bool sparse_test(u32 r, double aA, u64 B) {
-  const double b = exact_double(B);
-  const double u = __dadd_rn(__hiloint2double(0x41300000, (int)r), -1048576.0);
-  return __dmul_rn(u, __dadd_rn(aA, b)) < b;
-}
-
 __device__ __forceinline__ u32 scan32(u32 x, u32 lane) {
 #pragma unroll
   for (u32 o = 1; o < 32; o <<= 1) {
@@ -285,7 +249,7 @@ __device__ __forceinline__ u32 list_chunk(const WarpMem& wm, const u32* __restri
     a = wm.stage[2 * (j + 1)];
     b = wm.stage[2 * (j + 1) + 1];
     if (more) fetch(kd);
-    const u64 incl = scan64(x);
+    const u64 incl = group_scan<32>(x);
     const u64 B = __shfl_sync(kFullMask, incl, 31);
     const bool sp = sparse_test(r0, aA, B);
     u64 t = scale_u32(r1, B);
@@ -421,7 +385,7 @@ static __device__ __noinline__ u32 long_chunk(const WarpMem wm, const u32* q0, c
       }
       __syncwarp();
       if (more) fetch(j + 1, pos);
-      const u64 incl = scan64(x);
+      const u64 incl = group_scan<32>(x);
       const u64 B = __shfl_sync(kFullMask, incl, 31);
       sp = sparse_test(a.y, aA, B);
       if (sp) {
@@ -438,7 +402,7 @@ static __device__ __noinline__ u32 long_chunk(const WarpMem wm, const u32* q0, c
           const u32 f1 = min(nw, f * per + per);
           for (u32 e = f * per; e < f1; e += 32) {
             u32 p;
-            const u64 in2 = scan64(look_up(e + lane < f1 ? __ldg(crow + e + lane) : 0ull, &p));
+            const u64 in2 = group_scan<32>(look_up(e + lane < f1 ? __ldg(crow + e + lane) : 0ull, &p));
             const u64 all = __shfl_sync(kFullMask, in2, 31);
             if (all > t) {
               pos = __shfl_sync(kFullMask, p, __popc(__ballot_sync(kFullMask, in2 <= t)));
@@ -473,7 +437,7 @@ static __device__ __noinline__ u32 long_chunk(const WarpMem wm, const u32* q0, c
         }
       }
       __syncwarp();
-      const u64 incl = scan64(x);
+      const u64 incl = group_scan<32>(x);
       const u64 B = __shfl_sync(kFullMask, incl, 31);
       sp = sparse_test(a.y, aA, B);
       if (sp) {
@@ -485,7 +449,7 @@ static __device__ __noinline__ u32 long_chunk(const WarpMem wm, const u32* q0, c
         for (u32 e = f * per; e < f1; e += 32) {
           const u32 v = e + lane < f1 ? list[e + lane] : 0u;
           const u32 y = v & 0xffffu ? (wm.q ? q[e + lane] : __ldg(row + (v >> 16))) : 0u;
-          const u64 in2 = scan64((u64)(v & 0xffffu) * y);
+          const u64 in2 = group_scan<32>((u64)(v & 0xffffu) * y);
           const u64 all = __shfl_sync(kFullMask, in2, 31);
           if (all > t) {
             pos = e + __popc(__ballot_sync(kFullMask, in2 <= t));
@@ -525,8 +489,9 @@ __global__ void __launch_bounds__(256, 2) z_sweep_pairs_kernel(ListArgs a) {
   const ZLaunch& p = a.z;
   const u32 lane = threadIdx.x & 31;
   const u32 K = m.K, V = m.V, stride = bits_stride(m.K);
-  const WarpMem wm = warp_mem_at(zsm + (threadIdx.x >> 5) * warp_mem_bytes(a.cap, LONG ? K : 0u, LONG && a.with_q), a.cap,
-                                 LONG && a.with_q);
+  const bool with_q = LONG && a.with_q;
+  const WarpMem wm =
+      warp_mem_at(zsm + (threadIdx.x >> 5) * warp_mem_bytes(a.cap, LONG ? K : 0u, with_q), a.cap, with_q);
   const u32 n_items = LONG ? *p.n_rest : p.n_docs;
   double ll_acc = 0.0, ll_skip = 0.0;
   u32 status = 0;
@@ -661,7 +626,8 @@ __global__ void __launch_bounds__(256, 2) z_sweep_pairs_kernel(ListArgs a) {
     if (over) {  // the rest of the document is the other kernel's (whose lists are long enough)
       if (LONG)
         status |= kStatusListFull;
-      else if (lane == 0) p.rest[atomicAdd(p.n_rest, 1u)] = (u64)start << 32 | doc;
+      else if (lane == 0)
+        p.rest[atomicAdd(p.n_rest, 1u)] = (u64)start << 32 | doc;
       __syncwarp();
       continue;
     }
@@ -696,10 +662,6 @@ __global__ void __launch_bounds__(256, 2) z_sweep_pairs_kernel(ListArgs a) {
     atomicAdd(p.counters + kCtrSparseDraws, blk_stats[3]);
   }
 }
-
-}  // namespace
-
-namespace {
 
 template <bool LONG, bool FEW>
 void launch_lists(const ModelDev& m, const ZLaunch& z, cudaStream_t s, u32 cap) {
