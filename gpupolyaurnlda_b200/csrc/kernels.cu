@@ -335,8 +335,8 @@ __device__ __forceinline__ u64 fixed_phi(u32 x, u32 k, const u64* __restrict__ S
 constexpr u32 kPerThread = 8;
 constexpr u32 kAliasWarps = 4;  // a block's, a word each
 // Most topics of a word that a warp takes (18 bytes each set how many warps are
-// resident); a longer word takes a block, of a launch of its own where K has room
-// for such words.  K=1000: 128, 256 and 512 take 218,
+// resident); a longer word takes a block, above K = 2048 of a launch of its own.
+// K=1000: 128, 256 and 512 take 218,
 // 210 and 243 us at the mid corpus; K=10000, whose words' lists are longer: 1350,
 // 900 and 700 us.
 inline u32 alias_items(u32 K) { return std::min(K, K <= kMapMinK ? 256u : 512u); }
@@ -586,17 +586,41 @@ struct AliasSmem {
   uint16_t* idx;
   AliasScratch all;     // the block's
 };
-__device__ __forceinline__ AliasSmem alias_smem(unsigned char* raw, u32 most) {
+__device__ __forceinline__ AliasSmem alias_smem(unsigned char* raw, u32 most, u32 items) {
   AliasSmem a;
   unsigned char* own = raw + (size_t)(threadIdx.x >> 5) * alias_warp_bytes(most);
   a.ent = (u64*)own;
   a.vals = a.ent + most;
   a.idx = (uint16_t*)(a.vals + most);
-  a.all = alias_scratch_at(raw, most);
+  a.all = alias_scratch_at(raw, items);
   return a;
 }
 
 constexpr u32 kNnzWide = 0xffffffffu;  // marks a word that its warp left to a block
+
+// The i-th of a block's words: four neighbours at a time, or (spread) every
+// gridDim-th.  Words are ranked by frequency, so those with many topics are
+// neighbours, and a block builds those that its warps leave one after another.
+__device__ __forceinline__ u64 alias_nth(u32 i, bool spread) {
+  if (spread) return blockIdx.x + (u64)i * gridDim.x;
+  return ((u64)(i / kAliasWarps) * gridDim.x + blockIdx.x) * kAliasWarps + i % kAliasWarps;
+}
+
+// Blocks of an alias build over V words with room for `resident` of them on the
+// GPU, and whether they spread: with few words, so that each block has about one
+// of many topics (K=2000, 2,000 words of 250 topics: 140 us with four neighbours to
+// a block).  With many, the blocks are enough, and neighbours cost less (1e5
+// words 259 us, 269 spread).
+struct AliasGrid {
+  u32 blocks;
+  bool spread;
+};
+inline AliasGrid alias_grid(u32 V, u32 K, u32 most, u32 resident) {
+  AliasGrid g;
+  g.spread = K > most && V < 16 * resident;
+  g.blocks = std::min(std::max((V + kAliasWarps - 1) / kAliasWarps, g.spread ? std::min(V, resident) : 1u), 4 * resident);
+  return g;
+}
 
 // f(w) for the block's words of [w0, w1) that are marked, every gridDim-th, all
 // threads together.
@@ -637,18 +661,21 @@ __device__ __forceinline__ void alias_word_of(const ModelDev& ar, const BatchPhi
              smem_items, nullptr, nullptr, sh);
 }
 
-__global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_kernel(ModelDev m, u32 most) {
+// items: most topics of a word that the block takes (at least K, or 0: those that
+// its warps leave are alias_wide_kernel's).
+__global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_kernel(ModelDev m, u32 most, u32 items,
+                                                                       bool spread) {
   extern __shared__ __align__(16) unsigned char s_raw[];
   __shared__ u64 sh[33], sh_shares[2];
   __shared__ u32 wide;
-  const u32 K = m.K, nw = blockDim.x >> 5, warp = threadIdx.x >> 5;
+  const u32 K = m.K, warp = threadIdx.x >> 5;
   if (threadIdx.x < 2) sh_shares[threadIdx.x] = 0;
   if (threadIdx.x == 0) wide = 0;
   __syncthreads();
-  const AliasSmem sm = alias_smem(s_raw, most);
+  const AliasSmem sm = alias_smem(s_raw, most, items);
   u64 x_all = 0, x_long = 0;
-  const u64 step = (u64)gridDim.x * nw;
-  for (u64 w = (u64)blockIdx.x * nw + warp; w < m.V; w += step) {
+  u64 w;
+  for (u32 i = warp; (w = alias_nth(i, spread)) < m.V; i += kAliasWarps) {
     const size_t row = (size_t)w * K;
     if (alias_word_warp(K, m.q + row, m.S, m.Sinv, m.al + row, m.csr + row,
                         m.lists ? m.lists + (size_t)w * list_stride(K) : nullptr,
@@ -670,52 +697,43 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_kernel(ModelD
     }
   }
   __syncthreads();
-  if (wide && K <= most) {  // (draws that round to q = 0: no launch of their own)
-    for (u64 w0 = (u64)blockIdx.x * nw; w0 < m.V; w0 += step)
-      for (u64 w = w0; w < min((u64)m.V, w0 + nw); ++w)
-        if (m.nnz[w] == kNnzWide) alias_word_of(m, w, m.shares ? sh_shares : nullptr, sm.all, most, nullptr, sh);
+  if (wide && items) {
+    for (u32 i = 0; (w = alias_nth(i, spread)) < m.V; ++i)
+      if (m.nnz[w] == kNnzWide) alias_word_of(m, w, m.shares ? sh_shares : nullptr, sm.all, items, nullptr, sh);
     __syncthreads();
   }
   if (m.shares && threadIdx.x < 2)
     atomicAdd((unsigned long long*)m.shares + threadIdx.x, (unsigned long long)sh_shares[threadIdx.x]);
 }
 
-// The words that alias_build_kernel's warps left, a block to each.  Words are
-// ranked by frequency, so the wide ones are neighbours: as part of that kernel,
-// four to a block of half the threads, one block's words waited for each other
-// (K=4096, 2,000 words of 320 topics: 404 us, 99 before that kernel; K=12000,
-// 1,000 words of 750: 890 and 171).  Blocks take every gridDim-th word.
+// The words that alias_build_kernel's warps left, a block to each, K > 2048 (where
+// a word may need the block's slice of global scratch): K=4096, 2,000 words of 320
+// topics, 85 us together (404 with four of them to a block of that kernel);
+// K=12000, 1,000 words of 750, 191 (890).
 __global__ void __launch_bounds__(256) alias_wide_kernel(ModelDev m, unsigned char* gscratch, size_t slice,
                                                          u32 smem_items) {
   extern __shared__ __align__(16) unsigned char s_raw[];
-  __shared__ u64 sh[33], sh_shares[2];
-  if (threadIdx.x < 2) sh_shares[threadIdx.x] = 0;
-  __syncthreads();
+  __shared__ u64 sh[33];
   const AliasScratch all = alias_scratch_at(s_raw, smem_items);
-  unsigned char* g = gscratch ? gscratch + (size_t)blockIdx.x * slice : nullptr;
-  for_wide_words(m.nnz, 0, m.V, [&](u64 w) {
-    alias_word_of(m, w, m.shares ? sh_shares : nullptr, all, smem_items, g, sh);
-  });
-  __syncthreads();
-  if (m.shares && threadIdx.x < 2 && sh_shares[threadIdx.x])
-    atomicAdd((unsigned long long*)m.shares + threadIdx.x, (unsigned long long)sh_shares[threadIdx.x]);
+  unsigned char* g = gscratch + (size_t)blockIdx.x * slice;
+  for_wide_words(m.nnz, 0, m.V, [&](u64 w) { alias_word_of(m, w, nullptr, all, smem_items, g, sh); });
 }
 
 // Batched alias build over global words [w0, w1) of any problems; shared
 // memory sized for the largest K among them.
 __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_batch_kernel(ModelDev ar, BatchPhiDev bp, u32 most,
-                                                                             u32 Kmax, u32 w0, u32 w1) {
+                                                                             u32 Kmax, u32 w0, u32 w1, bool spread) {
   extern __shared__ __align__(16) unsigned char s_raw[];
   __shared__ u64 sh[33], sh_shares[2];
   __shared__ u32 wide;
-  const u32 nw = blockDim.x >> 5, warp = threadIdx.x >> 5;
+  const u32 warp = threadIdx.x >> 5;
   if (threadIdx.x < 2) sh_shares[threadIdx.x] = 0;
   if (threadIdx.x == 0) wide = 0;
   __syncthreads();
-  const AliasSmem sm = alias_smem(s_raw, most);
+  const AliasSmem sm = alias_smem(s_raw, most, Kmax);
   u64 x_all = 0, x_long = 0;
-  const u64 step = (u64)gridDim.x * nw, first = (u64)w0 + (u64)blockIdx.x * nw;
-  for (u64 w = first + warp; w < w1; w += step) {
+  u64 w;
+  for (u32 i = warp; (w = w0 + alias_nth(i, spread)) < w1; i += kAliasWarps) {
     const u32 pb = bp.wpid[w], K = bp.K[pb];
     const size_t row = bp.row_off[w];
     if (alias_word_warp(K, ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row,
@@ -735,26 +753,12 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_batch_kernel(
     atomicAdd((unsigned long long*)sh_shares + 1, (unsigned long long)x_long);
   }
   __syncthreads();
-  if (wide && Kmax <= most) {  // as alias_build_kernel
-    for (u64 wb = first; wb < w1; wb += step)
-      for (u64 w = wb; w < min((u64)w1, wb + nw); ++w)
-        if (ar.nnz[w] == kNnzWide) alias_word_of(ar, bp, w, sh_shares, sm.all, most, sh);
+  if (wide) {
+    for (u32 i = 0; (w = w0 + alias_nth(i, spread)) < w1; ++i)
+      if (ar.nnz[w] == kNnzWide) alias_word_of(ar, bp, w, sh_shares, sm.all, Kmax, sh);
     __syncthreads();
   }
   if (threadIdx.x < 2)
-    atomicAdd((unsigned long long*)ar.shares + threadIdx.x, (unsigned long long)sh_shares[threadIdx.x]);
-}
-
-// alias_wide_kernel for a batch.
-__global__ void __launch_bounds__(256) alias_wide_batch_kernel(ModelDev ar, BatchPhiDev bp, u32 Kmax, u32 w0, u32 w1) {
-  extern __shared__ __align__(16) unsigned char s_raw[];
-  __shared__ u64 sh[33], sh_shares[2];
-  if (threadIdx.x < 2) sh_shares[threadIdx.x] = 0;
-  __syncthreads();
-  const AliasScratch all = alias_scratch_at(s_raw, Kmax);
-  for_wide_words(ar.nnz, w0, w1, [&](u64 w) { alias_word_of(ar, bp, w, sh_shares, all, Kmax, sh); });
-  __syncthreads();
-  if (threadIdx.x < 2 && sh_shares[threadIdx.x])
     atomicAdd((unsigned long long*)ar.shares + threadIdx.x, (unsigned long long)sh_shares[threadIdx.x]);
 }
 
@@ -1004,20 +1008,12 @@ void launch_phi_draw_batch(const ModelDev& ar, const BatchPhiDev& bp, u32 n_bloc
 void launch_alias_build_batch(const ModelDev& ar, const BatchPhiDev& bp, u32 Kmax, u32 w0, u32 w1, cudaStream_t s) {
   if (w1 <= w0) return;
   const u32 most = alias_items(Kmax);
-  const size_t need = kAliasWarps * alias_warp_bytes(most);
+  const size_t need = std::max(kAliasWarps * alias_warp_bytes(most), alias_scratch_item_bytes(Kmax));
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, alias_build_batch_kernel, 32 * kAliasWarps, need);
   if (per_sm < 1) per_sm = 1;
-  const u32 blocks = std::min<u32>((w1 - w0 + kAliasWarps - 1) / kAliasWarps, (u32)(device_sm_count() * per_sm * 4));
-  alias_build_batch_kernel<<<blocks, 32 * kAliasWarps, need, s>>>(ar, bp, most, Kmax, w0, w1);
-  if (Kmax <= most) return;
-  const size_t smem = alias_scratch_item_bytes(Kmax);
-  const u32 nt = alias_threads(Kmax);
-  per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, alias_wide_batch_kernel, nt, smem);
-  if (per_sm < 1) per_sm = 1;
-  alias_wide_batch_kernel<<<std::min<u32>(w1 - w0, (u32)(device_sm_count() * per_sm)), nt, smem, s>>>(ar, bp, Kmax, w0,
-                                                                                                      w1);
+  const AliasGrid g = alias_grid(w1 - w0, Kmax, most, (u32)(device_sm_count() * per_sm));
+  alias_build_batch_kernel<<<g.blocks, 32 * kAliasWarps, need, s>>>(ar, bp, most, Kmax, w0, w1, g.spread);
 }
 
 void launch_bump(u32* t, cudaStream_t s) { bump_kernel<<<1, 1, 0, s>>>(t); }
@@ -1075,23 +1071,27 @@ size_t alias_build_scratch_bytes(u32 K) {
 u32 launch_alias_build(const ModelDev& m, cudaStream_t s, void* scratch, size_t scratch_bytes) {
   if (m.Sinv) topic_recip_kernel<<<(m.K + 255) / 256, 256, 0, s>>>(m.S, m.Sinv, m.K);
   const u32 most = alias_items(m.K), recip = m.Sinv ? 1u : 0u;
-  const size_t need = kAliasWarps * alias_warp_bytes(most);
+  const bool own = m.K <= kAliasSmemItems;
+  const size_t need = std::max(kAliasWarps * alias_warp_bytes(most), own ? alias_scratch_item_bytes(m.K) : 0);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, alias_build_kernel, 32 * kAliasWarps, need);
   if (per_sm < 1) per_sm = 1;
-  const u32 blocks = std::min<u32>((m.V + kAliasWarps - 1) / kAliasWarps,
-                                   (u32)(device_sm_count() * per_sm * (m.K <= kAliasSmemItems ? 4 : 1)));
-  alias_build_kernel<<<blocks, 32 * kAliasWarps, need, s>>>(m, most);
-  if (m.K <= most) return recip + 1;
-  const u32 items = std::min(m.K, kAliasSmemItems), nt = alias_threads(m.K);
-  const size_t smem = alias_scratch_item_bytes(items), slice = m.K > kAliasSmemItems ? alias_slice_bytes(m.K) : 0;
+  const u32 resident = (u32)(device_sm_count() * per_sm);
+  if (own) {
+    const AliasGrid g = alias_grid(m.V, m.K, most, resident);
+    alias_build_kernel<<<g.blocks, 32 * kAliasWarps, need, s>>>(m, most, m.K, g.spread);
+    return recip + 1;
+  }
+  const u32 blocks = std::min<u32>((m.V + kAliasWarps - 1) / kAliasWarps, resident);
+  alias_build_kernel<<<blocks, 32 * kAliasWarps, need, s>>>(m, most, 0u, false);
+  const u32 items = kAliasSmemItems, nt = alias_threads(m.K);
+  const size_t smem = alias_scratch_item_bytes(items), slice = alias_slice_bytes(m.K);
   per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, alias_wide_kernel, nt, smem);
   if (per_sm < 1) per_sm = 1;
-  u32 wide = std::min<u32>(m.V, (u32)(device_sm_count() * per_sm));
-  if (slice) wide = std::min<u32>(wide, (u32)(scratch_bytes / slice));
+  const u32 wide = std::min({m.V, (u32)(device_sm_count() * per_sm), (u32)(scratch_bytes / slice)});
   if (!wide) return recip + 1;  // no scratch: the caller allocates alias_build_scratch_bytes(K)
-  alias_wide_kernel<<<wide, nt, smem, s>>>(m, slice ? (unsigned char*)scratch : nullptr, slice, items);
+  alias_wide_kernel<<<wide, nt, smem, s>>>(m, (unsigned char*)scratch, slice, items);
   return recip + 2;
 }
 
