@@ -81,9 +81,9 @@ __device__ __forceinline__ Run lane_run(u32 nw, u32 l) {
 // A word's list is short up to this many entries.
 constexpr u32 kShortList = 160;
 
-// How many tokens of words with short lists make up for one whose word has a list
-// of nw entries (mostly_long_lists).
-__host__ __device__ inline u32 long_list_weight(u32 nw) { return nw > kShortList ? 11 + nw * nw / 100000 : 0; }
+// How many twelfths of a token whose word has a short list make up for one whose
+// word has a list of nw entries (mostly_long_lists): 10 + nw^2 / 1e5 tokens.
+__host__ __device__ inline u32 long_list_weight(u32 nw) { return nw > kShortList ? 120 + nw * nw / 8333 : 0; }
 
 struct ModelDev {
   u32 K, V;
@@ -253,7 +253,7 @@ void launch_z_sweep_words(const ModelDev& m, const BatchDev* b, u32 Kmax, const 
 // with one such token in 9, 10, 17 or 50; with documents of 400 in 20 or 70 of the
 // last two.  (One in 12 whatever the lengths: 2.15 for 1.03 ms with 8 % of the
 // tokens in lists of 2000 entries.)
-__device__ __forceinline__ bool mostly_long_lists(const u64* shares) { return shares[1] > shares[0]; }
+__device__ __forceinline__ bool mostly_long_lists(const u64* shares) { return shares[1] > 12 * shares[0]; }
 // The same sweep with each document's counts in a shared-memory hash map
 // (large K).  Documents longer than lmax are reported, not swept.  Returns
 // false without launching when lmax needs more shared memory than a block has.

@@ -652,7 +652,7 @@ int choose_walk(Server& s) {
     all += (double)A[w];
     in_long += (double)A[w] * long_list_weight(nnz[w]);
   }
-  s.words = s.fc.m.lists && in_long <= all;
+  s.words = s.fc.m.lists && in_long <= 12.0 * all;
   return GPULDA_OK;
 }
 
