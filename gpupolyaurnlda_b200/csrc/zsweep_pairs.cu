@@ -48,9 +48,12 @@ constexpr u32 kNone = 0xffffu;     // no topic (topics are below 32768)
 constexpr u32 kSparseBit = 0x8000u;
 constexpr u32 kLongAhead = 4;  // entries of a word's list that a lane reads ahead (2: up to a third slower)
 // Lists in shared memory have their q values there if that leaves a block this
-// many warps (three times the memory): K=9000, 2,000 documents of 1,000 tokens of
-// which the lengths are on the device only, 40 ms with one, 20 with two or three.
-constexpr u32 kStagedWarps = 2;
+// many warps (three times the memory).  2,000 documents of 1,000 tokens of which
+// the lengths are on the device only: 40 ms with one such warp (K=9000), 22 with
+// two (K=6000), 20 and 14 with the q values loaded as they are summed and room for
+// more warps; with lengths on the host and lists in shared memory for few of the
+// documents the q values there save 10 % (K=6000, 18.2 for 21.3).
+constexpr u32 kStagedWarps = 3;
 constexpr u32 kBitsAhead = 4;  // tokens whose words' bits are loaded at a time (1: 11.3 ms, 2: 10.3, 8: 10.0)
 constexpr u32 kBitsMost = 8;   // entries a lane with room for the bits in registers
 
