@@ -332,13 +332,14 @@ __device__ __forceinline__ u64 fixed_phi(u32 x, u32 k, const u64* __restrict__ S
 // kPerThread consecutive topics per tile, so a tile needs one block scan.
 // The alias build's scratch (10 bytes per nonzero) is shared memory when the
 // word's nonzeros fit smem_items, else the block's slice of global scratch.
+// listed: the draws (x << 32 | k) that stand in csrrow already, all of the row's,
+// or 0.
 constexpr u32 kPerThread = 8;
 constexpr u32 kAliasWarps = 4;  // a block's, a word each
 // Most topics of a word that a warp takes (18 bytes each set how many warps are
 // resident); a longer word takes a block, above K = 2048 of a launch of its own.
-// K=1000: 128, 256 and 512 take 218,
-// 210 and 243 us at the mid corpus; K=10000, whose words' lists are longer: 1350,
-// 900 and 700 us.
+// K=1000: 128, 256 and 512 take 218, 210 and 243 us at the mid corpus; K=10000,
+// whose words' lists are longer, before that launch: 1350, 900 and 700 us.
 inline u32 alias_items(u32 K) { return std::min(K, K <= kMapMinK ? 256u : 512u); }
 __host__ __device__ constexpr size_t alias_warp_bytes(u32 most) { return ((size_t)most * 18 + 15) & ~(size_t)15; }
 
@@ -356,14 +357,34 @@ __device__ __forceinline__ void list_bits(const u64* ent, u32 n, u32* bits, u32 
 
 __device__ __forceinline__ void alias_word(u32 K, u32* __restrict__ qrow, const u64* __restrict__ S,
                                            const u64* __restrict__ Sinv, u64* alrow, u64* csrrow, u64* eighths,
-                                           u32* bits, u64* A_out, u64* s_shares, u32* nnz_out, u64* s_vals,
-                                           uint16_t* s_idx, u32 smem_items, u64* g_vals, uint16_t* g_idx, u64* sh) {
+                                           u32* bits, u64* A_out, u64* s_shares, u32* nnz_out, u32 listed,
+                                           u64* s_vals, uint16_t* s_idx, u32 smem_items, u64* g_vals, uint16_t* g_idx,
+                                           u64* sh) {
   u64 part = 0, nz = 0;
   u32 xsum = 0;
   if (bits)
     for (u32 i = threadIdx.x; i < bits_stride(K); i += blockDim.x) bits[i] = 0;
+  if (listed) {
+    bool zero = false;
+    for (u32 i = threadIdx.x; i < listed; i += blockDim.x) {
+      const u64 e = csrrow[i];
+      const u64 qq = fixed_phi((u32)(e >> 32), (u32)e, S, Sinv);
+      zero |= !qq;
+      part += qq;
+      xsum += (u32)(e >> 32);
+      csrrow[i] = (qq << 32) | (u32)e;
+    }
+    if (__syncthreads_or(zero)) {  // a draw that rounds to q = 0 is not in the list: from the row, still as drawn
+      listed = 0;
+      part = 0;
+      xsum = 0;
+    } else {
+      for (u32 i = threadIdx.x; i < listed; i += blockDim.x) qrow[(u32)csrrow[i]] = (u32)(csrrow[i] >> 32);
+      nz = listed;
+    }
+  }
   const u32 tile = blockDim.x * kPerThread;
-  for (u32 t0 = 0; t0 < K; t0 += tile) {
+  for (u32 t0 = 0; !listed && t0 < K; t0 += tile) {
     const u32 k0 = t0 + threadIdx.x * kPerThread;
     u32 qv[kPerThread];
     u32 cnt = 0;
@@ -418,31 +439,26 @@ __device__ __forceinline__ void alias_word(u32 K, u32* __restrict__ qrow, const 
   __syncthreads();
 }
 
-// The same by one warp, for a word of at most `most` topics.  Returns false
-// with nothing written for a word of more, or with a draw that rounds to q = 0
-// (a topic's sum above 2^32).  A trained word has some tens of topics, so a
-// block on it waited at barriers: six scans of eight warps' sums for one or two
-// entries a lane.  Here the row is only looked through for its nonzero draws,
-// and everything after works on those: ent[most] holds them, vals and idx are
-// the alias build's scratch, all the warp's own.  Bound by instructions (about
-// 1,500 a word beside 4 KB of row at K=1000).  1e5 words of 65 topics (K=1000)
-// 622 -> 212 us, 1.4e5 words 816 -> 259; 3e4 words, K=10000, 1185 -> 726 us
-// where the rows' 1.2 GB take 183; from a random start (50,000 words of 100
-// to 1000 topics) 337 -> 146.
-__device__ __forceinline__ bool alias_word_warp(u32 K, u32* qrow, const u64* __restrict__ S,
-                                                const u64* __restrict__ Sinv, u64* alrow, u64* csrrow, u64* eighths,
-                                                u32* bits, u64* A_out, u32* nnz_out, u64& x_all, u64& x_long,
-                                                u64* ent, u64* vals, uint16_t* idx, u32 most) {
+constexpr u32 kNnzWide = 0x80000000u;  // marks a word that its warp left to a block, beside its listed draws
+
+// The aligned groups of four cells that a row lies in; it starts at cell `head` of
+// the first.
+__device__ __forceinline__ u32 row_head(const u32* qrow) { return (u32)((uintptr_t)qrow >> 2) & 3; }
+__device__ __forceinline__ u32 row_groups(const u32* qrow, u32 K) { return (K + row_head(qrow) + 3) / 4; }
+
+// Goes on through a row from its aligned group `g` of four cells: put(i, x << 32 | k)
+// for its i-th nonzero draw, i from n on.  Returns their number; where that would
+// pass `most`, the number before the groups from `g` on, else `g` is past the row.
+template <class Put>
+__device__ __forceinline__ u32 row_draws(const u32* qrow, u32 K, u32& g, u32 n, u32 most, Put put) {
   constexpr u32 kInFlight = 4;  // loads of 512 bytes; 8 take registers and a resident block (mid 212 -> 239 us)
   const u32 lane = threadIdx.x & 31, before = (1u << lane) - 1;
-  const u32 head = (u32)((uintptr_t)qrow >> 2) & 3;  // the row starts inside an aligned group of four
-  const u32 groups = (K + head + 3) / 4;
-  u32 n = 0;
-  for (u32 g0 = 0; g0 < groups; g0 += 32 * kInFlight) {
+  const u32 head = row_head(qrow), groups = row_groups(qrow, K);
+  for (; g < groups; g += 32 * kInFlight) {
     u32 v[kInFlight][4];
 #pragma unroll
     for (u32 u = 0; u < kInFlight; ++u) {
-      const i32 k = (i32)(4 * (g0 + 32 * u + lane)) - (i32)head;
+      const i32 k = (i32)(4 * (g + 32 * u + lane)) - (i32)head;
       if (k >= 0 && k + 4 <= (i32)K) {
         const uint4 x = *reinterpret_cast<const uint4*>(qrow + k);
         v[u][0] = x.x, v[u][1] = x.y, v[u][2] = x.z, v[u][3] = x.w;
@@ -458,14 +474,56 @@ __device__ __forceinline__ bool alias_word_warp(u32 K, u32* qrow, const u64* __r
       const u32 b0 = __ballot_sync(kFullMask, cnt & 1), b1 = __ballot_sync(kFullMask, cnt & 2),
                 b2 = __ballot_sync(kFullMask, cnt & 4);
       u32 pos = n + __popc(b0 & before) + 2 * __popc(b1 & before) + 4 * __popc(b2 & before);
-      n += __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
-      if (n > most) return false;
-      const u32 k = 4 * (g0 + 32 * u + lane) - head;
+      const u32 after = n + __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
+      if (after > most) {
+        g += 32 * u;
+        return n;
+      }
+      n = after;
+      const u32 k = 4 * (g + 32 * u + lane) - head;
 #pragma unroll
       for (u32 c = 0; c < 4; ++c)
-        if (v[u][c]) ent[pos++] = ((u64)v[u][c] << 32) | (k + c);
+        if (v[u][c]) put(pos++, ((u64)v[u][c] << 32) | (k + c));
     }
   }
+  return n;
+}
+
+// The rest of a row of too many draws for the warp's memory: ent's n, then those
+// from group `g` on, to the word's list.  Returns the word's marked number.
+static __device__ __noinline__ u32 list_wide(const u32* qrow, u32 K, u32 g, const u64* ent, u32 n, u64* csrrow) {
+  __syncwarp();
+  for (u32 i = threadIdx.x & 31; i < n; i += 32) csrrow[i] = ent[i];
+  return kNnzWide | row_draws(qrow, K, g, n, ~0u, [&](u32 i, u64 e) { csrrow[i] = e; });
+}
+
+// The same by one warp, for a word of at most `most` topics.  Returns 0, or
+// kNnzWide for a word that is left to a block: with nothing written if a draw
+// rounds to q = 0 (a topic's sum above 2^32) or there are too many in the first
+// `from` halves of the row, else with their number beside it and the draws
+// (x << 32 | k) listed in csrrow.  (Above K = 2048 all such rows are listed: K=4096,
+// 2,000 words of 640 topics 66 us, 85 if the block looks through the row again;
+// K=10000, 10,000 words of 750 349 and 646.  A block of the same launch looks
+// through the rest of a row faster than a warp lists it, so there rows that are
+// half done are: K=2000, 2,000 words of 320 topics 38 and 52 us, but 20,000 words
+// from a random start 185 and 170.)  A trained word has some tens of topics, so a
+// block on it waited at barriers: six scans of eight warps' sums for one or two
+// entries a lane.  Here the row is only looked through for its nonzero draws,
+// and everything after works on those: ent[most] holds them, vals and idx are
+// the alias build's scratch, all the warp's own.  Bound by instructions (about
+// 1,500 a word beside 4 KB of row at K=1000).  1e5 words of 65 topics (K=1000)
+// 622 -> 212 us, 1.4e5 words 816 -> 259; 3e4 words, K=10000, 1185 -> 726 us
+// where the rows' 1.2 GB take 183; from a random start (50,000 words of 100
+// to 1000 topics) 337 -> 146.
+__device__ __forceinline__ u32 alias_word_warp(u32 K, u32* qrow, const u64* __restrict__ S,
+                                               const u64* __restrict__ Sinv, u64* alrow, u64* csrrow, u64* eighths,
+                                               u32* bits, u64* A_out, u32* nnz_out, u64& x_all, u64& x_long, u64* ent,
+                                               u64* vals, uint16_t* idx, u32 most, u32 from) {
+  const u32 lane = threadIdx.x & 31;
+  u32 g = 0;
+  const u32 n = row_draws(qrow, K, g, 0, most, [&](u32 i, u64 e) { ent[i] = e; });
+  const u32 groups = row_groups(qrow, K);
+  if (g < groups) return g >= from * groups / 2 ? list_wide(qrow, K, g, ent, n, csrrow) : kNnzWide;
   __syncwarp();
   u64 part = 0, xsum = 0;
   bool zero = false;
@@ -477,7 +535,7 @@ __device__ __forceinline__ bool alias_word_warp(u32 K, u32* qrow, const u64* __r
     xsum += e >> 32;
     ent[i] = (qq << 32) | (u32)e;
   }
-  if (__any_sync(kFullMask, zero)) return false;
+  if (__any_sync(kFullMask, zero)) return kNnzWide;
   __syncwarp();
   const u64 A = warp_sum_u64(part);
   x_all += xsum;
@@ -501,7 +559,7 @@ __device__ __forceinline__ bool alias_word_warp(u32 K, u32* qrow, const u64* __r
     *A_out = A;
     *nnz_out = n;
   }
-  if (!n) return true;
+  if (!n) return 0;
   // alias_build_block's steps
   const u32 chunk = (n + 31) / 32, i0 = min(n, lane * chunk), i1 = min(n, i0 + chunk);
   u32 nl = 0;
@@ -565,7 +623,7 @@ __device__ __forceinline__ bool alias_word_warp(u32 K, u32* qrow, const u64* __r
     }
   }
   __syncwarp();
-  return true;
+  return 0;
 }
 
 // The block's alias scratch for one word of up to `items` topics.
@@ -596,8 +654,6 @@ __device__ __forceinline__ AliasSmem alias_smem(unsigned char* raw, u32 most, u3
   return a;
 }
 
-constexpr u32 kNnzWide = 0xffffffffu;  // marks a word that its warp left to a block
-
 // The i-th of a block's words: four neighbours at a time, or (spread) every
 // gridDim-th.  Words are ranked by frequency, so those with many topics are
 // neighbours, and a block builds those that its warps leave one after another.
@@ -608,9 +664,9 @@ __device__ __forceinline__ u64 alias_nth(u32 i, bool spread) {
 
 // Blocks of an alias build over V words with room for `resident` of them on the
 // GPU, and whether they spread: with few words, so that each block has about one
-// of many topics (K=2000, 2,000 words of 250 topics: 140 us with four neighbours to
-// a block).  With many, the blocks are enough, and neighbours cost less (1e5
-// words 259 us, 269 spread).
+// of many topics (K=2000, 2,000 words of 320 topics: 75 us with four neighbours to
+// a block, 52 spread, when each still looked through its row again).  With many,
+// the blocks are enough, and neighbours cost less (1e5 words 259 us, 269 spread).
 struct AliasGrid {
   u32 blocks;
   bool spread;
@@ -618,7 +674,8 @@ struct AliasGrid {
 inline AliasGrid alias_grid(u32 V, u32 K, u32 most, u32 resident) {
   AliasGrid g;
   g.spread = K > most && V < 16 * resident;
-  g.blocks = std::min(std::max((V + kAliasWarps - 1) / kAliasWarps, g.spread ? std::min(V, resident) : 1u), 4 * resident);
+  g.blocks = std::max((V + kAliasWarps - 1) / kAliasWarps, g.spread ? std::min(V, resident) : 1u);
+  g.blocks = std::min(g.blocks, 4 * resident);
   return g;
 }
 
@@ -630,7 +687,7 @@ __device__ __forceinline__ void for_wide_words(const u32* nnz, u64 w0, u64 w1, F
   const u32 nw = blockDim.x >> 5;
   for (u64 first = w0 + blockIdx.x; first < w1; first += (u64)gridDim.x * blockDim.x) {
     const u64 w = first + (u64)threadIdx.x * gridDim.x;
-    const u32 b = __ballot_sync(kFullMask, w < w1 && nnz[w] == kNnzWide);
+    const u32 b = __ballot_sync(kFullMask, w < w1 && (nnz[w] & kNnzWide));
     if ((threadIdx.x & 31) == 0) marked[threadIdx.x >> 5] = b;
     __syncthreads();
     for (u32 i = 0; i < nw; ++i)
@@ -647,8 +704,8 @@ __device__ __forceinline__ void alias_word_of(const ModelDev& m, u64 w, u64* s_s
   const size_t row = (size_t)w * K;
   alias_word(K, m.q + row, m.S, m.Sinv, m.al + row, m.csr + row,
              m.lists ? m.lists + (size_t)w * list_stride(K) : nullptr,
-             m.bits ? m.bits + (size_t)w * bits_stride(K) : nullptr, m.A + w, s_shares, m.nnz + w, all.vals, all.idx,
-             smem_items, (u64*)g, g ? (uint16_t*)((u64*)g + K) : nullptr, sh);
+             m.bits ? m.bits + (size_t)w * bits_stride(K) : nullptr, m.A + w, s_shares, m.nnz + w,
+             m.nnz[w] & ~kNnzWide, all.vals, all.idx, smem_items, (u64*)g, g ? (uint16_t*)((u64*)g + K) : nullptr, sh);
 }
 
 // Word w of a batch.
@@ -657,8 +714,8 @@ __device__ __forceinline__ void alias_word_of(const ModelDev& ar, const BatchPhi
   const u32 pb = bp.wpid[w];
   const size_t row = bp.row_off[w];
   alias_word(bp.K[pb], ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row,
-             ar.lists ? ar.lists + bp.list_off[w] : nullptr, nullptr, ar.A + w, s_shares, ar.nnz + w, all.vals, all.idx,
-             smem_items, nullptr, nullptr, sh);
+             ar.lists ? ar.lists + bp.list_off[w] : nullptr, nullptr, ar.A + w, s_shares, ar.nnz + w,
+             ar.nnz[w] & ~kNnzWide, all.vals, all.idx, smem_items, nullptr, nullptr, sh);
 }
 
 // items: most topics of a word that the block takes (at least K, or 0: those that
@@ -677,13 +734,13 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_kernel(ModelD
   u64 w;
   for (u32 i = warp; (w = alias_nth(i, spread)) < m.V; i += kAliasWarps) {
     const size_t row = (size_t)w * K;
-    if (alias_word_warp(K, m.q + row, m.S, m.Sinv, m.al + row, m.csr + row,
-                        m.lists ? m.lists + (size_t)w * list_stride(K) : nullptr,
-                        m.bits ? m.bits + (size_t)w * bits_stride(K) : nullptr, m.A + w, m.nnz + w, x_all, x_long,
-                        sm.ent, sm.vals, sm.idx, most))
-      continue;
+    const u32 left = alias_word_warp(K, m.q + row, m.S, m.Sinv, m.al + row, m.csr + row,
+                                     m.lists ? m.lists + (size_t)w * list_stride(K) : nullptr,
+                                     m.bits ? m.bits + (size_t)w * bits_stride(K) : nullptr, m.A + w, m.nnz + w, x_all,
+                                     x_long, sm.ent, sm.vals, sm.idx, most, items ? 1u : 0u);
+    if (!left) continue;
     if ((threadIdx.x & 31) == 0) {
-      m.nnz[w] = kNnzWide;
+      m.nnz[w] = left;
       wide = 1;
     }
     __syncwarp();
@@ -699,7 +756,7 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_kernel(ModelD
   __syncthreads();
   if (wide && items) {
     for (u32 i = 0; (w = alias_nth(i, spread)) < m.V; ++i)
-      if (m.nnz[w] == kNnzWide) alias_word_of(m, w, m.shares ? sh_shares : nullptr, sm.all, items, nullptr, sh);
+      if (m.nnz[w] & kNnzWide) alias_word_of(m, w, m.shares ? sh_shares : nullptr, sm.all, items, nullptr, sh);
     __syncthreads();
   }
   if (m.shares && threadIdx.x < 2)
@@ -707,9 +764,10 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_kernel(ModelD
 }
 
 // The words that alias_build_kernel's warps left, a block to each, K > 2048 (where
-// a word may need the block's slice of global scratch): K=4096, 2,000 words of 320
-// topics, 85 us together (404 with four of them to a block of that kernel);
-// K=12000, 1,000 words of 750, 191 (890).
+// a word may need the block's slice of global scratch): K=4096, 2,000 words of 640
+// topics, 66 us together (140 with four of them to a block of that kernel);
+// K=12000, 1,000 words of 750, 69 (267); K=10000, 10,000 of 750, 348 (1337).  Bound
+// by load latency and barriers.
 __global__ void __launch_bounds__(256) alias_wide_kernel(ModelDev m, unsigned char* gscratch, size_t slice,
                                                          u32 smem_items) {
   extern __shared__ __align__(16) unsigned char s_raw[];
@@ -736,12 +794,12 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_batch_kernel(
   for (u32 i = warp; (w = w0 + alias_nth(i, spread)) < w1; i += kAliasWarps) {
     const u32 pb = bp.wpid[w], K = bp.K[pb];
     const size_t row = bp.row_off[w];
-    if (alias_word_warp(K, ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row,
-                        ar.lists ? ar.lists + bp.list_off[w] : nullptr, nullptr, ar.A + w, ar.nnz + w, x_all, x_long,
-                        sm.ent, sm.vals, sm.idx, most))
-      continue;
+    const u32 left = alias_word_warp(K, ar.q + row, ar.S + bp.S_off[pb], nullptr, ar.al + row, ar.csr + row,
+                                     ar.lists ? ar.lists + bp.list_off[w] : nullptr, nullptr, ar.A + w, ar.nnz + w,
+                                     x_all, x_long, sm.ent, sm.vals, sm.idx, most, 1u);
+    if (!left) continue;
     if ((threadIdx.x & 31) == 0) {
-      ar.nnz[w] = kNnzWide;
+      ar.nnz[w] = left;
       wide = 1;
     }
     __syncwarp();
@@ -755,7 +813,7 @@ __global__ void __launch_bounds__(32 * kAliasWarps, 8) alias_build_batch_kernel(
   __syncthreads();
   if (wide) {
     for (u32 i = 0; (w = w0 + alias_nth(i, spread)) < w1; ++i)
-      if (ar.nnz[w] == kNnzWide) alias_word_of(ar, bp, w, sh_shares, sm.all, Kmax, sh);
+      if (ar.nnz[w] & kNnzWide) alias_word_of(ar, bp, w, sh_shares, sm.all, Kmax, sh);
     __syncthreads();
   }
   if (threadIdx.x < 2)
