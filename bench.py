@@ -172,9 +172,9 @@ def roofline_profile(workload: str, c) -> dict:
     scaled to this launch only for that workload."""
     if c.K > 2048:
         return {"kernel": "z_sweep_pairs_kernel", "traffic": None,
-                "traffic_note": "the committed ncu capture is a V=14,000 case of the kernel before its lists moved to "
-                                "registers (profiles/z_sweep_pairs_kernel_K10000_small_case.md), so no traffic is "
-                                "scaled to this launch"}
+                "traffic_note": "the committed ncu capture is a V=30,000 case of trained topics "
+                                "(profiles/z_sweep_pairs_kernel_K10000_bits.md: 321 B of DRAM traffic per token), so "
+                                "no traffic is scaled to this launch"}
     out = {"kernel": "z_sweep_kernel",
            "binding_resource": "L1 data pipe (74 % of wavefront slots in the ncu profile), issue (66 %) and "
                                "gather latency; DRAM at 2.6 %: 93 % of the gathers hit L2, half of them L1",

@@ -108,15 +108,15 @@ u32 at_least(const u32* d_len, const std::vector<u32>& order, u32 len) {
   return lo;
 }
 
-// Above kMapMinK topics a document's counts live in a shared-memory hash map
-// or list (a dense per-document count array would cost 2 K bytes of shared
-// memory); documents of at most kShortDoc tokens are swept by one launch with a
-// small map per warp, longer ones by a second launch sized for the longest.
+// Above kMapMinK topics a document's counts live in a list in a warp's registers
+// or, with GPULDA_FLAG_HASHMAP, in a hash map in shared memory (a dense
+// per-document count array would cost 2 K bytes of shared memory).  With the
+// map, documents of at most kShortDoc tokens are swept by one launch with a
+// small map per warp, longer ones by others sized for their longest.
 constexpr u32 kShortDoc = 256;
 
 // Documents longer than kShortDoc and at most kMidDoc tokens are swept by a
-// launch of their own, sized for them (and with the large-K store's topic
-// bitmap); the few longer ones by another.
+// launch of their own, sized for them; the few longer ones by another.
 constexpr u32 kMidDoc = 1024;
 
 // Longest-first order with the short documents (length <= kShortDoc) first:
@@ -1096,8 +1096,9 @@ int noalloc_launches(cudaStream_t s, u32* z, const u32* w, const u32* d_len, u32
   // The lengths are on the device only, so the launches take any document
   // length.  More documents than the GPU's warps (16 an SM) are swept longest
   // first, which the device finds out: 60,000 of 340 tokens' mean from a random
-  // start 17.5 -> 13.2 ms an iteration.  Fewer start at once, a warp each,
-  // in any order, and the three launches (9 us) would be lost on them.
+  // start 25 -> 22 ms for a chain's first iteration, 20.5 -> 16.5 for its
+  // twelfth.  Fewer start at once, a warp each, in any order, and the three
+  // launches (9 us) would be lost on them.
   ZLaunch zl = z_args(z, w, d_len, d_idx, nullptr, nullptr, n_docs, n_tokens, g.tok_offset);
   u32 n_long = n_docs;
   if (n_docs > 16u * (u32)device_sm_count()) {

@@ -45,9 +45,10 @@ __host__ __device__ inline u32 bits_stride(u32 K) { return (K + 255) / 256 * 8; 
 
 // Whether a large-K model keeps them (unless its sweeps are the hash map's, which
 // do not read them): where q takes several times the 126 MB of
-// L2, a gather of q mostly goes to HBM.  At 233 MB (K=7275) the bits made the
-// sweep 2.23 -> 2.44 ms and the alias build 0.36 -> 0.46; at 1.2 GB 13.7 -> 9.6
-// and 0.73 -> 0.78.
+// L2, a gather of q mostly goes to HBM.  At 233 MB (K=7275, few documents) the
+// bits made the sweep 2.23 -> 2.44 ms and the alias build 0.36 -> 0.46; at 1.2 GB
+// 13.7 -> 9.6 and 0.73 -> 0.78.  Between them, 150,000 documents of 80 tokens:
+// 5.80 -> 4.50 and 0.20 -> 0.22 at 320 MB, 6.37 -> 4.60 and 0.29 -> 0.30 at 580.
 inline bool bits_pay(u32 K, u32 V) { return K > kMapMinK && (u64)K * V * 4 > (512ull << 20); }
 
 // Where entry i of an eighths-stored list with c = list_pairs(n) stands; recip =

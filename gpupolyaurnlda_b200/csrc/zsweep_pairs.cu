@@ -21,17 +21,20 @@
 // GB there); before a chunk's draws each lane collects its topics' bits for the
 // chunk's words, many loads at a time, and only entries with mass are gathered:
 // 9.5 ms, 321 instead of 1,083 bytes of DRAM traffic a token, bound by issue (60
-// %) and a token's dependent steps.  (With the list in shared memory, searched and shifted at every draw,
-// 430 instructions, it was 25.3 ms.)  Documents in device memory at K=4096 (2e4 documents of up to 5000
-// tokens, no lengths on the host), whose lists had to be sized for K entries
-// each, 5.8 against 26 ms.
+// %) and a token's dependent steps.  (With the list in shared memory, searched
+// and shifted at every draw, 430 instructions, it was 25.3 ms.)  Documents in
+// device memory at K=4096 (2e4 documents of up to 5000 tokens, no lengths on the
+// host), whose lists had to be sized for K entries each: an iteration of 32 ms
+// now takes 12 to 15 while documents outgrow the registers (the first four of a
+// chain) and 6.5 to 8 after.
 //
 // A list in registers holds at most kListMost entries.  A document that outgrows
 // it is handed on with the token it stands at (its earlier tokens' new topics
-// are in z) to a second kernel, whose lists stay in shared memory: the list
-// standing still during a chunk, the positions of the tokens' topics and of
-// their dense draws' topics are looked up before the chunk's first draw, and a
-// draw changes two counts in place.
+// are in z) to a second kernel, whose lists stay in shared memory (long_chunk):
+// the list standing still during a chunk, the positions of the tokens' topics
+// and of their dense draws' topics are looked up before the chunk's first draw,
+// a draw changes two counts in place, and each token walks the document's or its
+// word's list, whichever is shorter.
 #include <algorithm>
 #include <cmath>
 
