@@ -370,8 +370,8 @@ def run_ours(args):
         srv_u.close()
         serving = {"metric": "served_docs_per_sec", "unit": "docs/s",
                    "workload": f"the chain's model after {args.warmup + args.steps} iterations, {SERVE_WORKLOAD}; "
-                               f"batched = persistent kernel (32 request warps per SM), unbatched = one launch per "
-                               f"document over {args.serve_slots} streams",
+                               f"batched = persistent kernel (24 or 28 request warps per SM), unbatched = one launch "
+                               f"per document over {args.serve_slots} streams",
                    "rates": [{"offered": r["offered_docs_per_sec"], "requests": r["requests"],
                               "batched": r["batched"], "unbatched": r["unbatched"],
                               "speedup": r["batched"]["docs_per_sec"] / r["unbatched"]["docs_per_sec"],
@@ -766,7 +766,7 @@ def run_serve(args):
     s = g.Sampler(c.alpha, c.beta, c.K, c.counts, buffer_size=16, max_D=4, seed=0)
     s.corpus_load(c.z.copy(), c.w, c.d_len)
     s.corpus_sweep(args.serve_train)
-    srv_b = Server(50, seed=0, max_inflight=1 << 17)  # persistent: 32 request warps per SM
+    srv_b = Server(50, seed=0, max_inflight=1 << 17)  # persistent: 24 or 28 request warps per SM
     srv_u = Server(50, mode="launch", slots=args.serve_slots, max_batch=1, seed=0)
     q_model = s.read_state(n=False, alias=False, A=False, S=False, nnz=False)["q"]
     s.close()
@@ -784,7 +784,7 @@ def run_serve(args):
                 "dtype": "u64", "data": "synthetic",
                 "config": {"workload": f"serving fold-in: K=1000 V=100000 model (mid corpus, {args.serve_train} "
                                        f"training iterations), {SERVE_WORKLOAD} at {list(args.rates)} docs/s",
-                           "batched": "persistent kernel, 32 request warps per SM",
+                           "batched": "persistent kernel, 24 or 28 request warps per SM",
                            "unbatched": f"one launch per document, {args.serve_slots} streams"},
                 "p50_ms": top["batched"]["p50_ms"], "p99_ms": top["batched"]["p99_ms"],
                 "unbatched": top["unbatched"],

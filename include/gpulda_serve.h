@@ -50,7 +50,8 @@ extern "C" {
 typedef struct GpuldaServeArgs {
   uint32_t n_iter;        /* fold-in iterations per request */
   uint32_t mode;          /* GPULDA_SERVE_PERSISTENT or GPULDA_SERVE_LAUNCH */
-  uint32_t slots;         /* persistent: request warps per SM, 1..32 (0: 32);
+  uint32_t slots;         /* persistent: request warps per SM, 1..32 (0: 32), of
+                             which up to 24 or 28 fit, by the model's lists;
                              launch: launches in flight (streams), 1..64 */
   uint32_t max_batch;     /* launch mode: requests per launch, 0: no limit */
   uint32_t max_inflight;  /* requests admitted and not yet handed out, 0: 16384 */
