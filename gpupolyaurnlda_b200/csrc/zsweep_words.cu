@@ -15,6 +15,8 @@ namespace {
 
 constexpr u32 kMaxDocLen = 65535u;
 constexpr size_t kZMaxSmem = 200 * 1024;
+constexpr u32 kSmSmem = 228 * 1024;      // an SM's shared memory
+constexpr u32 kBlockSmem = 1024 + 64;    // a block's beside the warps': the system's and its statistics
 
 struct ZWordArgs {
   ModelDev m;
@@ -217,8 +219,19 @@ __global__ void __launch_bounds__(256, 2) z_sweep_words_kernel(ZWordArgs a) {
 template <bool BATCH, bool LL>
 void launch_impl(const ZWordArgs& a, cudaStream_t s, u32 wpb, u32 blocks_per_sm) {
   const size_t per_warp = word_warp_bytes(a.Kmax);
-  // Warps per block: as many as fit the shared-memory budget (at most the request).
-  while (wpb > 1 && per_warp * wpb > kZMaxSmem) --wpb;
+  // Warps per block: the request, or fewer where more of them are resident then.
+  // (Above K = 1600 two blocks of 8 do not fit an SM's shared memory.  3e6 tokens
+  // over lists of 100 topics, with 8 warps resident and with 15 at K=1700 or 12 at
+  // K=2048: 0.84 -> 0.61 and 0.85 -> 0.71 ms.)
+  u32 most = 0, warps = 1;
+  for (u32 n = wpb; n; --n) {
+    const u32 resident = std::min<u32>(16, kSmSmem / (u32)(per_warp * n + kBlockSmem) * n);
+    if (per_warp * n <= kZMaxSmem && resident > most) {
+      most = resident;
+      warps = n;
+    }
+  }
+  wpb = warps;
   const size_t smem = per_warp * wpb;
   // The ceiling, not this launch's size: captured graphs may hold launches of
   // several sizes.  (The kernel's static shared memory counts towards the 48 KB
